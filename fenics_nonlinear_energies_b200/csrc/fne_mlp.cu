@@ -16,6 +16,7 @@
 //    without explicit transposes.
 //  * k_bias_silu_fwd, k_silu_bwd, k_colsum, k_adam, k_cast: elementwise work
 //    of the forward / backward pass and the optimiser.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -24,10 +25,12 @@
 
 #include "fne_internal.h"
 
+namespace cg = cooperative_groups;
+
 namespace fne {
 namespace {
 
-constexpr int kTcBM = 128, kTcBK = 64;  // C rows per CTA, K depth per staged slice
+constexpr int kTcBM = 128;  // rows per tile of the forward and input-gradient products
 constexpr long long kTcWaitLimit = 1LL << 22;
 
 // status of the tensor-core GEMM: 1 once an MMA-completion wait gave up
@@ -37,14 +40,14 @@ namespace tcg {
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
-// shared-memory matrix descriptor, no swizzle, K-major core matrices:
-// lbo = bytes between the two 16-byte K halves of one K = 16 step,
-// sbo = bytes between consecutive groups of 8 rows
-__device__ __forceinline__ uint64_t mat_desc(uint32_t a, uint32_t lbo, uint32_t sbo) {
+// shared-memory matrix descriptor: leading / stride byte offsets and swizzle (2, 4, 6: 128-, 64-, 32-byte lines).
+// K-major: stride = 8 rows; M/N-major: leading = next block of lines, stride = 8 lines.
+__device__ __forceinline__ uint64_t mat_desc(uint32_t a, uint32_t lbo, uint32_t sbo, uint32_t swizzle) {
   uint64_t d = (uint64_t)((a >> 4) & 0x3FFFu);
   d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
   d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
   d |= (uint64_t)1 << 46;  // descriptor version for sm_100
+  d |= (uint64_t)swizzle << 61;
   return d;
 }
 // instruction descriptor: D f32, A / B bf16, both K-major, M x N
@@ -64,11 +67,19 @@ __device__ __forceinline__ void commit(uint32_t mbar) {
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void mbar_init(uint32_t mbar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
+__device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, long long limit) {
+__device__ __forceinline__ void arrive(uint32_t mbar) {
+  asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}\n" ::"r"(mbar) : "memory");
+}
+// arrives once the thread's cp.async copies so far have landed
+__device__ __forceinline__ void arrive_copies(uint32_t mbar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(mbar) : "memory");
+}
+// Polls until the phase completed; gives up after `limit` polls, or early once *stop is set (may be null).
+__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, long long limit, const int* stop) {
   for (long long it = 0; it < limit; ++it) {
     uint32_t done;
     asm volatile(
@@ -78,144 +89,486 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, long l
         : "r"(mbar), "r"(parity)
         : "memory");
     if (done) return true;
+    if (stop && *reinterpret_cast<const volatile int*>(stop)) return false;
   }
   return false;
 }
 
 }  // namespace tcg
 
-// A(m, k) = A[m * sam + k * sak]; B(k, n) = B[k * sbk + n * sbn];
-// C(m, n) = C[m * ldc + n] (FP32).
-template <int BN>
-__global__ void __launch_bounds__(128) k_gemm_tc(int M, int N, int K, const __nv_bfloat16* __restrict__ A,
-                                                 long long sam, long long sak, const __nv_bfloat16* __restrict__ B,
-                                                 long long sbk, long long sbn, float* __restrict__ C, long long ldc,
-                                                 float beta, long long wait_limit) {
-  // core-matrix layout: element (row r, k) of a slice at [k / 8][r][k % 8]
-  __shared__ __align__(128) __nv_bfloat16 sA[kTcBK / 8][kTcBM][8];
-  __shared__ __align__(128) __nv_bfloat16 sB[kTcBK / 8][BN][8];
-  __shared__ __align__(8) unsigned long long s_bar;
+// ---------------------------------------------------------------------------
+// k_gemm_tc.  A(m, k) = A[m * sam + k * sak]; B(k, n) = B[k * sbk + n * sbn].
+//
+// What bounds it: at the network's sizes (8192 x 256 x 256) a product is
+// 1 GFLOP over 4 to 16 MB that stay in L2, so the MMAs are nearly free and the
+// time is the latency of one tile: loads, a few MMA steps, epilogue.  Hence
+//   * a ring of slices filled with cp.async by eight warps and multiplied by a
+//     ninth (full / empty mbarriers, no block barrier in the loop), laid down
+//     in the swizzled lines the MMA reads at full width: K-major for an operand
+//     whose K direction is contiguous, M/N-major (transposed descriptor) for
+//     one whose M/N direction is -- no operand is transposed by the threads;
+//   * 128 x 64 tiles below 148 tiles of 128 x 128, so that two CTAs share an
+//     SM and one's epilogue runs under the other's loads;
+//   * long products with few outputs (the weight gradient: 256 x 256, K = rows
+//     of the batch) take 64 x 16 tiles, 128-deep slices and an eight-stage
+//     ring: 64 CTAs instead of 4, each at the rate an SM reads from L2 (20 KB a
+//     slice, 43 bytes a cycle) with the MMA chain (65 cycles a step of 16) just
+//     below it.  The K loop is not split: the accumulator in TMEM rounds
+//     towards zero at every step, so partial sums over parts of K would change
+//     the weight gradient by 1e-9 of its size per row of the batch (1e-4 at
+//     60,000 rows);
+//   * the epilogue goes through shared memory so that rows leave in 16-byte
+//     stores.
+// Measured (warm L2): 256 x 256 x 8192 with both operands M/N-contiguous 37 us
+// (one 128 x 128 tile per CTA staged value by value: 2243 us); 8192 x 256 x 256
+// 9.5 to 12 us (23 to 28 us).
+// ---------------------------------------------------------------------------
+constexpr int kTcThreads = 256;  // filling / epilogue threads; one more warp multiplies
+enum { EPI_PLAIN = 0, EPI_FWD = 1, EPI_BWD = 2 };
+enum { LD_K16 = 0, LD_MN16 = 1, LD_SCALAR = 2 };  // how an operand is staged
+
+struct GemmArgs {
+  int M, N, K;
+  const __nv_bfloat16* A;
+  long long sam, sak;
+  const __nv_bfloat16* B;
+  long long sbk, sbn;
+  int mode_a, mode_b;
+  float* C;  // EPI_PLAIN: C = A B + beta C; EPI_FWD: the pre-activation (may be null); [M][ldc]
+  long long ldc;
+  float beta;
+  int vec_c;  // rows of every FP32 / BF16 array of the epilogue start 16 / 8 bytes aligned
+  // EPI_FWD: z = A B + bias; h32 / h16 = act ? silu(z) : z (either may be null); [M][N]
+  const float* bias;
+  int act;
+  float* h32;
+  __nv_bfloat16* h16;
+  // EPI_BWD: h16 = bf16(d), d = act ? (A B) silu'(z) : A B; colpart[m tile][n] = column sums of d
+  const float* z;
+  double* colpart;
+  // EPI_PLAIN: gb[m] = sum_j bias_part[j][m], by the CTA of n tile 0
+  const double* bias_part;
+  int n_parts;
+  float* gb;
+  long long wait_limit;
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// One operand's slice in shared memory, ROWS x BK values (rows r0.., depth k0..), in the swizzled layouts the
+// MMA reads at full width (the unswizzled core matrices cost about four times the cycles per MMA):
+//   K-major:   64-deep blocks of ROWS x 128 bytes, 16-byte chunk c of row r at chunk c ^ (r & 7);
+//   M/N-major: blocks of W = min(ROWS, 64) rows, BK lines of 2 W bytes, 16-byte chunk c of line k at
+//              c ^ (k & 7), (k >> 1) & 3 or (k >> 2) & 1 for lines of 128, 64 or 32 bytes.
+template <int ROWS, int BK>
+struct Operand {
+  static constexpr int RB = ROWS < 64 ? 2 * ROWS : 128;  // bytes of an M/N-major line
+  static constexpr int kChunks = ROWS * BK / 8, NC = (kChunks + kTcThreads - 1) / kTcThreads;
+
+  static __device__ __forceinline__ uint32_t k_major(int r, int c8) {
+    return (uint32_t)((c8 >> 3) * ROWS * 128 + r * 128 + (((c8 & 7) ^ (r & 7)) << 4));
+  }
+  static __device__ __forceinline__ uint32_t mn_major(int c, int k) {
+    constexpr int per = RB / 16;
+    const int sw = RB == 128 ? (k & 7) : RB == 64 ? ((k >> 1) & 3) : ((k >> 2) & 1);
+    return (uint32_t)((c / per) * BK * RB + k * RB + (((c % per) ^ sw) << 4));
+  }
+  static __device__ __forceinline__ uint64_t desc(uint32_t addr, int mode) {
+    if (mode != LD_MN16) return tcg::mat_desc(addr, 16, 1024, 2);
+    return tcg::mat_desc(addr, BK * RB, 8 * RB, RB == 128 ? 2 : RB == 64 ? 4 : 6);
+  }
+  // address offset of the 16-deep step kk
+  static __device__ __forceinline__ uint32_t step(int kk, int mode) {
+    return mode == LD_MN16 ? (uint32_t)(kk * 16 * RB) : (uint32_t)((kk >> 2) * ROWS * 128 + (kk & 3) * 32);
+  }
+
+  // this thread's chunks: source of the next slice, place in the slice, depth, valid rows
+  const __nv_bfloat16* p[NC];
+  uint32_t d[NC];
+  int kk[NC], rows[NC];
+  long long adv;
+  int mode;
+  bool whole;
+
+  __device__ __forceinline__ void init(const __nv_bfloat16* P, long long sr, long long sk, int md, int r0, int R) {
+    mode = md;
+    adv = sk * BK;
+    whole = true;
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      const int idx = threadIdx.x + i * kTcThreads;
+      // consecutive threads take consecutive 16 bytes of a line: whole 128-byte requests, and no bank
+      // conflicts with the swizzle
+      if (md == LD_K16) {
+        const int r = (idx >> 3) % ROWS, c8 = (idx & 7) + 8 * (idx / (8 * ROWS));
+        p[i] = P + (long long)(r0 + r) * sr + 8 * c8;
+        d[i] = k_major(r, c8);
+        kk[i] = 8 * c8;
+        rows[i] = r0 + r < R ? 8 : 0;
+      } else {
+        constexpr int per = RB / 16;
+        const int g = idx % per + per * (idx / (per * BK)), k = (idx / per) % BK;
+        p[i] = P + (long long)k * sk + r0 + 8 * g;
+        d[i] = mn_major(g, k);
+        kk[i] = k;
+        rows[i] = max(0, min(8, R - r0 - 8 * g));
+      }
+      whole = whole && rows[i] == 8;
+    }
+  }
+  // Issues this thread's copies of the slice at depth k0 (zero beyond (R, K)).
+  __device__ __forceinline__ void copy(unsigned char* slot, int k0, int K) {
+    const uint32_t dst = tcg::saddr(slot);
+    if (whole && k0 + BK <= K) {  // no edge in this thread's chunks: copies back to back
+#pragma unroll
+      for (int i = 0; i < NC; ++i)
+        if (kChunks % kTcThreads == 0 || i < NC - 1 || threadIdx.x + i * kTcThreads < kChunks)
+          cp_async16(dst + d[i], p[i]);
+#pragma unroll
+      for (int i = 0; i < NC; ++i) p[i] += adv;
+      return;
+    }
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      if (kChunks % kTcThreads && threadIdx.x + i * kTcThreads >= kChunks) break;
+      const int left = K - k0 - kk[i];
+      const int n = mode == LD_K16 ? min(rows[i], left) : (left > 0 ? rows[i] : 0);
+      if (n == 8) {
+        cp_async16(dst + d[i], p[i]);
+      } else {  // edge of the operand: what is there, zeros behind it
+        __nv_bfloat16 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = j < n ? p[i][j] : __float2bfloat16(0.f);
+        *reinterpret_cast<uint4*>(slot + d[i]) = *reinterpret_cast<const uint4*>(v);
+      }
+      p[i] += adv;
+    }
+  }
+  // Any strides and alignment (the 12 features, the 3 outputs): value by value into the K-major image, eight
+  // loads in flight a thread.  Chunks without a value are zeroed when the slot is first used and in a last,
+  // partial slice.
+  static __device__ __forceinline__ void scalar(unsigned char* slot, const __nv_bfloat16* __restrict__ P,
+                                                long long sr, long long sk, int r0, int R, int k0, int K, bool first) {
+    const int rv = min(ROWS, R - r0), left = min(BK, K - k0), cv = (left + 7) >> 3;
+    if (first || left < BK)
+      for (int idx = threadIdx.x; idx < kChunks; idx += kTcThreads) {
+        const int r = idx / (BK / 8), c8 = idx % (BK / 8);
+        if (r >= rv || c8 >= cv) *reinterpret_cast<uint4*>(slot + k_major(r, c8)) = make_uint4(0u, 0u, 0u, 0u);
+      }
+    int lg = 3;  // depth covered by a group of threads: the power of two at or above the chunks that hold values
+    while ((1 << lg) < 8 * cv) ++lg;
+    const int c = threadIdx.x & ((1 << lg) - 1), step = kTcThreads >> lg;
+    if (c >= 8 * cv) return;
+    const bool in = c < left;
+    const __nv_bfloat16* q = P + (long long)(k0 + c) * sk + (long long)r0 * sr;
+    const __nv_bfloat16 zero = __float2bfloat16(0.f);
+    for (int r = threadIdx.x >> lg; r < rv; r += 8 * step) {
+      __nv_bfloat16 v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = in && r + j * step < rv ? q[(long long)(r + j * step) * sr] : zero;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (r + j * step < rv)
+          *reinterpret_cast<__nv_bfloat16*>(slot + k_major(r + j * step, c >> 3) + 2 * (c & 7)) = v[j];
+    }
+  }
+};
+
+// Tile shape, slice depth and ring length of one instantiation.
+template <int BM_, int BN_, int BK_, int NST_>
+struct GemmCfg {
+  static constexpr int BM = BM_, BN = BN_, BK = BK_, NST = NST_;
+  static constexpr int kA = BM * BK * 2, kB = BN * BK * 2, kStage = kA + kB;
+  static constexpr int kLd = BN + 4;  // floats per row of the output tile: 16-byte rows, conflict-free quads
+  static constexpr int kTile = BM * kLd * 4;
+  static constexpr int kRing = NST * kStage;
+  static constexpr int kBody = kRing > kTile ? kRing : kTile;
+  static constexpr int kSums = 8 * 128 * 8;  // column sums: 8 warps x 128 doubles
+  static constexpr int kBytes = kBody + kSums + 1024;  // + alignment of the ring
+  static constexpr int kCols = BN < 32 ? 32 : BN;  // TMEM columns
+};
+using GemmWide = GemmCfg<128, 128, 64, 4>;
+using GemmMid = GemmCfg<128, 64, 64, 4>;
+using GemmNarrow = GemmCfg<128, 32, 64, 4>;
+using GemmLong = GemmCfg<64, 16, 128, 8>;
+
+template <class CF, int EPI>
+__global__ void __launch_bounds__(kTcThreads + 32) k_gemm_tc(const GemmArgs a) {
+  constexpr int BM = CF::BM, BN = CF::BN, BK = CF::BK, NST = CF::NST;
+  extern __shared__ unsigned char smem_raw[];
+  // the swizzle works on address bits: slots start on 1024-byte boundaries
+  unsigned char* smem = smem_raw + ((1024u - (tcg::saddr(smem_raw) & 1023u)) & 1023u);
+  __shared__ __align__(8) unsigned long long s_full[NST], s_empty[NST];
   __shared__ uint32_t s_tmem;
   __shared__ int s_fail;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * kTcBM, n0 = blockIdx.x * BN;
-  constexpr int TCOLS = BN < 32 ? 32 : BN;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tcg::saddr(&s_tmem)),
-                 "r"(TCOLS)
+                 "r"(CF::kCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
-    tcg::mbar_init(tcg::saddr(&s_bar));
+    for (int i = 0; i < NST; ++i) {
+      tcg::mbar_init(tcg::saddr(&s_full[i]), 2 * kTcThreads);
+      tcg::mbar_init(tcg::saddr(&s_empty[i]), 1);
+    }
     s_fail = 0;
   }
   tcg::fence_before();
   __syncthreads();
   tcg::fence_after();
-  const uint32_t tmem = s_tmem, bar = tcg::saddr(&s_bar);
-  constexpr uint32_t idesc = tcg::idesc_bf16(kTcBM, BN);
-  const __nv_bfloat16 zero = __float2bfloat16(0.f);
-  uint32_t phase = 0;
-  // operands whose K direction is contiguous and 16-byte aligned are staged
-  // eight values (one core-matrix row of 16 bytes) per load
-  const bool a_vec = sak == 1 && (K & 7) == 0 && (sam & 7) == 0 && ((uintptr_t)A & 15) == 0;
-  const bool b_vec = sbk == 1 && (K & 7) == 0 && (sbn & 7) == 0 && ((uintptr_t)B & 15) == 0;
-  for (int k0 = 0; k0 < K; k0 += kTcBK) {
-    // stage the slices (walking the operand's contiguous direction fastest)
-    if (a_vec) {
-      for (int idx = tid; idx < kTcBM * (kTcBK / 8); idx += 128) {
-        const int r = idx / (kTcBK / 8), c8 = idx - r * (kTcBK / 8);
-        const int m = m0 + r, k = k0 + 8 * c8;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (m < M && k < K) v = __ldg(reinterpret_cast<const uint4*>(A + (long long)m * sam + k));
-        *reinterpret_cast<uint4*>(&sA[c8][r][0]) = v;
+  const uint32_t tmem = s_tmem, base = tcg::saddr(smem);
+  const int ns = (a.K + BK - 1) / BK;
+  const uint32_t idesc = tcg::idesc_bf16(BM, BN) | (a.mode_a == LD_MN16 ? 1u << 15 : 0u) |
+                         (a.mode_b == LD_MN16 ? 1u << 16 : 0u);
+  using OpA = Operand<BM, BK>;
+  using OpB = Operand<BN, BK>;
+  // Warps 0..7 fill the ring, one thread of warp 8 multiplies.  A slice is full once every filling thread's
+  // copies landed (cp.async arrival) and its plain stores are done (ordinary arrival); the multiplying thread
+  // then fences the generic proxy's writes for the tensor core.  That fence has to sit in a thread without
+  // copies of its own in flight: it waits for them, which held the ring to one slice per memory latency when
+  // the filling threads ran it.
+  int fail = 0, issued = 0;
+  if (warp < 8) {
+    OpA oa;
+    OpB ob;
+    oa.init(a.A, a.sam, a.sak, a.mode_a, m0, a.M);
+    ob.init(a.B, a.sbn, a.sbk, a.mode_b, n0, a.N);
+    for (int i = 0; i < ns; ++i) {
+      if (i >= NST && !tcg::mbar_wait(tcg::saddr(&s_empty[i % NST]), ((i / NST) - 1) & 1, a.wait_limit, &s_fail)) {
+        fail = 1;
+        break;
       }
-    } else
-    for (int idx = tid; idx < kTcBM * kTcBK; idx += 128) {
-      int r, c;
-      if (sak == 1) {
-        r = idx / kTcBK; c = idx - r * kTcBK;
-      } else {
-        c = idx / kTcBM; r = idx - c * kTcBM;
-      }
-      const int m = m0 + r, k = k0 + c;
-      sA[c >> 3][r][c & 7] = (m < M && k < K) ? A[(long long)m * sam + (long long)k * sak] : zero;
+      unsigned char* slot = smem + (i % NST) * CF::kStage;
+      const int k0 = i * BK;
+      if (a.mode_a == LD_SCALAR)
+        OpA::scalar(slot, a.A, a.sam, a.sak, m0, a.M, k0, a.K, i < NST);
+      else
+        oa.copy(slot, k0, a.K);
+      if (a.mode_b == LD_SCALAR)
+        OpB::scalar(slot + CF::kA, a.B, a.sbn, a.sbk, n0, a.N, k0, a.K, i < NST);
+      else
+        ob.copy(slot + CF::kA, k0, a.K);
+      tcg::arrive_copies(tcg::saddr(&s_full[i % NST]));
+      tcg::arrive(tcg::saddr(&s_full[i % NST]));
     }
-    if (b_vec) {
-      for (int idx = tid; idx < BN * (kTcBK / 8); idx += 128) {
-        const int r = idx / (kTcBK / 8), c8 = idx - r * (kTcBK / 8);
-        const int n = n0 + r, k = k0 + 8 * c8;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (n < N && k < K) v = __ldg(reinterpret_cast<const uint4*>(B + (long long)n * sbn + k));
-        *reinterpret_cast<uint4*>(&sB[c8][r][0]) = v;
+  } else if (lane == 0) {
+    // one thread's instruction latency is on the chain of every slice: the descriptors of stage 0 are formed
+    // once, a stage or a 16-deep step only adds to their address field (14 bits of 16-byte units, no carry out)
+    const uint64_t da = OpA::desc(base, a.mode_a), db = OpB::desc(base + CF::kA, a.mode_b);
+    for (int i = 0; i < ns; ++i) {
+      if (!tcg::mbar_wait(tcg::saddr(&s_full[i % NST]), (i / NST) & 1, a.wait_limit, &s_fail)) {
+        fail = 1;
+        break;
       }
-    } else
-    for (int idx = tid; idx < BN * kTcBK; idx += 128) {
-      int r, c;
-      if (sbk == 1) {
-        r = idx / kTcBK; c = idx - r * kTcBK;
-      } else {
-        c = idx / BN; r = idx - c * BN;
-      }
-      const int n = n0 + r, k = k0 + c;
-      sB[c >> 3][r][c & 7] = (n < N && k < K) ? B[(long long)k * sbk + (long long)n * sbn] : zero;
-    }
-    tcg::fence_proxy_async();  // the generic-proxy stores, visible to the tensor core
-    __syncthreads();
-    if (tid == 0) {
-      tcg::fence_after();
+      tcg::fence_proxy_async();
+      const uint64_t off = (uint64_t)((i % NST) * (CF::kStage >> 4));
 #pragma unroll
-      for (int kk = 0; kk < kTcBK / 16; ++kk) {
-        const uint64_t ad = tcg::mat_desc(tcg::saddr(&sA[2 * kk][0][0]), kTcBM * 16, 128);
-        const uint64_t bd = tcg::mat_desc(tcg::saddr(&sB[2 * kk][0][0]), BN * 16, 128);
-        tcg::mma(tmem, ad, bd, idesc, (k0 > 0 || kk > 0) ? 1u : 0u);
-      }
-      tcg::commit(bar);
-      if (!tcg::mbar_wait(bar, phase, wait_limit)) s_fail = 1;
+      for (int kk = 0; kk < BK / 16; ++kk)
+        tcg::mma(tmem, da + off + (OpA::step(kk, a.mode_a) >> 4), db + off + (OpB::step(kk, a.mode_b) >> 4), idesc,
+                 (i > 0 || kk > 0) ? 1u : 0u);
+      tcg::commit(tcg::saddr(&s_empty[i % NST]));
+      issued = i + 1;
     }
-    phase ^= 1u;
-    __syncthreads();  // the slices stay until their MMAs completed
-    if (s_fail) break;
+    // the last commit covers every MMA before it
+    if (issued > 0 && !tcg::mbar_wait(tcg::saddr(&s_empty[(issued - 1) % NST]), ((issued - 1) / NST) & 1,
+                                      a.wait_limit, nullptr)) {
+      fail = 1;
+      // none in flight when shared memory is reused and TMEM released
+      tcg::mbar_wait(tcg::saddr(&s_empty[(issued - 1) % NST]), ((issued - 1) / NST) & 1, kTcWaitLimit, nullptr);
+    }
   }
-  if (s_fail) {
-    if (tid == 0) {
-      tcg::mbar_wait(bar, phase ^ 1u, kTcWaitLimit);  // no MMA in flight when TMEM is released
-      atomicExch(&g_gemm_err, 1);
-    }
-  } else if (K > 0) {
-    tcg::fence_after();
-    const int m = m0 + warp * 32 + lane;
-#pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 8) {
-      uint32_t r[8];
-      const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
-      asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                   : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                   : "r"(ta)
-                   : "memory");
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (m < M)
+  if (fail) s_fail = 1;
+  cp_async_wait_all();
+  fail = __syncthreads_or(fail);
+  if (fail && tid == 0) atomicExch(&g_gemm_err, 1);
+  // accumulator -> shared tile [BM][BN + 4] (the ring is free: all MMAs completed).  A warp reads its
+  // quadrant of 32 TMEM lanes; with BM = 64 the rows sit in the first 16 lanes of each quadrant.
+  float* tile = reinterpret_cast<float*>(smem);
+  tcg::fence_after();
+  if (!fail && warp < 8) {
+    constexpr int kRowsQ = BM / 4;
+    const int row = (warp & 3) * kRowsQ + lane, half = (warp >> 2) * (BN / 2);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int n = n0 + c0 + j;
-          if (n < N) {
-            float* cp = C + (long long)m * ldc + n;
-            *cp = __uint_as_float(r[j]) + (beta != 0.f ? beta * *cp : 0.f);
-          }
-        }
-    }
-  } else {  // K = 0: C = beta C
-    for (int idx = tid; idx < kTcBM * BN; idx += 128) {
-      const int m = m0 + idx / BN, n = n0 + idx % BN;
-      if (m < M && n < N) C[(long long)m * ldc + n] *= beta;
+    for (int c0 = 0; c0 < BN / 2; c0 += 8) {
+      uint32_t r[8];
+      const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(half + c0);
+      if (ns > 0) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(ta)
+                     : "memory");
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) r[q] = 0u;
+      }
+      if (lane < kRowsQ) {
+        *reinterpret_cast<uint4*>(tile + row * CF::kLd + half + c0) = make_uint4(r[0], r[1], r[2], r[3]);
+        *reinterpret_cast<uint4*>(tile + row * CF::kLd + half + c0 + 4) = make_uint4(r[4], r[5], r[6], r[7]);
+      }
     }
   }
   tcg::fence_before();
   __syncthreads();
   tcg::fence_after();
+  const bool ok = !fail && warp < 8;
+  // epilogue: four columns a thread
+  constexpr int QN = BN / 4, RPW = 32 / QN;  // quads per row; rows per warp step
+  const int quad = lane % QN, sub = lane / QN, n = n0 + 4 * quad;
+  double cs[4] = {0.0, 0.0, 0.0, 0.0};
+  if (ok) {
+    float bv[4] = {0.f, 0.f, 0.f, 0.f};
+    if (EPI == EPI_FWD && a.bias)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (n + q < a.N) bv[q] = a.bias[n + q];
+    const bool full = a.vec_c && n + 4 <= a.N;
+#pragma unroll 4
+    for (int r = warp * RPW + sub; r < BM; r += 8 * RPW) {
+      const int m = m0 + r;
+      if (m >= a.M || n >= a.N) continue;
+      const float4 t = *reinterpret_cast<const float4*>(tile + r * CF::kLd + 4 * quad);
+      float v[4] = {t.x, t.y, t.z, t.w};
+      const long long at = (long long)m * a.ldc + n;
+      if (EPI == EPI_PLAIN) {
+        if (full) {
+          if (a.beta != 0.f) {
+            const float4 c = *reinterpret_cast<const float4*>(a.C + at);
+            v[0] += a.beta * c.x;
+            v[1] += a.beta * c.y;
+            v[2] += a.beta * c.z;
+            v[3] += a.beta * c.w;
+          }
+          *reinterpret_cast<float4*>(a.C + at) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (n + q < a.N) a.C[at + q] = v[q] + (a.beta != 0.f ? a.beta * a.C[at + q] : 0.f);
+        }
+      } else if (EPI == EPI_FWD) {
+        float h[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          v[q] += bv[q];
+          h[q] = a.act ? v[q] / (1.f + expf(-v[q])) : v[q];
+        }
+        if (full) {
+          if (a.C) *reinterpret_cast<float4*>(a.C + at) = make_float4(v[0], v[1], v[2], v[3]);
+          if (a.h32) *reinterpret_cast<float4*>(a.h32 + at) = make_float4(h[0], h[1], h[2], h[3]);
+          if (a.h16) {
+            __nv_bfloat162 p[2] = {__floats2bfloat162_rn(h[0], h[1]), __floats2bfloat162_rn(h[2], h[3])};
+            *reinterpret_cast<uint2*>(a.h16 + at) = *reinterpret_cast<uint2*>(p);
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (n + q < a.N) {
+              if (a.C) a.C[at + q] = v[q];
+              if (a.h32) a.h32[at + q] = h[q];
+              if (a.h16) a.h16[at + q] = __float2bfloat16(h[q]);
+            }
+        }
+      } else {
+        float z[4] = {0.f, 0.f, 0.f, 0.f};
+        if (a.act) {
+          if (full) {
+            const float4 zz = *reinterpret_cast<const float4*>(a.z + at);
+            z[0] = zz.x;
+            z[1] = zz.y;
+            z[2] = zz.z;
+            z[3] = zz.w;
+          } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (n + q < a.N) z[q] = a.z[at + q];
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float sg = 1.f / (1.f + expf(-z[q]));
+            v[q] *= sg * (1.f + z[q] * (1.f - sg));
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cs[q] += (double)v[q];
+        if (full) {
+          __nv_bfloat162 p[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+          *reinterpret_cast<uint2*>(a.h16 + at) = *reinterpret_cast<uint2*>(p);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (n + q < a.N) a.h16[at + q] = __float2bfloat16(v[q]);
+        }
+      }
+    }
+    if (EPI == EPI_PLAIN && a.gb && blockIdx.x == 0)
+      for (int m = m0 + tid; m < min(a.M, m0 + BM); m += kTcThreads) {
+        double acc = 0.0;
+        for (int j = 0; j < a.n_parts; ++j) acc += a.bias_part[(long long)j * a.M + m];
+        a.gb[m] = (float)acc;
+      }
+  }
+  if (EPI == EPI_BWD) {  // column sums of this tile: warps and row lanes in a fixed order
+    double* sums = reinterpret_cast<double*>(smem + CF::kBody);
+    if (warp < 8)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) sums[(warp * RPW + sub) * BN + 4 * quad + q] = cs[q];
+    __syncthreads();
+    if (ok && tid < BN && n0 + tid < a.N) {
+      double acc = 0.0;
+#pragma unroll
+      for (int w = 0; w < 8 * RPW; ++w) acc += sums[w * BN + tid];
+      a.colpart[(long long)blockIdx.y * a.N + n0 + tid] = acc;
+    }
+  }
+  __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(CF::kCols) : "memory");
+}
+
+// How an operand with element (r, k) at P[r * sr + k * sk] is staged: 16-byte
+// copies along its contiguous direction where every copy starts 16-byte
+// aligned (the other stride a multiple of 8 values), else value by value.
+int load_mode(const void* P, long long sr, long long sk) {
+  const bool aligned = ((uintptr_t)P & 15) == 0;
+  if (aligned && sk == 1 && (sr & 7) == 0) return LD_K16;
+  if (aligned && sr == 1 && (sk & 7) == 0) return LD_MN16;
+  return LD_SCALAR;
+}
+
+template <class CF, int EPI>
+int launch_gemm(const GemmArgs& a, cudaStream_t st) {
+  auto* k = &k_gemm_tc<CF, EPI>;
+  const long long mt = (a.M + CF::BM - 1) / CF::BM;
+  if (mt > 65535) return set_error(FNE_EBOUNDS, "fne_gemm_bf16: M too large");
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, CF::kBytes);
+  if (e == cudaSuccess) {
+    k<<<dim3((a.N + CF::BN - 1) / CF::BN, (unsigned)mt), kTcThreads + 32, CF::kBytes, st>>>(a);
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) return set_error(FNE_ECUDA, std::string("k_gemm_tc: ") + cudaGetErrorString(e));
+  return FNE_OK;
+}
+
+// Tile choice.  Width: 32 for the network's narrow outputs; 128 once that
+// gives every SM a tile, else 64 (twice the CTAs, two per SM).  Plain products
+// that leave most SMs without a tile of 128 x 64 and are at least 1024 deep
+// take the long form (below that a tile's fixed cost outweighs the loop).
+template <int EPI>
+int run_gemm(GemmArgs& a, cudaStream_t st) {
+  const long long mt = (a.M + kTcBM - 1) / kTcBM;
+  a.mode_a = load_mode(a.A, a.sam, a.sak);
+  a.mode_b = load_mode(a.B, a.sbn, a.sbk);
+  if constexpr (EPI == EPI_PLAIN)
+    if (a.K >= 1024 && mt * ((a.N + 63) / 64) <= 148 / 4) return launch_gemm<GemmLong, EPI>(a, st);
+  if (a.N <= 32) return launch_gemm<GemmNarrow, EPI>(a, st);
+  if (mt * ((a.N + 127) / 128) < 148) return launch_gemm<GemmMid, EPI>(a, st);
+  return launch_gemm<GemmWide, EPI>(a, st);
 }
 
 // Z[n, m] += b[m]; H = silu(Z) (FP32 and BF16 copies); act = 0 leaves H = Z.
@@ -246,13 +599,41 @@ __global__ void k_act_bwd(long long n, const float* __restrict__ Z, const float*
   }
 }
 
-// out[m] = sum_n X[n, m] (bias gradient), one thread per column, fixed order.
-__global__ void k_colsum(long long rows, int cols, const float* __restrict__ X, float* __restrict__ out) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= cols) return;
+// out[m] = sum_n X[n, m] (bias gradient) in FP64, fixed order.  A cluster of 8
+// CTAs takes 32 columns: CTA r the r-th eighth of the rows, its 32 warps every
+// 32nd row each (128-byte reads); the warps' sums meet in shared memory, the
+// CTAs' in the distributed shared memory of rank 0.  (One thread per column
+// over all rows, as before, took 567 us for 8192 x 256 on the latency of its
+// serial loads.)
+constexpr int kSumCtas = 8;
+__global__ void __cluster_dims__(1, kSumCtas, 1) __launch_bounds__(1024)
+    k_colsum(long long rows, int cols, const float* __restrict__ X, float* __restrict__ out) {
+  __shared__ double s[32][33];
+  __shared__ double total[32];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = blockIdx.y;
+  const int m = blockIdx.x * 32 + lane;
+  const long long n1 = rows * (r + 1) / kSumCtas;
   double acc = 0.0;
-  for (long long n = 0; n < rows; ++n) acc += X[n * cols + m];
-  out[m] = (float)acc;
+  if (m < cols)
+#pragma unroll 8
+    for (long long n = rows * r / kSumCtas + w; n < n1; n += 32) acc += (double)__ldg(X + n * cols + m);
+  s[w][lane] = acc;
+  __syncthreads();
+  if (w == 0) {
+    acc = 0.0;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) acc += s[j][lane];
+    total[lane] = acc;
+  }
+  cluster.sync();
+  if (r == 0 && w == 0) {
+    acc = 0.0;
+#pragma unroll
+    for (int j = 0; j < kSumCtas; ++j) acc += cluster.map_shared_rank(total, j)[lane];
+    if (m < cols) out[m] = (float)acc;
+  }
+  cluster.sync();
 }
 
 // Adam on FP32 master weights; refreshes the BF16 copy used by the GEMMs.
@@ -314,17 +695,22 @@ extern "C" int fne_gemm_bf16(int M, int N, int K, const void* A, int64_t sam, in
       (K * (int64_t)N > 0 && !B))
     return set_error(FNE_EINVAL, "fne_gemm_bf16: bad arguments");
   if (M == 0 || N == 0) return FNE_OK;
-  const int bn = N <= 32 ? 32 : 128;
-  const dim3 grid((N + bn - 1) / bn, (M + kTcBM - 1) / kTcBM);
-  if (grid.y > 65535) return set_error(FNE_EBOUNDS, "fne_gemm_bf16: M too large");
-  const long long lim = g_gemm_wait_limit;
-  if (bn == 32)
-    k_gemm_tc<32><<<grid, 128, 0, (cudaStream_t)stream>>>(M, N, K, (const __nv_bfloat16*)A, sam, sak,
-                                                          (const __nv_bfloat16*)B, sbk, sbn, C, ldc, beta, lim);
-  else
-    k_gemm_tc<128><<<grid, 128, 0, (cudaStream_t)stream>>>(M, N, K, (const __nv_bfloat16*)A, sam, sak,
-                                                           (const __nv_bfloat16*)B, sbk, sbn, C, ldc, beta, lim);
-  return launch_status("fne_gemm_bf16");
+  GemmArgs a = {};
+  a.M = M;
+  a.N = N;
+  a.K = K;
+  a.A = (const __nv_bfloat16*)A;
+  a.sam = sam;
+  a.sak = sak;
+  a.B = (const __nv_bfloat16*)B;
+  a.sbk = sbk;
+  a.sbn = sbn;
+  a.C = C;
+  a.ldc = ldc;
+  a.beta = beta;
+  a.vec_c = ((uintptr_t)C & 15) == 0 && (ldc & 3) == 0;
+  a.wait_limit = g_gemm_wait_limit;
+  return run_gemm<EPI_PLAIN>(a, (cudaStream_t)stream);
 }
 
 extern "C" int fne_mlp_bias_act(int64_t rows, int cols, float* Z, const float* bias, int act, float* H32, void* H16,
@@ -347,7 +733,7 @@ extern "C" int fne_mlp_act_bwd(int64_t n, const float* Z, const float* dH, int a
 
 extern "C" int fne_mlp_colsum(int64_t rows, int cols, const float* X, float* out, void* stream) {
   if (rows < 0 || cols <= 0 || !X || !out) return set_error(FNE_EINVAL, "fne_mlp_colsum: bad arguments");
-  k_colsum<<<(cols + 127) / 128, 128, 0, (cudaStream_t)stream>>>(rows, cols, X, out);
+  k_colsum<<<dim3((cols + 31) / 32, kSumCtas), 1024, 0, (cudaStream_t)stream>>>(rows, cols, X, out);
   return launch_status("fne_mlp_colsum");
 }
 
