@@ -1,21 +1,16 @@
 // Kernels of the learned Newton warm start: a small MLP over nodal features
 // (BF16 weights and activations, FP32 accumulation and master weights).
 //
-//  * k_gemm_tc: C[M x N] (FP32) = op(A)[M x K] * op(B)[K x N] (+ beta * C) on
-//    the 5th-generation tensor cores: tcgen05.mma kind::f16 with BF16
-//    operands and an FP32 accumulator in tensor memory (TMEM).  One CTA per
-//    128 x BN tile of C (BN = 32 or 128); the 128 threads stage each 64-deep K
-//    slice of A and B into shared memory in the no-swizzle K-major
-//    core-matrix layout (8 rows x 16 bytes; zero-filled at the edges; eight
-//    values per load where an operand's K direction is contiguous), one
-//    thread issues the four K = 16 MMAs of the slice and commits them to an
-//    mbarrier (bounded wait), and the epilogue reads the accumulator back
-//    with tcgen05.ld (each warp its 32-lane quadrant).  Operands are
-//    addressed through (row, col) strides, so one kernel covers the forward
-//    product H W^T, the weight gradient dZ^T H and the input gradient dZ W
-//    without explicit transposes.
-//  * k_bias_silu_fwd, k_silu_bwd, k_colsum, k_adam, k_cast: elementwise work
-//    of the forward / backward pass and the optimiser.
+//  * k_gemm_tc: op(A)[M x K] * op(B)[K x N] on the 5th-generation tensor
+//    cores (tcgen05.mma kind::f16, BF16 operands, FP32 accumulator in TMEM)
+//    with the layer's elementwise work in its epilogue: bias + SiLU forward,
+//    SiLU derivative + column sums backward, a plain C = A B + beta C for the
+//    weight gradient and for fne_gemm_bf16.  Operands are addressed through
+//    (row, col) strides, so one kernel covers the forward product H W^T, the
+//    weight gradient dZ^T H and the input gradient dZ W without explicit
+//    transposes.
+//  * k_bias_act_fwd, k_act_bwd, k_colsum, k_adam, k_adam_set, k_cast_bf16:
+//    the elementwise pieces on their own, and the optimiser.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -652,6 +647,36 @@ __global__ void k_adam(long long n, float* __restrict__ p, const float* __restri
   }
 }
 
+// The same update over up to kAdamMax tensors in one launch (a step of the
+// network touches eight, the largest 65,536 values: alone each launch is its
+// own latency).
+constexpr int kAdamMax = 32;
+struct AdamSet {
+  long long end[kAdamMax];  // running total of the sizes
+  float* p[kAdamMax];
+  const float* g[kAdamMax];
+  float* m[kAdamMax];
+  float* v[kAdamMax];
+  __nv_bfloat16* p16[kAdamMax];
+  int count;
+};
+__global__ void k_adam_set(const AdamSet T, float lr, float b1, float b2, float eps, float c1, float c2) {
+  const long long n = T.end[T.count - 1];
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+    int t = 0;
+    while (k >= T.end[t]) ++t;
+    const long long i = k - (t ? T.end[t - 1] : 0);
+    const float gi = T.g[t][i];
+    const float mi = b1 * T.m[t][i] + (1.f - b1) * gi;
+    const float vi = b2 * T.v[t][i] + (1.f - b2) * gi * gi;
+    T.m[t][i] = mi;
+    T.v[t][i] = vi;
+    const float pi = T.p[t][i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    T.p[t][i] = pi;
+    if (T.p16[t]) T.p16[t][i] = __float2bfloat16(pi);
+  }
+}
+
 __global__ void k_cast_bf16(long long n, const float* __restrict__ x, __nv_bfloat16* __restrict__ y) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     y[i] = __float2bfloat16(x[i]);
@@ -713,6 +738,85 @@ extern "C" int fne_gemm_bf16(int M, int N, int K, const void* A, int64_t sam, in
   return run_gemm<EPI_PLAIN>(a, (cudaStream_t)stream);
 }
 
+namespace {
+bool aligned(const void* p, uintptr_t to) { return ((uintptr_t)p & (to - 1)) == 0; }
+}  // namespace
+
+extern "C" int fne_mlp_linear_fwd(int rows, int din, int dout, const void* X16, const void* W16, const float* bias,
+                                  int act, float* Z, float* H32, void* H16, void* stream) {
+  if (rows < 0 || din <= 0 || dout <= 0 || (rows > 0 && (!X16 || !W16)))
+    return set_error(FNE_EINVAL, "fne_mlp_linear_fwd: bad arguments");
+  if (rows == 0) return FNE_OK;
+  GemmArgs a = {};
+  a.M = rows;
+  a.N = dout;
+  a.K = din;
+  a.A = (const __nv_bfloat16*)X16;
+  a.sam = din;
+  a.sak = 1;
+  a.B = (const __nv_bfloat16*)W16;
+  a.sbk = 1;
+  a.sbn = din;
+  a.C = Z;
+  a.ldc = dout;
+  a.bias = bias;
+  a.act = act;
+  a.h32 = H32;
+  a.h16 = (__nv_bfloat16*)H16;
+  a.vec_c = (dout & 3) == 0 && aligned(Z, 16) && aligned(H32, 16) && aligned(H16, 8);
+  a.wait_limit = g_gemm_wait_limit;
+  return run_gemm<EPI_FWD>(a, (cudaStream_t)stream);
+}
+
+extern "C" int fne_mlp_linear_bwd_data(int rows, int din, int dout, const void* dZ16, const void* W16,
+                                       const float* Zin, int act, void* dZin16, double* colpart, void* stream) {
+  if (rows < 0 || din <= 0 || dout <= 0 || (rows > 0 && (!dZ16 || !W16 || !dZin16 || !colpart || (act && !Zin))))
+    return set_error(FNE_EINVAL, "fne_mlp_linear_bwd_data: bad arguments");
+  if (rows == 0) return FNE_OK;
+  GemmArgs a = {};
+  a.M = rows;
+  a.N = din;
+  a.K = dout;
+  a.A = (const __nv_bfloat16*)dZ16;
+  a.sam = dout;
+  a.sak = 1;
+  a.B = (const __nv_bfloat16*)W16;
+  a.sbk = din;
+  a.sbn = 1;
+  a.ldc = din;
+  a.act = act;
+  a.z = Zin;
+  a.h16 = (__nv_bfloat16*)dZin16;
+  a.colpart = colpart;
+  a.vec_c = (din & 3) == 0 && aligned(Zin, 16) && aligned(dZin16, 8);
+  a.wait_limit = g_gemm_wait_limit;
+  return run_gemm<EPI_BWD>(a, (cudaStream_t)stream);
+}
+
+extern "C" int fne_mlp_linear_bwd_weight(int rows, int din, int dout, const void* dZ16, const void* X16, float* gW,
+                                         const double* colpart, float* gb, void* stream) {
+  if (rows < 0 || din <= 0 || dout <= 0 || !gW || (rows > 0 && (!dZ16 || !X16)) || ((gb != nullptr) != (colpart != nullptr)))
+    return set_error(FNE_EINVAL, "fne_mlp_linear_bwd_weight: bad arguments");
+  GemmArgs a = {};
+  a.M = dout;
+  a.N = din;
+  a.K = rows;
+  a.A = (const __nv_bfloat16*)dZ16;
+  a.sam = 1;
+  a.sak = dout;
+  a.B = (const __nv_bfloat16*)X16;
+  a.sbk = din;
+  a.sbn = 1;
+  a.C = gW;
+  a.ldc = din;
+  a.vec_c = (din & 3) == 0 && aligned(gW, 16);
+  a.bias_part = colpart;
+  a.n_parts = (rows + kTcBM - 1) / kTcBM;
+  a.gb = gb;
+  a.wait_limit = g_gemm_wait_limit;
+  return run_gemm<EPI_PLAIN>(a, (cudaStream_t)stream);
+}
+
 extern "C" int fne_mlp_bias_act(int64_t rows, int cols, float* Z, const float* bias, int act, float* H32, void* H16,
                                 void* stream) {
   if (rows < 0 || cols <= 0 || !Z) return set_error(FNE_EINVAL, "fne_mlp_bias_act: bad arguments");
@@ -745,6 +849,36 @@ extern "C" int fne_mlp_adam(int64_t n, float* p, const float* g, float* m, float
   k_adam<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(n, p, g, m, v, lr, b1, b2, eps, c1, c2,
                                                           (__nv_bfloat16*)p16);
   return launch_status("fne_mlp_adam");
+}
+
+extern "C" int fne_mlp_adam_set(int count, const int64_t* n, float* const* p, const float* const* g, float* const* m,
+                                float* const* v, void* const* p16, float lr, float b1, float b2, float eps, int step,
+                                void* stream) {
+  if (count < 0 || step < 1 || (count > 0 && (!n || !p || !g || !m || !v || !p16)))
+    return set_error(FNE_EINVAL, "fne_mlp_adam_set: bad arguments");
+  const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
+  for (int k = 0; k < count; ++k)
+    if (n[k] < 0 || (n[k] > 0 && (!p[k] || !g[k] || !m[k] || !v[k])))
+      return set_error(FNE_EINVAL, "fne_mlp_adam_set: bad arguments");
+  for (int k0 = 0; k0 < count; k0 += kAdamMax) {
+    AdamSet T = {};
+    T.count = std::min(kAdamMax, count - k0);
+    long long total = 0;
+    for (int k = 0; k < T.count; ++k) {
+      total += n[k0 + k];
+      T.end[k] = total;
+      T.p[k] = p[k0 + k];
+      T.g[k] = g[k0 + k];
+      T.m[k] = m[k0 + k];
+      T.v[k] = v[k0 + k];
+      T.p16[k] = (__nv_bfloat16*)p16[k0 + k];
+    }
+    if (total == 0) continue;
+    k_adam_set<<<grid_for(total), 256, 0, (cudaStream_t)stream>>>(T, lr, b1, b2, eps, c1, c2);
+    const int rc = launch_status("fne_mlp_adam_set");
+    if (rc != FNE_OK) return rc;
+  }
+  return FNE_OK;
 }
 
 extern "C" int fne_mlp_cast_bf16(int64_t n, const float* x, void* y, void* stream) {

@@ -11,6 +11,7 @@ start, otherwise the plain start is used (``run_load_path``).
 
 from __future__ import annotations
 
+import ctypes
 import math
 import time
 
@@ -63,20 +64,20 @@ class NodalMLP:
         h16 = X16
         saved = []
         out = None
+        st = _stream()
         for l in range(self.n_layers):
             din, dout = self.dims[l], self.dims[l + 1]
-            Z = torch.empty(N, dout, dtype=torch.float32, device=X16.device)
-            gemm(h16, din, 1, self.W16[l], 1, din, N, dout, din, Z)
             last = l == self.n_layers - 1
+            # the pre-activation is kept for backward; a prediction never writes it
+            Z = torch.empty(N, dout, dtype=torch.float32, device=X16.device) if keep and not last else None
             if last:
-                out = torch.empty_like(Z)
-                check(lib.fne_mlp_bias_act(N, dout, Z.data_ptr(), self.b[l].data_ptr(), 0, out.data_ptr(), None,
-                                           _stream()))
+                out = torch.empty(N, dout, dtype=torch.float32, device=X16.device)
             else:
                 nxt = torch.empty(N, dout, dtype=BF16, device=X16.device)
-                check(lib.fne_mlp_bias_act(N, dout, Z.data_ptr(), self.b[l].data_ptr(), 1, None, nxt.data_ptr(),
-                                           _stream()))
-            self.kernel_launches += 2
+            check(lib.fne_mlp_linear_fwd(N, din, dout, h16.data_ptr(), self.W16[l].data_ptr(), self.b[l].data_ptr(),
+                                         0 if last else 1, Z.data_ptr() if Z is not None else None,
+                                         out.data_ptr() if last else None, None if last else nxt.data_ptr(), st))
+            self.kernel_launches += 1
             if keep:
                 saved.append((h16, Z))
             if not last:
@@ -88,37 +89,45 @@ class NodalMLP:
     # -- backward ------------------------------------------------------------
     def backward(self, dY):
         """Gradients of the parameters for ``dL/dY = dY`` (FP32, shape (N, d_out))."""
-        N = dY.shape[0]
+        N, dev, st = dY.shape[0], dY.device, _stream()
         gW, gb = [None] * self.n_layers, [None] * self.n_layers
-        dH = dY.contiguous()
+        dY = dY.contiguous()
+        l = self.n_layers - 1
+        dZ16 = torch.empty(dY.shape, dtype=BF16, device=dev)
+        gb[l] = torch.empty(self.dims[-1], dtype=torch.float32, device=dev)
+        check(lib.fne_mlp_cast_bf16(dY.numel(), dY.data_ptr(), dZ16.data_ptr(), st))
+        check(lib.fne_mlp_colsum(N, self.dims[-1], dY.data_ptr(), gb[l].data_ptr(), st))
+        self.kernel_launches += 2
+        part = None  # column sums of dZ16's FP32 values, per 128 rows
         for l in reversed(range(self.n_layers)):
             din, dout = self.dims[l], self.dims[l + 1]
-            h16, Z = self._saved[l]
-            act = 0 if l == self.n_layers - 1 else 1
-            dZ32 = torch.empty(N, dout, dtype=torch.float32, device=dY.device)
-            dZ16 = torch.empty(N, dout, dtype=BF16, device=dY.device)
-            check(lib.fne_mlp_act_bwd(N * dout, Z.data_ptr(), dH.data_ptr(), act, dZ32.data_ptr(), dZ16.data_ptr(),
-                                      _stream()))
-            gW[l] = torch.empty(dout, din, dtype=torch.float32, device=dY.device)
-            gemm(dZ16, 1, dout, h16, din, 1, dout, din, N, gW[l])            # dZ^T H
-            gb[l] = torch.empty(dout, dtype=torch.float32, device=dY.device)
-            check(lib.fne_mlp_colsum(N, dout, dZ32.data_ptr(), gb[l].data_ptr(), _stream()))
-            self.kernel_launches += 3
+            h16, _ = self._saved[l]
+            gW[l] = torch.empty(dout, din, dtype=torch.float32, device=dev)
+            if gb[l] is None:
+                gb[l] = torch.empty(dout, dtype=torch.float32, device=dev)
+            check(lib.fne_mlp_linear_bwd_weight(N, din, dout, dZ16.data_ptr(), h16.data_ptr(), gW[l].data_ptr(),
+                                                part.data_ptr() if part is not None else None,
+                                                gb[l].data_ptr() if part is not None else None, st))
+            self.kernel_launches += 1
             if l > 0:
-                dH = torch.empty(N, din, dtype=torch.float32, device=dY.device)
-                gemm(dZ16, dout, 1, self.W16[l], din, 1, N, din, dout, dH)   # dZ W
+                nxt = torch.empty(N, din, dtype=BF16, device=dev)
+                part = torch.empty(-(-N // 128), din, dtype=torch.float64, device=dev)
+                check(lib.fne_mlp_linear_bwd_data(N, din, dout, dZ16.data_ptr(), self.W16[l].data_ptr(),
+                                                  self._saved[l - 1][1].data_ptr(), 1, nxt.data_ptr(),
+                                                  part.data_ptr(), st))
+                dZ16 = nxt
                 self.kernel_launches += 1
         return gW, gb
 
     def adam_step(self, gW, gb, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         self.step += 1
-        params = self.W + self.b
-        grads = gW + gb
-        for i, (p, g) in enumerate(zip(params, grads)):
-            p16 = self.W16[i] if i < self.n_layers else None
-            check(lib.fne_mlp_adam(p.numel(), p.data_ptr(), g.data_ptr(), self.m[i].data_ptr(), self.v[i].data_ptr(),
-                                   lr, b1, b2, eps, self.step, p16.data_ptr() if p16 is not None else None, _stream()))
-            self.kernel_launches += 1
+        params, grads = self.W + self.b, gW + gb
+        k = len(params)
+        sizes = (ctypes.c_int64 * k)(*(p.numel() for p in params))
+        ptrs = [(ctypes.c_void_p * k)(*(t.data_ptr() for t in ts)) for ts in (params, grads, self.m, self.v)]
+        p16 = (ctypes.c_void_p * k)(*([w.data_ptr() for w in self.W16] + [None] * len(self.b)))
+        check(lib.fne_mlp_adam_set(k, sizes, *ptrs, p16, lr, b1, b2, eps, self.step, _stream()))
+        self.kernel_launches += 1
 
     def state(self):
         return {"dims": self.dims, "W": [w.cpu() for w in self.W], "b": [b.cpu() for b in self.b]}

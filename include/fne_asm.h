@@ -369,6 +369,23 @@ int fne_gemm_set_wait_limit(int64_t polls);
 /* Z += bias (per column); H = silu(Z) (act = 1) or Z (act = 0); H32 / H16 may be NULL. */
 int fne_mlp_bias_act(int64_t rows, int cols, float* Z, const float* bias, int act, float* H32, void* H16,
                      void* stream);
+/* One layer forward: z = X W^T + bias (X [rows][din], W [dout][din] BF16, bias
+ * may be NULL); Z = z, H32 / H16 = silu(z) (act = 1) or z (act = 0).  Z, H32 and
+ * H16 may each be NULL.  The values are those of fne_gemm_bf16 followed by
+ * fne_mlp_bias_act; one launch, same bounded waits and status. */
+int fne_mlp_linear_fwd(int rows, int din, int dout, const void* X16, const void* W16, const float* bias, int act,
+                       float* Z, float* H32, void* H16, void* stream);
+/* One layer's input gradient: d = dZ W (dZ [rows][dout], W [dout][din] BF16), times
+ * silu'(Zin) when act = 1 (Zin [rows][din]: the previous layer's z); dZin16 = d in
+ * BF16; colpart [ceil(rows / 128)][din] = sums of d over each 128 rows (FP64,
+ * fixed order), which fne_mlp_linear_bwd_weight turns into the bias gradient. */
+int fne_mlp_linear_bwd_data(int rows, int din, int dout, const void* dZ16, const void* W16, const float* Zin, int act,
+                            void* dZin16, double* colpart, void* stream);
+/* One layer's weight gradient: gW [dout][din] = dZ^T X; with colpart (from the call
+ * that produced dZ, [ceil(rows / 128)][dout]) also gb [dout], its column sums.
+ * colpart and gb are both NULL or both given. */
+int fne_mlp_linear_bwd_weight(int rows, int din, int dout, const void* dZ16, const void* X16, float* gW,
+                              const double* colpart, float* gb, void* stream);
 /* dZ = dH * silu'(Z) (act = 1) or dH (act = 0); dZ32 / dZ16 may be NULL. */
 int fne_mlp_act_bwd(int64_t n, const float* Z, const float* dH, int act, float* dZ32, void* dZ16, void* stream);
 /* out[c] = sum_r X[r, c] (FP64 accumulation, fixed order). */
@@ -377,6 +394,10 @@ int fne_mlp_colsum(int64_t rows, int cols, const float* X, float* out, void* str
  * writes the BF16 copy p16 when it is not NULL. */
 int fne_mlp_adam(int64_t n, float* p, const float* g, float* m, float* v, float lr, float b1, float b2, float eps,
                  int step, void* p16, void* stream);
+/* The same Adam step on ``count`` tensors (host arrays of sizes and device pointers;
+ * p16[k] may be NULL) in one launch per 32 tensors. */
+int fne_mlp_adam_set(int count, const int64_t* n, float* const* p, const float* const* g, float* const* m,
+                     float* const* v, void* const* p16, float lr, float b1, float b2, float eps, int step, void* stream);
 int fne_mlp_cast_bf16(int64_t n, const float* x, void* y, void* stream);
 
 const char* fne_last_error(void);

@@ -129,3 +129,46 @@ def test_learned_warm_start_cuts_newton_iterations():
     t = res["test"]
     assert t["accepted_steps"] >= t["steps"] - 1
     assert t["learned_newton_its"] <= 0.85 * t["plain_newton_its"], t
+
+
+@pytest.mark.parametrize("rows", [1, 127, 129, 1300])
+@pytest.mark.parametrize("din,dout", [(12, 64), (64, 3), (40, 33), (72, 200)])
+def test_fused_layer_edges(rows, din, dout):
+    """One layer's fused forward, input gradient and weight gradient at the edges of
+    their tiles (rows 128, columns 32 / 64, depth 64 / 128; 1300 rows take the long
+    product) and with unaligned row pitches, against float64 products of the same
+    BF16 operands: FP32 accumulation (1e-5 of the largest entry, as for the plain
+    product) and one BF16 rounding (2^-8 relative)."""
+    from fenics_nonlinear_energies_b200 import _lib
+
+    L, vp = _lib.lib, lambda t: t.data_ptr()  # noqa: E731
+    f32 = {"dtype": torch.float32}  # the oracle sets float64 as torch's default
+    g = torch.Generator().manual_seed(rows * 1000 + din + dout)
+    X = torch.randn(rows, din, generator=g).to(torch.bfloat16).cuda()
+    W = (torch.randn(dout, din, generator=g) / din ** 0.5).to(torch.bfloat16).cuda()
+    b = torch.randn(dout, generator=g, **f32).cuda()
+    Z = torch.empty(rows, dout, device="cuda", **f32)
+    H = torch.empty(rows, dout, dtype=torch.bfloat16, device="cuda")
+    _lib.check(L.fne_mlp_linear_fwd(rows, din, dout, vp(X), vp(W), vp(b), 1, vp(Z), None, vp(H), None))
+    ref = X.double() @ W.double().T + b.double()
+    assert (Z.double() - ref).abs().max() <= 1e-5 * ref.abs().max() + 1e-5
+    silu = torch.nn.functional.silu(Z.double())
+    assert ((H.double() - silu).abs() <= 2.0 ** -8 * silu.abs() + 1e-6).all()
+
+    dZ = torch.randn(rows, dout, generator=g).to(torch.bfloat16).cuda()
+    Zin = torch.randn(rows, din, generator=g, **f32).cuda()
+    dIn = torch.empty(rows, din, dtype=torch.bfloat16, device="cuda")
+    part = torch.empty(-(-rows // 128), din, dtype=torch.float64, device="cuda")
+    _lib.check(L.fne_mlp_linear_bwd_data(rows, din, dout, vp(dZ), vp(W), vp(Zin), 1, vp(dIn), vp(part), None))
+    s = torch.sigmoid(Zin.double())
+    ref = (dZ.double() @ W.double()) * (s * (1 + Zin.double() * (1 - s)))
+    assert ((dIn.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * ref.abs().max() + 1e-5).all()
+    assert (part.sum(0) - ref.sum(0)).abs().max() <= 1e-5 * ref.abs().sum(0).max()
+
+    gW = torch.empty(din, dout, device="cuda", **f32)  # gradient of a layer dout -> din whose dZ is dIn
+    gb = torch.empty(din, device="cuda", **f32)
+    _lib.check(L.fne_mlp_linear_bwd_weight(rows, dout, din, vp(dIn), vp(dZ), vp(gW), vp(part), vp(gb), None))
+    ref = dIn.double().T @ dZ.double()
+    assert (gW.double() - ref).abs().max() <= 1e-5 * ref.abs().max() + 1e-5
+    assert (gb.double() - part.sum(0)).abs().max() <= 1e-6 * part.sum(0).abs().max() + 1e-6
+    _lib.check(L.fne_gemm_check_status())
