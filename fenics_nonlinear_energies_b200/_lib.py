@@ -109,8 +109,10 @@ def _load():
         "fne_mlp_adam": (C.c_int, [C.c_int64, vp, vp, vp, vp, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int,
                                    vp, vp]),
         "fne_mlp_linear_fwd": (C.c_int, [C.c_int, C.c_int, C.c_int, vp, vp, vp, C.c_int, vp, vp, vp, vp]),
-        "fne_mlp_linear_bwd_data": (C.c_int, [C.c_int, C.c_int, C.c_int, vp, vp, vp, C.c_int, vp, vp, vp]),
-        "fne_mlp_linear_bwd_weight": (C.c_int, [C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, vp, vp]),
+        "fne_mlp_linear_bwd_data": (C.c_int, [C.c_int, C.c_int, C.c_int, vp, C.c_int, vp, vp, C.c_int, vp, vp, vp]),
+        "fne_mlp_linear_bwd_weight": (C.c_int, [C.c_int, C.c_int, C.c_int, vp, C.c_int, vp, C.c_int, vp, vp, vp,
+                                                vp]),
+        "fne_mlp_pad_rows": (C.c_int, [C.c_int64, C.c_int, vp, C.c_int, C.c_int, vp, vp]),
         "fne_mlp_adam_set": (C.c_int, [C.c_int, vp, vp, vp, vp, vp, vp, C.c_float, C.c_float, C.c_float, C.c_float,
                                        C.c_int, vp]),
         "fne_mlp_cast_bf16": (C.c_int, [C.c_int64, vp, vp, vp]),

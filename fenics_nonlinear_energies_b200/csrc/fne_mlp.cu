@@ -129,6 +129,7 @@ struct GemmArgs {
   const __nv_bfloat16* B;
   long long sbk, sbn;
   int mode_a, mode_b;
+  int ra, rb;  // M / N extents that may be read (an M/N-contiguous operand's padded pitch); 0: M, N
   float* C;  // EPI_PLAIN: C = A B + beta C; EPI_FWD: the pre-activation (may be null); [M][ldc]
   long long ldc;
   float beta;
@@ -332,8 +333,8 @@ __global__ void __launch_bounds__(kTcThreads + 32) k_gemm_tc(const GemmArgs a) {
   if (warp < 8) {
     OpA oa;
     OpB ob;
-    oa.init(a.A, a.sam, a.sak, a.mode_a, m0, a.M);
-    ob.init(a.B, a.sbn, a.sbk, a.mode_b, n0, a.N);
+    oa.init(a.A, a.sam, a.sak, a.mode_a, m0, a.ra);
+    ob.init(a.B, a.sbn, a.sbk, a.mode_b, n0, a.rb);
     for (int i = 0; i < ns; ++i) {
       if (i >= NST && !tcg::mbar_wait(tcg::saddr(&s_empty[i % NST]), ((i / NST) - 1) & 1, a.wait_limit, &s_fail)) {
         fail = 1;
@@ -559,6 +560,8 @@ int run_gemm(GemmArgs& a, cudaStream_t st) {
   const long long mt = (a.M + kTcBM - 1) / kTcBM;
   a.mode_a = load_mode(a.A, a.sam, a.sak);
   a.mode_b = load_mode(a.B, a.sbn, a.sbk);
+  if (a.ra < a.M) a.ra = a.M;
+  if (a.rb < a.N) a.rb = a.N;
   if constexpr (EPI == EPI_PLAIN)
     if (a.K >= 1024 && mt * ((a.N + 63) / 64) <= 148 / 4) return launch_gemm<GemmLong, EPI>(a, st);
   if (a.N <= 32) return launch_gemm<GemmNarrow, EPI>(a, st);
@@ -677,6 +680,18 @@ __global__ void k_adam_set(const AdamSet T, float lr, float b1, float b2, float 
   }
 }
 
+// Rows of `cols` values (FP32 or BF16) as BF16 rows of pitch `pitch`, zeros behind them.
+template <typename T>
+__global__ void k_pad_rows(long long rows, int cols, const T* __restrict__ x, int pitch,
+                           __nv_bfloat16* __restrict__ y) {
+  const long long n = rows * pitch;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const long long r = i / pitch;
+    const int c = (int)(i - r * pitch);
+    y[i] = c < cols ? static_cast<__nv_bfloat16>(x[r * cols + c]) : __float2bfloat16(0.f);
+  }
+}
+
 __global__ void k_cast_bf16(long long n, const float* __restrict__ x, __nv_bfloat16* __restrict__ y) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     y[i] = __float2bfloat16(x[i]);
@@ -768,9 +783,21 @@ extern "C" int fne_mlp_linear_fwd(int rows, int din, int dout, const void* X16, 
   return run_gemm<EPI_FWD>(a, (cudaStream_t)stream);
 }
 
-extern "C" int fne_mlp_linear_bwd_data(int rows, int din, int dout, const void* dZ16, const void* W16,
+extern "C" int fne_mlp_pad_rows(int64_t rows, int cols, const void* x, int x_fp32, int pitch, void* y, void* stream) {
+  if (rows < 0 || cols <= 0 || pitch < cols || (rows > 0 && (!x || !y)))
+    return set_error(FNE_EINVAL, "fne_mlp_pad_rows: bad arguments");
+  if (rows == 0) return FNE_OK;
+  const int grid = grid_for(rows * (long long)pitch);
+  if (x_fp32)
+    k_pad_rows<<<grid, 256, 0, (cudaStream_t)stream>>>(rows, cols, (const float*)x, pitch, (__nv_bfloat16*)y);
+  else
+    k_pad_rows<<<grid, 256, 0, (cudaStream_t)stream>>>(rows, cols, (const __nv_bfloat16*)x, pitch, (__nv_bfloat16*)y);
+  return launch_status("fne_mlp_pad_rows");
+}
+
+extern "C" int fne_mlp_linear_bwd_data(int rows, int din, int dout, const void* dZ16, int ldz, const void* W16,
                                        const float* Zin, int act, void* dZin16, double* colpart, void* stream) {
-  if (rows < 0 || din <= 0 || dout <= 0 || (rows > 0 && (!dZ16 || !W16 || !dZin16 || !colpart || (act && !Zin))))
+  if (rows < 0 || din <= 0 || dout <= 0 || ldz < dout || (rows > 0 && (!dZ16 || !W16 || !dZin16 || !colpart || (act && !Zin))))
     return set_error(FNE_EINVAL, "fne_mlp_linear_bwd_data: bad arguments");
   if (rows == 0) return FNE_OK;
   GemmArgs a = {};
@@ -778,7 +805,7 @@ extern "C" int fne_mlp_linear_bwd_data(int rows, int din, int dout, const void* 
   a.N = din;
   a.K = dout;
   a.A = (const __nv_bfloat16*)dZ16;
-  a.sam = dout;
+  a.sam = ldz;
   a.sak = 1;
   a.B = (const __nv_bfloat16*)W16;
   a.sbk = din;
@@ -793,9 +820,9 @@ extern "C" int fne_mlp_linear_bwd_data(int rows, int din, int dout, const void* 
   return run_gemm<EPI_BWD>(a, (cudaStream_t)stream);
 }
 
-extern "C" int fne_mlp_linear_bwd_weight(int rows, int din, int dout, const void* dZ16, const void* X16, float* gW,
-                                         const double* colpart, float* gb, void* stream) {
-  if (rows < 0 || din <= 0 || dout <= 0 || !gW || (rows > 0 && (!dZ16 || !X16)) || ((gb != nullptr) != (colpart != nullptr)))
+extern "C" int fne_mlp_linear_bwd_weight(int rows, int din, int dout, const void* dZ16, int ldz, const void* X16,
+                                         int ldx, float* gW, const double* colpart, float* gb, void* stream) {
+  if (rows < 0 || din <= 0 || dout <= 0 || ldz < dout || ldx < din || !gW || (rows > 0 && (!dZ16 || !X16)) || ((gb != nullptr) != (colpart != nullptr)))
     return set_error(FNE_EINVAL, "fne_mlp_linear_bwd_weight: bad arguments");
   GemmArgs a = {};
   a.M = dout;
@@ -803,10 +830,12 @@ extern "C" int fne_mlp_linear_bwd_weight(int rows, int din, int dout, const void
   a.K = rows;
   a.A = (const __nv_bfloat16*)dZ16;
   a.sam = 1;
-  a.sak = dout;
+  a.sak = ldz;
+  a.ra = ldz;
   a.B = (const __nv_bfloat16*)X16;
-  a.sbk = din;
+  a.sbk = ldx;
   a.sbn = 1;
+  a.rb = ldx;
   a.C = gW;
   a.ldc = din;
   a.vec_c = (din & 3) == 0 && aligned(gW, 16);

@@ -93,29 +93,37 @@ class NodalMLP:
         gW, gb = [None] * self.n_layers, [None] * self.n_layers
         dY = dY.contiguous()
         l = self.n_layers - 1
-        dZ16 = torch.empty(dY.shape, dtype=BF16, device=dev)
+        # operands of odd width (3 outputs, 12 features) in rows of a pitch the GEMM reads 16 bytes at a time
+        ldz = -(-self.dims[-1] // 8) * 8
+        dZ16 = torch.empty(N, ldz, dtype=BF16, device=dev)
         gb[l] = torch.empty(self.dims[-1], dtype=torch.float32, device=dev)
-        check(lib.fne_mlp_cast_bf16(dY.numel(), dY.data_ptr(), dZ16.data_ptr(), st))
+        check(lib.fne_mlp_pad_rows(N, self.dims[-1], dY.data_ptr(), 1, ldz, dZ16.data_ptr(), st))
         check(lib.fne_mlp_colsum(N, self.dims[-1], dY.data_ptr(), gb[l].data_ptr(), st))
         self.kernel_launches += 2
         part = None  # column sums of dZ16's FP32 values, per 128 rows
         for l in reversed(range(self.n_layers)):
             din, dout = self.dims[l], self.dims[l + 1]
             h16, _ = self._saved[l]
+            ldx = -(-din // 8) * 8
+            if ldx != din:
+                padded = torch.empty(N, ldx, dtype=BF16, device=dev)
+                check(lib.fne_mlp_pad_rows(N, din, h16.data_ptr(), 0, ldx, padded.data_ptr(), st))
+                h16 = padded
+                self.kernel_launches += 1
             gW[l] = torch.empty(dout, din, dtype=torch.float32, device=dev)
             if gb[l] is None:
                 gb[l] = torch.empty(dout, dtype=torch.float32, device=dev)
-            check(lib.fne_mlp_linear_bwd_weight(N, din, dout, dZ16.data_ptr(), h16.data_ptr(), gW[l].data_ptr(),
+            check(lib.fne_mlp_linear_bwd_weight(N, din, dout, dZ16.data_ptr(), ldz, h16.data_ptr(), ldx, gW[l].data_ptr(),
                                                 part.data_ptr() if part is not None else None,
                                                 gb[l].data_ptr() if part is not None else None, st))
             self.kernel_launches += 1
             if l > 0:
                 nxt = torch.empty(N, din, dtype=BF16, device=dev)
                 part = torch.empty(-(-N // 128), din, dtype=torch.float64, device=dev)
-                check(lib.fne_mlp_linear_bwd_data(N, din, dout, dZ16.data_ptr(), self.W16[l].data_ptr(),
+                check(lib.fne_mlp_linear_bwd_data(N, din, dout, dZ16.data_ptr(), ldz, self.W16[l].data_ptr(),
                                                   self._saved[l - 1][1].data_ptr(), 1, nxt.data_ptr(),
                                                   part.data_ptr(), st))
-                dZ16 = nxt
+                dZ16, ldz = nxt, din
                 self.kernel_launches += 1
         return gW, gb
 

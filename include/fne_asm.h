@@ -375,17 +375,22 @@ int fne_mlp_bias_act(int64_t rows, int cols, float* Z, const float* bias, int ac
  * fne_mlp_bias_act; one launch, same bounded waits and status. */
 int fne_mlp_linear_fwd(int rows, int din, int dout, const void* X16, const void* W16, const float* bias, int act,
                        float* Z, float* H32, void* H16, void* stream);
-/* One layer's input gradient: d = dZ W (dZ [rows][dout], W [dout][din] BF16), times
+/* y[r][0..cols) = x[r][0..cols) as BF16 and zeros up to ``pitch`` (x FP32 or BF16,
+ * rows of ``cols``): pitches that are a multiple of 8 let the products below read
+ * narrow operands (12 features, 3 outputs) 16 bytes at a time. */
+int fne_mlp_pad_rows(int64_t rows, int cols, const void* x, int x_fp32, int pitch, void* y, void* stream);
+/* One layer's input gradient: d = dZ W (dZ rows of pitch ldz >= dout, W [dout][din] BF16), times
  * silu'(Zin) when act = 1 (Zin [rows][din]: the previous layer's z); dZin16 = d in
  * BF16; colpart [ceil(rows / 128)][din] = sums of d over each 128 rows (FP64,
  * fixed order), which fne_mlp_linear_bwd_weight turns into the bias gradient. */
-int fne_mlp_linear_bwd_data(int rows, int din, int dout, const void* dZ16, const void* W16, const float* Zin, int act,
-                            void* dZin16, double* colpart, void* stream);
-/* One layer's weight gradient: gW [dout][din] = dZ^T X; with colpart (from the call
+int fne_mlp_linear_bwd_data(int rows, int din, int dout, const void* dZ16, int ldz, const void* W16, const float* Zin,
+                            int act, void* dZin16, double* colpart, void* stream);
+/* One layer's weight gradient: gW [dout][din] = dZ^T X, rows of dZ and X of pitch ldz
+ * and ldx (columns up to the pitch are readable); with colpart (from the call
  * that produced dZ, [ceil(rows / 128)][dout]) also gb [dout], its column sums.
  * colpart and gb are both NULL or both given. */
-int fne_mlp_linear_bwd_weight(int rows, int din, int dout, const void* dZ16, const void* X16, float* gW,
-                              const double* colpart, float* gb, void* stream);
+int fne_mlp_linear_bwd_weight(int rows, int din, int dout, const void* dZ16, int ldz, const void* X16, int ldx,
+                              float* gW, const double* colpart, float* gb, void* stream);
 /* dZ = dH * silu'(Z) (act = 1) or dH (act = 0); dZ32 / dZ16 may be NULL. */
 int fne_mlp_act_bwd(int64_t n, const float* Z, const float* dH, int act, float* dZ32, void* dZ16, void* stream);
 /* out[c] = sum_r X[r, c] (FP64 accumulation, fixed order). */

@@ -159,7 +159,8 @@ def test_fused_layer_edges(rows, din, dout):
     Zin = torch.randn(rows, din, generator=g, **f32).cuda()
     dIn = torch.empty(rows, din, dtype=torch.bfloat16, device="cuda")
     part = torch.empty(-(-rows // 128), din, dtype=torch.float64, device="cuda")
-    _lib.check(L.fne_mlp_linear_bwd_data(rows, din, dout, vp(dZ), vp(W), vp(Zin), 1, vp(dIn), vp(part), None))
+    _lib.check(L.fne_mlp_linear_bwd_data(rows, din, dout, vp(dZ), dout, vp(W), vp(Zin), 1, vp(dIn),
+                                         vp(part), None))
     s = torch.sigmoid(Zin.double())
     ref = (dZ.double() @ W.double()) * (s * (1 + Zin.double() * (1 - s)))
     assert ((dIn.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * ref.abs().max() + 1e-5).all()
@@ -167,8 +168,19 @@ def test_fused_layer_edges(rows, din, dout):
 
     gW = torch.empty(din, dout, device="cuda", **f32)  # gradient of a layer dout -> din whose dZ is dIn
     gb = torch.empty(din, device="cuda", **f32)
-    _lib.check(L.fne_mlp_linear_bwd_weight(rows, dout, din, vp(dIn), vp(dZ), vp(gW), vp(part), vp(gb), None))
+    _lib.check(L.fne_mlp_linear_bwd_weight(rows, dout, din, vp(dIn), din, vp(dZ), dout, vp(gW), vp(part),
+                                           vp(gb), None))
     ref = dIn.double().T @ dZ.double()
     assert (gW.double() - ref).abs().max() <= 1e-5 * ref.abs().max() + 1e-5
     assert (gb.double() - part.sum(0)).abs().max() <= 1e-6 * part.sum(0).abs().max() + 1e-6
+    # the same from rows padded to a multiple of eight values: the same sums in the same order
+    ldx, ldz = -(-dout // 8) * 8, -(-din // 8) * 8
+    Xp, Zp = (torch.full((rows, ld), 9.0, dtype=torch.bfloat16, device="cuda") for ld in (ldx, ldz))
+    _lib.check(L.fne_mlp_pad_rows(rows, dout, vp(dZ), 0, ldx, vp(Xp), None))
+    dIn32 = dIn.float()
+    _lib.check(L.fne_mlp_pad_rows(rows, din, vp(dIn32), 1, ldz, vp(Zp), None))
+    assert (Xp[:, :dout] == dZ).all() and (Xp[:, dout:] == 0).all() and (Zp[:, :din] == dIn).all()
+    gP = torch.empty_like(gW)
+    _lib.check(L.fne_mlp_linear_bwd_weight(rows, dout, din, vp(Zp), ldz, vp(Xp), ldx, vp(gP), None, None, None))
+    assert torch.equal(gP, gW)
     _lib.check(L.fne_gemm_check_status())
