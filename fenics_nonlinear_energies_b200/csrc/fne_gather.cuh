@@ -239,29 +239,36 @@ __global__ void __launch_bounds__(256) k_fixup2(int n_blk, const int4* __restric
   }
 }
 
-// Gradient rows, one thread per row node: the node's element entries summed
-// in element order, minus the load vector.
+// Gradient rows of one row node: its element entries summed in element order,
+// minus the load vector.
+template <typename Real, int BS>
+__device__ __forceinline__ void rowgrad_node(int A, const int* __restrict__ rn_inc, const int* __restrict__ inc,
+                                             const int* __restrict__ rn_gpos, const Real* __restrict__ gbuf,
+                                             const double* __restrict__ rhs, double* __restrict__ grad) {
+  Real gs[BS];
+#pragma unroll
+  for (int c = 0; c < BS; ++c) gs[c] = Real(0);
+  const int i1 = __ldg(rn_inc + A + 1);
+  for (int i = __ldg(rn_inc + A); i < i1; ++i) {
+    const long long code = __ldg(inc + i);
+#pragma unroll
+    for (int c = 0; c < BS; ++c) gs[c] += gbuf[code * BS + c];
+  }
+#pragma unroll
+  for (int c = 0; c < BS; ++c) {
+    const int gp = __ldg(rn_gpos + A * BS + c);
+    if (gp >= 0) grad[gp] = (double)gs[c] - (rhs ? rhs[gp] : 0.0);
+  }
+}
+
+// Gradient rows, one thread per row node.
 template <typename Real, int BS>
 __global__ void __launch_bounds__(256) k_rowgrad(int n_rnodes, const int* __restrict__ rn_inc,
                                                  const int* __restrict__ inc, const int* __restrict__ rn_gpos,
                                                  const Real* __restrict__ gbuf, const double* __restrict__ rhs,
                                                  double* __restrict__ grad) {
-  for (int A = blockIdx.x * blockDim.x + threadIdx.x; A < n_rnodes; A += gridDim.x * blockDim.x) {
-    Real gs[BS];
-#pragma unroll
-    for (int c = 0; c < BS; ++c) gs[c] = Real(0);
-    const int i1 = __ldg(rn_inc + A + 1);
-    for (int i = __ldg(rn_inc + A); i < i1; ++i) {
-      const long long code = __ldg(inc + i);
-#pragma unroll
-      for (int c = 0; c < BS; ++c) gs[c] += gbuf[code * BS + c];
-    }
-#pragma unroll
-    for (int c = 0; c < BS; ++c) {
-      const int gp = __ldg(rn_gpos + A * BS + c);
-      if (gp >= 0) grad[gp] = (double)gs[c] - (rhs ? rhs[gp] : 0.0);
-    }
-  }
+  for (int A = blockIdx.x * blockDim.x + threadIdx.x; A < n_rnodes; A += gridDim.x * blockDim.x)
+    rowgrad_node<Real, BS>(A, rn_inc, inc, rn_gpos, gbuf, rhs, grad);
 }
 
 }  // namespace fne

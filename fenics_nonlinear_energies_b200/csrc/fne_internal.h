@@ -191,6 +191,7 @@ struct BlockPlan {
   std::vector<uint32_t> blk;
   std::vector<int32_t> con, inc;
   std::vector<int32_t> elem_rn;  // [n_local * npn] row node of each element node, -1 if none
+  std::vector<int32_t> blk_rn;   // bs = 3: row node that is the block's column node, -1 if it has no owned row
 };
 
 // Direct-write plan for kernels that hold whole element matrices: for every

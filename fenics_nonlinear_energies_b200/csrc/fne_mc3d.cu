@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "fne_gather.cuh"
@@ -136,12 +137,13 @@ __device__ __forceinline__ void m3_bcol(Real gx, Real gy, Real gz, int c, Real b
 // w psi.  Not inlined, so every instantiation of the element kernel runs the
 // same machine code here and the separate energy / gradient / Hessian passes
 // reproduce the fused pass bit for bit.
+// ``gq``: the point's row of the element's basis gradients, gx at gq[a], gy and
+// gz nq * NP and 2 nq * NP behind it (shared or global memory).
 template <typename Real, int NP>
-__device__ __noinline__ double m3_point_update(const double* __restrict__ grad, const int* __restrict__ codes,
+__device__ __noinline__ double m3_point_update(const double* gq, const int* __restrict__ codes,
                                                const double* __restrict__ u, const double* __restrict__ dir,
                                                const double* __restrict__ pt, int el, int q, int nq, double tiny,
                                                int elastic, Real* sig_out, Real* D_out) {
-  const double* gq = grad + (long long)el * 3 * nq * NP + q * NP;
   const int* cd = codes + (long long)el * 3 * NP;
   double e[6] = {0, 0, 0, 0, 0, 0};
   for (int a = 0; a < NP; ++a) {
@@ -151,7 +153,7 @@ __device__ __noinline__ double m3_point_update(const double* __restrict__ grad, 
       const int code = __ldg(cd + 3 * a + c);
       uc[c] = code >= 0 ? __ldg(u + code) : __ldg(dir + (-1 - code));
     }
-    const double gx = __ldg(gq + a), gy = __ldg(gq + nq * NP + a), gz = __ldg(gq + 2 * nq * NP + a);
+    const double gx = gq[a], gy = gq[nq * NP + a], gz = gq[2 * nq * NP + a];
     e[0] += gx * uc[0];
     e[1] += gy * uc[1];
     e[2] += gz * uc[2];
@@ -176,133 +178,186 @@ __device__ __noinline__ double m3_point_update(const double* __restrict__ grad, 
   return w * psi;
 }
 
+// Order of the node-pair blocks of an element in kbuf, and how the block of the
+// ordered pair (a, b) is read from it.
+//   P1 / P2: pair {b, (b + s) mod NP} at s * NP + b, s = 0 .. NP / 2 (the last
+//     distance only for b < NP / 2), holding B(b + s)^T (w D) B(b): the blocks
+//     one lane per node forms, in the order the lanes write them;
+//   P4: a <= b, row-major upper triangle, holding B(a)^T (w D) B(b).
+template <int NP>
+__host__ __device__ inline int m3_block(int a, int b, bool& transposed) {
+  if constexpr (NP > 10) {
+    transposed = a > b;
+    const int lo = transposed ? b : a, hi = transposed ? a : b;
+    return lo * NP - lo * (lo - 1) / 2 + (hi - lo);
+  } else {
+    const int s = a >= b ? a - b : a - b + NP;  // distance from b up to a
+    transposed = 2 * s > NP || (2 * s == NP && b >= NP / 2);
+    return transposed ? (s ? NP - s : 0) * NP + a : s * NP + b;
+  }
+}
+
+// Tile of k_mc3d_elem in dynamic shared memory.
+template <typename Real, int NP>
+struct M3Tile {
+  static constexpr int NT = 32 * kM3Warps, DS = 22;  // points; values of w D per point, padded to pairs
+  Real D[NT][DS];                                    // w D, upper triangle row-major
+  Real sig[NT][6];                                   // w sigma
+  Real out[kM3Warps][32 * 9];                        // one block per lane on its way to kbuf
+  // then: double g[elements of the tile][3][nq][NP], basis gradients
+  static size_t bytes(int nq) { return sizeof(M3Tile) + (size_t)(NT / nq) * 3 * nq * NP * sizeof(double); }
+};
+
+// Contraction split: one lane per node b, 32 / NP elements a warp (three P2
+// tets: 30 of 32 lanes, and the 11 elements of a tile in one round of the
+// four warps).  Per point a lane forms T = (w D) B(b) in registers (54
+// products from the 21 values every lane of the element reads alike) and adds
+// B(a)^T T for the nodes a = b, b + 1, ... at distance up to NP / 2, three at
+// a time, so each unordered pair is formed once.  Shared memory bounded the
+// earlier split (lanes over pairs, 21 loads of T and B(a) per 27 products, and
+// 72-byte blocks stored value by value: 607 us for 61,440 P2 tets, of which
+// the FP64 units need 105); here a lane loads 20 values per 81 products, and
+// blocks leave through shared memory in whole lines.
 template <typename Real, int NP, int WANT>
 __global__ void __launch_bounds__(32 * kM3Warps, 3) k_mc3d_elem(Mc3dArgs A, Real* __restrict__ kbuf,
                                                              Real* __restrict__ gbuf) {
   constexpr int N = 3 * NP, NPAIR = NP * (NP + 1) / 2, NT = 32 * kM3Warps;
-  __shared__ Real s_sig[NT][6];                      // w sigma per point of the tile
-  __shared__ Real s_D[NT][21];                       // w D, upper triangle row-major
-  __shared__ Real s_g[kM3Warps][3][kM3MaxQ * NP];    // gx, gy, gz of the warp's element
-  __shared__ Real s_T[kM3Warps][NP][18];             // (w D) B(b) of one point, per node
+  constexpr int EPW = 32 / NP, SP = 3;  // elements per warp; distances per pass
+  using Tile = M3Tile<Real, NP>;
+  using V2 = typename std::conditional<sizeof(Real) == 8, double2, float2>::type;
+  extern __shared__ __align__(16) unsigned char m3_smem[];
+  Tile& T_ = *reinterpret_cast<Tile*>(m3_smem);
+  double* s_g = reinterpret_cast<double*>(m3_smem + sizeof(Tile));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nq = A.nq, epc = NT / nq;                // elements per tile: all their points in one pass
+  const int gs = 3 * nq * NP;                        // basis gradients per element (even: NP is)
   double eacc = 0.0;
   for (int el0 = blockIdx.x * epc; el0 < A.n_el; el0 += gridDim.x * epc) {
     const int ne = min(epc, A.n_el - el0);
+    {  // the tile's basis gradients, one contiguous run
+      const double2* src = reinterpret_cast<const double2*>(A.grad + (long long)el0 * gs);
+      double2* dst = reinterpret_cast<double2*>(s_g);
+#pragma unroll 4
+      for (int i = threadIdx.x; i < ne * gs / 2; i += NT) dst[i] = __ldg(src + i);
+    }
+    {  // the next tile's, into L2
+      const int el1 = el0 + gridDim.x * epc, n1 = min(epc, A.n_el - el1);
+      const char* p = reinterpret_cast<const char*>(A.grad + (long long)el1 * gs);
+      for (int i = threadIdx.x * 128; i < n1 * gs * 8; i += NT * 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
+      const char* m = reinterpret_cast<const char*>(A.pt + (long long)el1 * nq * kM3Pt);
+      for (int i = threadIdx.x * 128; i < n1 * nq * kM3Pt * 8; i += NT * 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(m + i));
+    }
+    __syncthreads();
     // constitutive update, one thread per (element, quadrature point) of the
     // tile (FP64): strain from the nodal values, then the point function
     if ((int)threadIdx.x < ne * nq) {
       const int j = threadIdx.x / nq, q = threadIdx.x - j * nq, el = el0 + j;
-      const double wpsi = m3_point_update<Real, NP>(A.grad, A.codes, A.u, A.dir, A.pt, el, q, nq, A.tiny,
-                                                    A.elastic, s_sig[threadIdx.x], s_D[threadIdx.x]);
+      const double wpsi = m3_point_update<Real, NP>(s_g + j * gs + q * NP, A.codes, A.u, A.dir, A.pt, el, q, nq,
+                                                    A.tiny, A.elastic, T_.sig[threadIdx.x], T_.D[threadIdx.x]);
       if ((WANT & 1) && __ldg(A.wflag + el)) eacc += wpsi;
     }
     __syncthreads();
-    // contraction: one warp per element of the tile
-    for (int j = warp; (WANT & 6) && j < ne; j += kM3Warps) {
-      const int el = el0 + j;
-      const Real(*sg)[6] = s_sig + j * nq;
-      const Real(*sD)[21] = s_D + j * nq;
-      const double* gsrc = A.grad + (long long)el * 3 * nq * NP;
-      for (int i = lane; i < 3 * nq * NP; i += 32) {
-        const int k = i / (nq * NP), r = i - k * nq * NP;
-        s_g[warp][k][r] = (Real)__ldg(gsrc + i);
-      }
-      __syncwarp();
-      // element gradient: lanes over (node, component)
-      if (WANT & 2) {
-        for (int i = lane; i < N; i += 32) {
-          const int a = i / 3, c = i - 3 * a;
-          Real s = Real(0);
-          for (int q = 0; q < nq; ++q) {
-            Real b[6];
-            m3_bcol<Real>(s_g[warp][0][q * NP + a], s_g[warp][1][q * NP + a], s_g[warp][2][q * NP + a], c, b);
-#pragma unroll
-            for (int k = 0; k < 6; ++k) s += b[k] * sg[q][k];
-          }
-          gbuf[(long long)el * N + i] = s;
-        }
-      }
-      // Hessian blocks B(a)^T (w D) B(b) over the node pairs a <= b.  Each
-      // column of B has three nonzeros (DOF (b, d) feeds three strain rows), so
-      // per quadrature point the lanes first form T_b = (w D) B(b) (6 x 3, 18
-      // products of three terms) and the lanes over pairs then add B(a)^T T_b
-      // (9 sums of three terms)
-      if (WANT & 4) {
-        constexpr int PPL = (NPAIR + 31) / 32;  // pairs per lane
-        Real K[PPL][3][3];
-        int pa[PPL], pb[PPL];
-#pragma unroll
-        for (int k = 0; k < PPL; ++k) {
-          int a = 0, rem = lane + 32 * k;
-          while (a < NP && rem >= NP - a) {
-            rem -= NP - a;
-            ++a;
-          }
-          pa[k] = a;
-          pb[k] = a + rem;
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int d = 0; d < 3; ++d) K[k][c][d] = Real(0);
-        }
-        // (w D) B(b): lanes over (node b, strain row i), each forming row i
-        // of T_b from row i of w D (upper-triangle positions precomputed)
-        constexpr int NTI = NP * 6, TPL = (NTI + 31) / 32;
-        int tb[TPL], ti[TPL], didx[TPL][6];
-#pragma unroll
-        for (int k = 0; k < TPL; ++k) {
-          const int it = min(lane + 32 * k, NTI - 1);
-          tb[k] = it / 6;
-          ti[k] = it - 6 * tb[k];
-#pragma unroll
-          for (int j = 0; j < 6; ++j) {
-            const int lo = min(ti[k], j), hi = max(ti[k], j);
-            didx[k][j] = lo * 6 - lo * (lo - 1) / 2 + (hi - lo);
-          }
-        }
+    const int sub = lane / NP, b = lane - sub * NP;
+    for (int j0 = warp * EPW; (WANT & 6) && j0 < ne; j0 += kM3Warps * EPW) {
+      const int j = j0 + sub;
+      const bool on = sub < EPW && j < ne;
+      const int jj = on ? j : j0;  // idle lanes follow the first element and store nothing
+      const double* gx_ = s_g + jj * gs;
+      const double* gy_ = gx_ + nq * NP;
+      const double* gz_ = gy_ + nq * NP;
+      if (WANT & 2) {  // element gradient: node b's three components
+        Real r0 = Real(0), r1 = Real(0), r2 = Real(0);
         for (int q = 0; q < nq; ++q) {
+          const Real* sg = T_.sig[jj * nq + q];
+          const Real gx = (Real)gx_[q * NP + b], gy = (Real)gy_[q * NP + b], gz = (Real)gz_[q * NP + b];
+          r0 += gx * sg[0];
+          r0 += gy * sg[3];
+          r0 += gz * sg[5];
+          r1 += gy * sg[1];
+          r1 += gx * sg[3];
+          r1 += gz * sg[4];
+          r2 += gz * sg[2];
+          r2 += gy * sg[4];
+          r2 += gx * sg[5];
+        }
+        if (on) {
+          Real* o = gbuf + (long long)(el0 + j) * N + 3 * b;
+          o[0] = r0;
+          o[1] = r1;
+          o[2] = r2;
+        }
+      }
+      if (WANT & 4) {
+        for (int s0 = 0; s0 <= NP / 2; s0 += SP) {
+          Real K[SP][9];
+          int aa[SP];
 #pragma unroll
-          for (int k = 0; k < TPL; ++k) {
-            if (lane + 32 * k >= NTI) continue;
-            const Real* Dq = sD[q];
-            const Real d0 = Dq[didx[k][0]], d1 = Dq[didx[k][1]], d2 = Dq[didx[k][2]], d3 = Dq[didx[k][3]],
-                       d4 = Dq[didx[k][4]], d5 = Dq[didx[k][5]];
-            const Real gx = s_g[warp][0][q * NP + tb[k]], gy = s_g[warp][1][q * NP + tb[k]],
-                       gz = s_g[warp][2][q * NP + tb[k]];
-            Real* T = s_T[warp][tb[k]] + 3 * ti[k];
-            T[0] = d0 * gx + d3 * gy + d5 * gz;
-            T[1] = d1 * gy + d3 * gx + d4 * gz;
-            T[2] = d2 * gz + d4 * gy + d5 * gx;
+          for (int s = 0; s < SP; ++s) {
+            aa[s] = b + s0 + s < NP ? b + s0 + s : b + s0 + s - NP;
+#pragma unroll
+            for (int i = 0; i < 9; ++i) K[s][i] = Real(0);
           }
-          __syncwarp();
+#pragma unroll 1
+          for (int q = 0; q < nq; ++q) {
+            Real d[Tile::DS];
+            const V2* Dq = reinterpret_cast<const V2*>(T_.D[jj * nq + q]);
 #pragma unroll
-          for (int k = 0; k < PPL; ++k) {
-            if (lane + 32 * k >= NPAIR) continue;
-            const Real ax = s_g[warp][0][q * NP + pa[k]], ay = s_g[warp][1][q * NP + pa[k]],
-                       az = s_g[warp][2][q * NP + pa[k]];
-            const Real* T = s_T[warp][pb[k]];
+            for (int i = 0; i < 11; ++i) {
+              const V2 v = Dq[i];
+              d[2 * i] = v.x;
+              d[2 * i + 1] = v.y;
+            }
+            const Real gx = (Real)gx_[q * NP + b], gy = (Real)gy_[q * NP + b], gz = (Real)gz_[q * NP + b];
+            Real T[6][3];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-              K[k][0][d] += ax * T[0 * 3 + d] + ay * T[3 * 3 + d] + az * T[5 * 3 + d];
-              K[k][1][d] += ay * T[1 * 3 + d] + ax * T[3 * 3 + d] + az * T[4 * 3 + d];
-              K[k][2][d] += az * T[2 * 3 + d] + ay * T[4 * 3 + d] + ax * T[5 * 3 + d];
+            for (int i = 0; i < 6; ++i) {
+              Real Di[6];
+#pragma unroll
+              for (int k = 0; k < 6; ++k) {
+                const int lo = i < k ? i : k, hi = i < k ? k : i;
+                Di[k] = d[lo * 6 - lo * (lo - 1) / 2 + (hi - lo)];
+              }
+              T[i][0] = Di[0] * gx + Di[3] * gy + Di[5] * gz;
+              T[i][1] = Di[1] * gy + Di[3] * gx + Di[4] * gz;
+              T[i][2] = Di[2] * gz + Di[4] * gy + Di[5] * gx;
+            }
+#pragma unroll
+            for (int s = 0; s < SP; ++s) {
+              const Real ax = (Real)gx_[q * NP + aa[s]], ay = (Real)gy_[q * NP + aa[s]],
+                         az = (Real)gz_[q * NP + aa[s]];
+#pragma unroll
+              for (int k = 0; k < 3; ++k) {
+                K[s][k] += ax * T[0][k] + ay * T[3][k] + az * T[5][k];
+                K[s][3 + k] += ay * T[1][k] + ax * T[3][k] + az * T[4][k];
+                K[s][6 + k] += az * T[2][k] + ay * T[4][k] + ax * T[5][k];
+              }
             }
           }
-          __syncwarp();
-        }
+          // one distance at a time: the warp's blocks through shared memory, then per element the run of
+          // blocks of that distance (NP of them, NP / 2 at the last) in whole lines
+          Real* st = T_.out[warp];
 #pragma unroll
-        for (int k = 0; k < PPL; ++k) {
-          const int p = lane + 32 * k;
-          if (p >= NPAIR) continue;
-          Real* o = kbuf + ((long long)el * NPAIR + p) * 9;
+          for (int s = 0; s < SP; ++s) {
+            const int dist = s0 + s;
+            if (2 * dist > NP) break;
+            const int run = 9 * (2 * dist == NP ? NP / 2 : NP);
+            __syncwarp();
 #pragma unroll
-          for (int c = 0; c < 3; ++c)
+            for (int i = 0; i < 9; ++i) st[lane * 9 + i] = K[s][i];
+            __syncwarp();
 #pragma unroll
-            for (int d = 0; d < 3; ++d) o[c * 3 + d] = K[k][c][d];
+            for (int e = 0; e < EPW; ++e)
+              if (j0 + e < ne) {
+                Real* o = kbuf + ((long long)(el0 + j0 + e) * NPAIR + dist * NP) * 9;
+#pragma unroll
+                for (int i = lane; i < 9 * NP; i += 32)
+                  if (i < run) o[i] = st[e * 9 * NP + i];
+              }
+          }
         }
       }
-      __syncwarp();
     }
     __syncthreads();
   }
@@ -336,8 +391,9 @@ __global__ void __launch_bounds__(32 * kM3Warps) k_mc3d_elem_hi(Mc3dArgs A, Real
     const int ne = min(epc, A.n_el - el0);
     if ((int)threadIdx.x < ne * nq) {
       const int j = threadIdx.x / nq, q = threadIdx.x - j * nq, el = el0 + j;
-      const double wpsi = m3_point_update<Real, NP>(A.grad, A.codes, A.u, A.dir, A.pt, el, q, nq, A.tiny,
-                                                    A.elastic, s_sig[threadIdx.x], s_D[threadIdx.x]);
+      const double wpsi = m3_point_update<Real, NP>(A.grad + (long long)el * 3 * nq * NP + q * NP, A.codes, A.u,
+                                                    A.dir, A.pt, el, q, nq, A.tiny, A.elastic, s_sig[threadIdx.x],
+                                                    s_D[threadIdx.x]);
       if ((WANT & 1) && __ldg(A.wflag + el)) eacc += wpsi;
     }
     __syncthreads();
@@ -426,6 +482,100 @@ __global__ void __launch_bounds__(32 * kM3Warps) k_mc3d_elem_hi(Mc3dArgs A, Real
   }
 }
 
+// One unordered pair of row nodes (A, B): the block (A, B) and, mirrored, the
+// block (B, A) are the same sum over elements.
+struct alignas(16) M3Pair {
+  int start;      // contributions 5, 6, ... in the contribution array
+  unsigned meta;  // contributions (bits 0-15), free components of B (16-18) and of A (19-21)
+  unsigned off;   // column offset of B in the rows of A (bits 0-15), of A in the rows of B (16-31)
+  int node_b;     // row node B whose rows get the mirrored block, -1: none (A itself, or not an owned row)
+  int code[4];    // the first contributions: 2 * (block in kbuf) + transposed, element order; -1 beyond the last
+};
+
+// Sums the stored blocks into the COO values, and the element gradients into
+// the owned gradient.  Nine lanes per pair of nodes: lane (c, d) adds its entry
+// of every contributing element's block in element order and writes it to row
+// (A, c) and, mirrored, to row (B, d); a warp takes three pairs twice.  The
+// next pairs' records, with their first four contributions in them, are loaded
+// while these are summed, so the blocks are the only loads waited for.  A block is read as 72 consecutive bytes by
+// nine lanes, three or four lines a load instruction, and each is read once.
+// (One warp per row node and one lane per block, as k_node_gather does for the
+// other families, read every off-diagonal block twice, 470 MB from DRAM, with
+// nine loads of 32 lines each: 234 us for 61,440 P2 tets.)  No atomics;
+// bit-reproducible.
+template <typename Real, typename HOut, bool WANT_G>
+__global__ void __launch_bounds__(256) k_mc3d_gather(int n_pairs, const M3Pair* __restrict__ pairs,
+                                                     const int* __restrict__ pair_a, NodeGatherArgs G,
+                                                     const Real* __restrict__ kbuf, const Real* __restrict__ gbuf,
+                                                     HOut* __restrict__ out, double* __restrict__ grad) {
+  if (WANT_G)
+    for (int A = blockIdx.x * blockDim.x + threadIdx.x; A < G.n_rnodes; A += gridDim.x * blockDim.x)
+      rowgrad_node<Real, 3>(A, G.rn_inc, G.inc, G.rn_gpos, gbuf, G.rhs, grad);
+  constexpr int U = 4;
+  const int lane = threadIdx.x & 31, grp = lane / 9, ent = lane - 9 * grp;
+  const int c = ent / 3, d = ent - 3 * c, ent_t = 3 * d + c;
+  const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int nw = (int)((gridDim.x * blockDim.x) >> 5);
+  if (grp == 3) return;  // no warp-wide operation below
+  int4 rec[2], codes[2];
+  int node_a[2];
+  auto fetch = [&](int t0) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int t = t0 + 3 * h + grp;
+      const bool in = t >= 0 && t < n_pairs;
+      rec[h] = in ? __ldg(reinterpret_cast<const int4*>(pairs + t)) : make_int4(0, 0, 0, -1);
+      codes[h] = in ? __ldg(reinterpret_cast<const int4*>(pairs + t) + 1) : make_int4(-1, -1, -1, -1);
+      node_a[h] = in ? __ldg(pair_a + t) : -1;
+    }
+  };
+  // last pairs first: the blocks the element kernel wrote last are still in L2
+  int t0 = (n_pairs - 1) / 6 * 6 - gw * 6;
+  fetch(t0);
+  for (; t0 >= 0; t0 -= nw * 6) {
+    int4 pr[2];
+    int row_a[2], row_b[2];
+    Real v[2][4], acc[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      pr[h] = rec[h];
+      const int code[4] = {codes[h].x, codes[h].y, codes[h].z, codes[h].w};
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        v[h][x] = code[x] >= 0 ? __ldg(kbuf + (long long)(code[x] >> 1) * 9 + ((code[x] & 1) ? ent_t : ent)) : Real(0);
+      row_a[h] = node_a[h] >= 0 && (((unsigned)pr[h].y >> (16 + d)) & 1u) ? __ldg(G.rn_row + 3 * node_a[h] + c) : -1;
+      row_b[h] = pr[h].w >= 0 && (((unsigned)pr[h].y >> (19 + c)) & 1u) ? __ldg(G.rn_row + 3 * pr[h].w + d) : -1;
+    }
+    fetch(t0 - nw * 6);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int n = pr[h].y & 0xFFFF;
+      acc[h] = Real(0);
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        if (x < n) acc[h] += v[h][x];
+      for (int j = 4; j < n; j += 6) {  // beyond the fourth: six at a time
+        int cd[6];
+        Real w[6];
+#pragma unroll
+        for (int x = 0; x < 6; ++x) cd[x] = j + x < n ? __ldg(G.con + pr[h].x + j + x - 4) : -1;
+#pragma unroll
+        for (int x = 0; x < 6; ++x)
+          w[x] = cd[x] >= 0 ? __ldg(kbuf + (long long)(cd[x] >> 1) * 9 + ((cd[x] & 1) ? ent_t : ent)) : Real(0);
+#pragma unroll
+        for (int x = 0; x < 6; ++x)
+          if (cd[x] >= 0) acc[h] += w[x];
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const unsigned meta = (unsigned)pr[h].y, off = (unsigned)pr[h].z, db = (meta >> 16) & 7u, da = (meta >> 19) & 7u;
+      if (row_a[h] >= 0) out[row_a[h] + (int)(off & 0xFFFFu) + __popc(db & ((1u << d) - 1u))] = (HOut)acc[h];
+      if (row_b[h] >= 0) out[row_b[h] + (int)(off >> 16) + __popc(da & ((1u << c) - 1u))] = (HOut)acc[h];
+    }
+  }
+}
+
 }  // namespace
 
 struct Mc3dHandle {
@@ -439,9 +589,9 @@ struct Mc3dHandle {
   unsigned* counter = nullptr;
   void *kbuf = nullptr, *gbuf = nullptr;
   int grid_elem = 1, n_rnodes = 0;
-  int *bp_rn_blk = nullptr, *bp_rn_con = nullptr, *bp_rn_row = nullptr, *bp_rn_gpos = nullptr,
-      *bp_rn_inc = nullptr, *bp_con = nullptr, *bp_inc = nullptr;
-  unsigned* bp_blk = nullptr;
+  int *bp_rn_row = nullptr, *bp_rn_gpos = nullptr, *bp_rn_inc = nullptr, *bp_con = nullptr, *bp_inc = nullptr;
+  M3Pair* pairs = nullptr;
+  int *pair_a = nullptr, n_pairs = 0;
   int64_t device_bytes = 0, n_contrib = 0;
 };
 
@@ -461,15 +611,105 @@ int m3_upload(Mc3dHandle* h, T** p, const T* src, size_t count) {
   return FNE_OK;
 }
 
-// resident CTAs per SM of the fused pass (registers and shared memory)
+// Pairs of row nodes from the node-block plan: every block (A, B) with element
+// contributions once, from the row node with the smaller index when both have
+// owned rows.  Codes stay
+// below 2^31: n_elem * pairs * 9 < 2^33 is checked by the caller.
+int build_pairs(const BlockPlan& bp, int64_t n_el, int np, std::vector<M3Pair>& pairs, std::vector<int32_t>& pair_a,
+                std::vector<int32_t>& con) {
+  const int npair = np * (np + 1) / 2, n = bp.n_rnodes;
+  // blocks of every row node in the order of their column's row node, to find (B, A)
+  std::vector<int32_t> order(bp.blk.size());
+  for (int32_t k = 0; k < n; ++k) {
+    for (int32_t b = bp.rn_blk[k]; b < bp.rn_blk[k + 1]; ++b) order[b] = b;
+    std::sort(order.begin() + bp.rn_blk[k], order.begin() + bp.rn_blk[k + 1],
+              [&](int32_t x, int32_t y) { return bp.blk_rn[x] < bp.blk_rn[y]; });
+  }
+  pairs.reserve(bp.blk.size() / 2 + n);
+  pair_a.reserve(bp.blk.size() / 2 + n);
+  for (int32_t A = 0; A < n; ++A) {
+    int64_t at = bp.rn_con[A];
+    for (int32_t b = bp.rn_blk[A]; b < bp.rn_blk[A + 1]; ++b) {
+      const uint32_t w = bp.blk[b];
+      const int32_t cnt = (int32_t)(w >> 19), B = bp.blk_rn[b];
+      const int64_t c0 = at;
+      at += cnt;
+      // element contributions come in both directions; a block without any (a pattern wider than the element
+      // graph, which need not be symmetric) is a zero of its own
+      const bool both = cnt > 0 && B >= 0;
+      if (both && B < A) continue;
+      M3Pair p;
+      for (int x = 0; x < 4; ++x) p.code[x] = -1;
+      p.start = (int32_t)con.size();
+      p.meta = (uint32_t)cnt | ((w >> 16) & 7u) << 16;
+      p.off = w & 0xFFFFu;
+      p.node_b = -1;
+      if (both && B > A) {
+        const auto first = order.begin() + bp.rn_blk[B], last = order.begin() + bp.rn_blk[B + 1];
+        const auto it = std::lower_bound(first, last, A, [&](int32_t x, int32_t v) { return bp.blk_rn[x] < v; });
+        if (it == last || bp.blk_rn[*it] != A || (int32_t)(bp.blk[*it] >> 19) != cnt)
+          return set_error(FNE_ELAYOUT, "Mohr-Coulomb 3-D: COO pattern is not symmetric over the owned rows");
+        p.meta |= ((bp.blk[*it] >> 16) & 7u) << 19;
+        p.off |= (bp.blk[*it] & 0xFFFFu) << 16;
+        p.node_b = B;
+      }
+      for (int64_t k = c0; k < c0 + cnt; ++k) {
+        const int el = bp.con[k] / (np * np), r = bp.con[k] - el * np * np, a = r / np, bb = r - a * np;
+        bool tr = false;
+        const int q = np == 35 ? m3_block<35>(a, bb, tr) : np == 10 ? m3_block<10>(a, bb, tr) : m3_block<4>(a, bb, tr);
+        const int code = 2 * (el * npair + q) + (tr ? 1 : 0);
+        if (k - c0 < 4)
+          p.code[k - c0] = code;
+        else
+          con.push_back(code);
+      }
+      pairs.push_back(p);
+      pair_a.push_back(A);
+    }
+  }
+  // in the order of their first contributing element (pairs without one first): the blocks are then read as
+  // they lie, once; in row-node order the vertices' and the edge nodes' pairs each swept the whole buffer
+  const auto bucket = [&](const M3Pair& p) { return p.code[0] < 0 ? 0 : p.code[0] / 2 / npair + 1; };
+  std::vector<int32_t> at((size_t)n_el + 2, 0);
+  for (const M3Pair& p : pairs) ++at[bucket(p) + 1];
+  for (size_t k = 1; k < at.size(); ++k) at[k] += at[k - 1];
+  std::vector<M3Pair> sorted(pairs.size());
+  std::vector<int32_t> sorted_a(pairs.size());
+  for (size_t k = 0; k < pairs.size(); ++k) {
+    const int32_t to = at[bucket(pairs[k])]++;
+    sorted[to] = pairs[k];
+    sorted_a[to] = pair_a[k];
+  }
+  pairs.swap(sorted);
+  pair_a.swap(sorted_a);
+  return FNE_OK;
+}
+
+// resident CTAs per SM of the fused pass (registers and shared memory); allows
+// every instantiation of the P1 / P2 kernel its tile of shared memory
+template <typename Real, int NP>
+cudaError_t m3_prepare(int nq, int* per_sm) {
+  const size_t bytes = M3Tile<Real, NP>::bytes(nq);
+  cudaError_t e = cudaSuccess;
+  auto allow = [&](auto* k) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  allow(&k_mc3d_elem<Real, NP, 1>);
+  allow(&k_mc3d_elem<Real, NP, 2>);
+  allow(&k_mc3d_elem<Real, NP, 3>);
+  allow(&k_mc3d_elem<Real, NP, 4>);
+  allow(&k_mc3d_elem<Real, NP, 5>);
+  allow(&k_mc3d_elem<Real, NP, 6>);
+  allow(&k_mc3d_elem<Real, NP, 7>);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_mc3d_elem<Real, NP, 7>, 32 * kM3Warps, bytes);
+  return e;
+}
 template <typename Real>
-int m3_ctas_per_sm(int np) {
-  int n = 0;
-  const cudaError_t e =
-      np == 35   ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_mc3d_elem_hi<Real, 35, 7>, 32 * kM3Warps, 0)
-      : np == 10 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_mc3d_elem<Real, 10, 7>, 32 * kM3Warps, 0)
-                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_mc3d_elem<Real, 4, 7>, 32 * kM3Warps, 0);
-  return e == cudaSuccess && n > 0 ? n : 2;
+cudaError_t m3_ctas_per_sm(int np, int nq, int* per_sm) {
+  if (np == 10) return m3_prepare<Real, 10>(nq, per_sm);
+  if (np == 4) return m3_prepare<Real, 4>(nq, per_sm);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_mc3d_elem_hi<Real, 35, 7>, 32 * kM3Warps, 0);
 }
 
 template <typename Real, typename HOut, int NP>
@@ -486,7 +726,7 @@ cudaError_t m3_launch(Mc3dHandle* h, int flags, const double* u, double* energy,
     if constexpr (NP > 10)                                            \
       k_mc3d_elem_hi<Real, NP, W><<<grid, block, 0, st>>>(A, kb, gb); \
     else                                                              \
-      k_mc3d_elem<Real, NP, W><<<grid, block, 0, st>>>(A, kb, gb);    \
+      k_mc3d_elem<Real, NP, W><<<grid, block, M3Tile<Real, NP>::bytes(h->nq), st>>>(A, kb, gb); \
     break;
   switch (flags) {
     M3_CASE(1)
@@ -501,15 +741,21 @@ cudaError_t m3_launch(Mc3dHandle* h, int flags, const double* u, double* energy,
 #undef M3_CASE
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || !(flags & 6) || h->n_rnodes == 0) return e;
-  NodeGatherArgs G{h->n_rnodes, h->bp_rn_blk, h->bp_rn_con, h->bp_rn_row, h->bp_rn_gpos,
-                   h->bp_rn_inc, h->bp_blk,   h->bp_con,    h->bp_inc,    h->rhs};
+  NodeGatherArgs G{};
+  G.n_rnodes = h->n_rnodes;
+  G.rn_row = h->bp_rn_row;
+  G.rn_gpos = h->bp_rn_gpos;
+  G.rn_inc = h->bp_rn_inc;
+  G.con = h->bp_con;
+  G.inc = h->bp_inc;
+  G.rhs = h->rhs;
   HOut* H = static_cast<HOut*>(hess);
   if (flags & 4) {
-    const int gg = std::max(1, std::min(h->num_sms * 16, (h->n_rnodes + 7) / 8));
+    const int gg = std::max(1, std::min(h->num_sms * 16, (h->n_pairs + 47) / 48));
     if (flags & 2)
-      k_node_gather<Real, HOut, 3, NP, true, true><<<gg, 256, 0, st>>>(G, kb, gb, H, grad);
+      k_mc3d_gather<Real, HOut, true><<<gg, 256, 0, st>>>(h->n_pairs, h->pairs, h->pair_a, G, kb, gb, H, grad);
     else
-      k_node_gather<Real, HOut, 3, NP, true, false><<<gg, 256, 0, st>>>(G, kb, gb, H, grad);
+      k_mc3d_gather<Real, HOut, false><<<gg, 256, 0, st>>>(h->n_pairs, h->pairs, h->pair_a, G, kb, gb, H, grad);
   } else {
     const int gr = std::max(1, std::min(h->num_sms * 8, (h->n_rnodes + 255) / 256));
     k_rowgrad<Real, 3><<<gr, 256, 0, st>>>(h->n_rnodes, h->bp_rn_inc, h->bp_inc, h->bp_rn_gpos, gb, h->rhs, grad);
@@ -530,8 +776,7 @@ cudaError_t m3_dispatch(Mc3dHandle* h, int flags, const double* u, double* energ
 void mc3d_destroy(Mc3dHandle* h) {
   if (!h) return;
   void* ptrs[] = {h->codes, h->grad, h->pt, h->dir, h->rhs, h->partials, h->wflag, h->counter, h->kbuf, h->gbuf,
-                  h->bp_rn_blk, h->bp_rn_con, h->bp_rn_row, h->bp_rn_gpos, h->bp_rn_inc, h->bp_con, h->bp_inc,
-                  h->bp_blk};
+                  h->bp_rn_row, h->bp_rn_gpos, h->bp_rn_inc, h->bp_con, h->bp_inc, h->pairs, h->pair_a};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete h;
@@ -612,7 +857,13 @@ int mc3d_create(const fne_desc* d, Mc3dHandle** out) {
   // tiles of 128 / nq elements (all their points in one pass of the CTA);
   // one wave of resident CTAs, each striding over the tiles
   const int64_t epc = 32 * kM3Warps / nq;
-  const int per_sm = d->precision == FNE_FP64 ? m3_ctas_per_sm<double>(h->np) : m3_ctas_per_sm<float>(h->np);
+  int per_sm = 0;
+  const cudaError_t oe = d->precision == FNE_FP64 ? m3_ctas_per_sm<double>(h->np, nq, &per_sm)
+                                                  : m3_ctas_per_sm<float>(h->np, nq, &per_sm);
+  if (oe != cudaSuccess || per_sm < 1) {
+    mc3d_destroy(h);
+    return set_error(FNE_ECUDA, std::string("Mohr-Coulomb 3-D: occupancy: ") + cudaGetErrorString(oe));
+  }
   h->grid_elem = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)h->num_sms * per_sm, (nl + epc - 1) / epc));
   const size_t rsz = d->precision == FNE_FP32 ? sizeof(float) : sizeof(double);
   int rc = FNE_OK;
@@ -636,13 +887,16 @@ int mc3d_create(const fne_desc* d, Mc3dHandle** out) {
     mc3d_destroy(h);
     return set_error(FNE_ECUDA, "Mohr-Coulomb 3-D: cudaMemset");
   }
-  M3_TRY(m3_upload(h, &h->bp_rn_blk, bp.rn_blk.data(), bp.rn_blk.size()));
-  M3_TRY(m3_upload(h, &h->bp_rn_con, bp.rn_con.data(), bp.rn_con.size()));
   M3_TRY(m3_upload(h, &h->bp_rn_row, bp.rn_row.data(), bp.rn_row.size()));
   M3_TRY(m3_upload(h, &h->bp_rn_gpos, bp.rn_gpos.data(), bp.rn_gpos.size()));
   M3_TRY(m3_upload(h, &h->bp_rn_inc, bp.rn_inc.data(), bp.rn_inc.size()));
-  M3_TRY(m3_upload(h, &h->bp_blk, bp.blk.data(), bp.blk.size()));
-  M3_TRY(m3_upload(h, &h->bp_con, bp.con.data(), bp.con.size()));
+  std::vector<M3Pair> pairs;
+  std::vector<int32_t> pair_a, con;
+  M3_TRY(build_pairs(bp, nl, np, pairs, pair_a, con));
+  h->n_pairs = (int)pairs.size();
+  M3_TRY(m3_upload(h, &h->pairs, pairs.data(), pairs.size()));
+  M3_TRY(m3_upload(h, &h->pair_a, pair_a.data(), pair_a.size()));
+  M3_TRY(m3_upload(h, &h->bp_con, con.data(), con.size()));
   M3_TRY(m3_upload(h, &h->bp_inc, bp.inc.data(), bp.inc.size()));
   unsigned char* kb = nullptr;
   M3_TRY(m3_upload(h, &kb, (const unsigned char*)nullptr, std::max<size_t>(1, (size_t)nl * npair * 9 * rsz)));

@@ -56,25 +56,36 @@ FNE_HD void eigh3(const double A0[3][3], double w[3], double V[3][3]) {
       // ends the solve (3 to 4 sweeps for almost every strain)
       if (apq == 0.0 || fabs(apq) <= 2.220446049250313e-16 * fabs(a[q][q] - a[p][p])) continue;
       rotated = true;
-      const double theta = (a[q][q] - a[p][p]) / (2.0 * apq);
-      const double t = fabs(theta) > 1e100 ? 0.5 / theta
-                                            : (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+      // t = sign(d) 2 apq / (|d| + sqrt(d^2 + 4 apq^2)), d = aqq - app: one
+      // square root and one division, with theta = d / (2 apq) only where the
+      // squares leave the range of a double; c = 1 / sqrt(t^2 + 1)
+      const double d = a[q][q] - a[p][p], d2 = d * d + 4.0 * apq * apq;
+      double t;
+      if (d2 > 1e-280 && d2 < 1e280) {
+        t = (d >= 0.0 ? 2.0 * apq : -2.0 * apq) / (fabs(d) + sqrt(d2));
+      } else {
+        const double theta = d / (2.0 * apq);
+        t = fabs(theta) > 1e100 ? 0.5 / theta
+                                : (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+      }
+#ifdef __CUDA_ARCH__
+      const double c = rsqrt(t * t + 1.0), s = t * c;
+#else
       const double c = 1.0 / sqrt(t * t + 1.0), s = t * c;
-      // a <- R^T a R with R = identity except R_pp = R_qq = c, R_pq = s, R_qp = -s
-      for (int k = 0; k < 3; ++k) {  // columns p, q
-        const double akp = a[k][p], akq = a[k][q];
-        a[k][p] = c * akp - s * akq;
-        a[k][q] = s * akp + c * akq;
-      }
-      for (int k = 0; k < 3; ++k) {  // rows p, q
-        const double apk = a[p][k], aqk = a[q][k];
-        a[p][k] = c * apk - s * aqk;
-        a[q][k] = s * apk + c * aqk;
-      }
-      for (int k = 0; k < 3; ++k) {
-        const double vkp = V[k][p], vkq = V[k][q];
-        V[k][p] = c * vkp - s * vkq;
-        V[k][q] = s * vkp + c * vkq;
+#endif
+      // a <- R^T a R with R = identity except R_pp = R_qq = c, R_pq = s, R_qp = -s; with the third index k
+      // only a_pp, a_qq, a_kp and a_kq change, and a_pq becomes zero
+      const int k = 3 - p - q;
+      const double akp = a[k][p], akq = a[k][q];
+      a[p][p] -= t * apq;
+      a[q][q] += t * apq;
+      a[p][q] = a[q][p] = 0.0;
+      a[k][p] = a[p][k] = c * akp - s * akq;
+      a[k][q] = a[q][k] = s * akp + c * akq;
+      for (int i = 0; i < 3; ++i) {
+        const double vip = V[i][p], viq = V[i][q];
+        V[i][p] = c * vip - s * viq;
+        V[i][q] = s * vip + c * viq;
       }
     }
     if (!rotated) break;
@@ -120,6 +131,17 @@ FNE_HD int point(const double e[6], double c_bar, double sp, double mu, double K
   const double Qv = e[0] * e[0] + e[1] * e[1] + e[2] * e[2] + 0.5 * (e[3] * e[3] + e[4] * e[4] + e[5] * e[5]);
   // branch tests (primal values, the reference's order)
   const double f_tr = 2.0 * mu * ((1.0 + sp) * l1 - (1.0 - sp) * l3) + 2.0 * lame * sp * I1 - c_bar;
+  if (f_tr <= 0.0) {  // elastic: lame/2 I1^2 + mu Q, no eigenvectors
+    psi = 0.5 * lame * I1 * I1 + mu * Qv;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      sig[m] = mu * (m < 3 ? 2.0 * e[m] : e[m]) + (m < 3 ? lame * I1 : 0.0);
+#pragma unroll
+      for (int n = 0; n < 6; ++n)
+        D[m][n] = (m == n ? mu * (m < 3 ? 2.0 : 1.0) : 0.0) + (m < 3 && n < 3 ? lame : 0.0);
+    }
+    return 0;
+  }
   const double g_sl = (l1 - l2) / fmax(tiny, 1.0 + sp), g_sr = (l2 - l3) / fmax(tiny, 1.0 - sp);
   const double g_la = (l1 + l2 - 2.0 * l3) / fmax(tiny, 3.0 - sp), g_ra = (2.0 * l1 - l2 - l3) / fmax(tiny, 3.0 + sp);
   // raw denominators (they weight the return terms) and their signed-tiny
@@ -138,8 +160,7 @@ FNE_HD int point(const double e[6], double c_bar, double sp, double mu, double K
   auto lin = [&](const double a[4]) { return a[0] * l1 + a[1] * l2 + a[2] * l3 + a[3] * I1 - c_bar; };
   const double lam_s = f_tr / d_s, lam_l = lin(al) / d_l, lam_r = lin(ar) / d_r;
   int br;
-  if (f_tr <= 0.0) br = 0;
-  else if (lam_s <= fmin(g_sl, g_sr)) br = 1;
+  if (lam_s <= fmin(g_sl, g_sr)) br = 1;
   else if (g_sl < g_sr && lam_l >= g_sl && lam_l <= g_la) br = 2;
   else if (g_sl > g_sr && lam_r >= g_sr && lam_r <= g_ra) br = 3;
   else br = 4;
@@ -172,10 +193,10 @@ FNE_HD int point(const double e[6], double c_bar, double sp, double mu, double K
     psi = 0.5 * lame * I1 * I1;
     Fz[3] += lame * I1;
     add_quad(3, 3, lame);
-    if (br <= 1) {
+    if (br == 1) {
       psi += mu * Qv;
       wQ = mu;
-      if (br == 1) add_neg_sq(as, r_s, d_s);
+      add_neg_sq(as, r_s, d_s);
     } else if (br == 2) {  // mu (l3^2 + (l1 + l2)^2 / 2)
       psi += mu * (l3 * l3 + 0.5 * (l1 + l2) * (l1 + l2));
       Fz[2] += 2.0 * mu * l3;

@@ -619,9 +619,11 @@ int build_block_plan(int64_t n_local, int npn, int bs, const int64_t* elem_dofs,
     }
   }
   P.blk.resize(blk_node.size());
+  if (bs == 3) P.blk_rn.resize(blk_node.size());  // (the 3-D families use it)
   for (size_t b = 0; b < blk_node.size(); ++b) {
     const int32_t c = cnt[b + 1] - cnt[b];
     if (c >= (1 << 13)) return set_error(FNE_EBOUNDS, "block plan: more than 8191 contributions to one block");
+    if (bs == 3) P.blk_rn[b] = rn_of[blk_node[b]];
     P.blk[b] = blk_word[b] | ((uint32_t)c << 19);
   }
   P.rn_blk = std::move(rn_blk);

@@ -176,3 +176,45 @@ def test_mc3d_separate_callbacks_and_rank_split():
         np.testing.assert_allclose(hp.cpu().numpy(), h[pos], rtol=0, atol=1e-12 * np.abs(h).max())
     # the element energies are split by ownership; the load term by owned rows
     assert abs(energies - e) <= 1e-11 * max(1.0, abs(e))
+
+
+@pytest.mark.parametrize("degree,n", [(1, (4, 2, 3)), (2, (2, 1, 3)), (4, (1, 1, 3))])
+def test_mc3d_pattern_wider_than_the_element_graph(degree, n):
+    """A COO pattern with extra node blocks, not symmetric: the element graph's
+    values are those of the plain pattern (the same sums in the same order,
+    mirrored blocks included), the extra entries are zero."""
+    from scipy import sparse
+
+    from fenics_nonlinear_energies_b200.assembler import SlopeStability3DCudaAssembler
+    from oracle.layout import element_adjacency
+
+    p = meshes.slope3d_problem(nx=n[0], ny=n[1], nz=n[2], degree=degree, lam=1.2)
+    free = np.asarray(p["freedofs"])
+    adj = element_adjacency(p["elems"], free, p["u_0"].size).tocsr()
+    node = free // 3
+    full_nodes = np.flatnonzero(np.bincount(node) == 3)
+    rng = np.random.default_rng(degree)
+    extra_r, extra_c = rng.choice(full_nodes, 12), rng.choice(full_nodes, 12)
+    rows, cols = [], []
+    for a, b in zip(extra_r, extra_c):
+        ra, cb = np.flatnonzero(node == a), np.flatnonzero(node == b)
+        rows.append(np.repeat(ra, 3))
+        cols.append(np.tile(cb, 3))
+    rows, cols = np.concatenate(rows), np.concatenate(cols)
+    wide = (adj + sparse.coo_matrix((np.ones(rows.size), (rows, cols)), shape=adj.shape)).tocsr()
+    wide.data[:] = 1.0
+    u = 4e-2 * rng.standard_normal(free.size)
+    plain = SlopeStability3DCudaAssembler(p)
+    wider = SlopeStability3DCudaAssembler(p, adjacency=wide)
+    out = {}
+    for name, asm in (("plain", plain), ("wider", wider)):
+        asm.owned_values.fill_(7.0)
+        _, g, h = asm.eval(torch.as_tensor(u, device="cuda"), 7)
+        lay = asm.layout
+        out[name] = (g.cpu().numpy(), sparse.csr_matrix((h.cpu().numpy(), (lay.owned_rows, lay.owned_cols)),
+                                                        shape=adj.shape))
+    np.testing.assert_array_equal(out["plain"][0], out["wider"][0])
+    assert out["wider"][1].nnz > out["plain"][1].nnz
+    assert abs(out["wider"][1] - out["plain"][1]).max() == 0.0
+    sym = out["plain"][1]
+    assert abs(sym - sym.T).max() <= 1e-12 * abs(sym).max()
