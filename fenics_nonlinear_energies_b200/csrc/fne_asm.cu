@@ -495,6 +495,7 @@ __device__ void energy_finalize(double v, const EnergyOut& eo) {
   if (!is_last) return;
   __threadfence();
   double s = 0.0;
+#pragma unroll 16
   for (int j = threadIdx.x; j < (int)gridDim.x; j += blockDim.x) s += __ldcg(eo.partials + j);
   s = block_sum(s, ws);
   if (threadIdx.x == 0) {
@@ -658,6 +659,262 @@ __global__ void __launch_bounds__(kTetRows) k_rows_tet(RowArgs A, const Chunk* _
 #pragma unroll
       for (int s2 = 1; s2 < G; ++s2) v += sacc[s2 * clen + j];
       hess[cs + j] = (HOut)v;
+    }
+  }
+  if (WANT & W_E) energy_finalize(eacc, eo);
+}
+
+// ---------------------------------------------------------------------------
+// Node-row kernel (P1 tets, default): a CTA owns a run of consecutive row nodes
+// (a contiguous slice of the COO values) and has one thread per (node, incident
+// tet): it evaluates the tet once and forms the node's three gradient entries
+// and its 3 x 12 strip of Hessian values into shared memory.  Then three lanes
+// per output block (one per row) add the block's entries of the incident strips
+// in element order, and the slice leaves shared memory in coalesced stores.  No
+// atomics; bit-reproducible.
+//
+// Why: one thread per DOF row (k_rows_tet) evaluates every tet twelve times,
+// 615 FP64 operations a row node and tet; per row node it is 270 (F, its
+// cofactor and the four cofactor-gradient products serve three rows).  What
+// remains is the rate at which an SM looks up scattered lines, so the tile's
+// nodal values (some 60 nodes for 480 references) and its block list are
+// fetched once into shared memory, and the incidences of a tile are sorted by
+// element, so that neighbouring threads read neighbouring records (those that
+// carry a tet's energy first, so that one warp in four evaluates logarithms).
+// Four persistent CTAs per SM walk the tiles; a tile's incidence words and node
+// codes are loaded one tile ahead, which leaves one round of dependent loads
+// per tile.  kNodeT = 128 threads: five interior nodes of a Kuhn mesh (24 tets
+// each) fill 120.
+// ---------------------------------------------------------------------------
+constexpr int kNodeT = 128;
+constexpr int kNodeRounds = 3;              // block rows per thread
+constexpr int kNodeUni = 128;               // nodes a tile refers to
+constexpr int kNodeBlob = 256;              // 16-byte units of a tile's block list
+constexpr int kStrip = 39;                  // values per strip: 36 Hessian, 3 gradient; odd: conflict-free stores
+struct alignas(16) NodeTile {
+  int inc0, n_inc;   // incidences: one thread each
+  int uni0, n_uni;   // nodes referred to
+  int node0, n_node; // row nodes
+  int blob0;         // block list (16-byte units): n_blk descriptors, then the contribution codes
+  int n_blob, n_blk;
+  int pos0, n_pos;   // COO slice
+  int pad;
+};
+struct NodeTetArgs {
+  const NodeTile* __restrict__ tile;
+  const uint2* __restrict__ inc;           // x: tet * 8 + local node * 2 + energy flag; y: places of its 4 nodes, 8 bits each
+  const int* __restrict__ uni;             // gather codes
+  const uint4* __restrict__ blob;          // per block, most contributions first: x: first code | codes << 16; y, z: place of
+                                           // its rows in the slice, 16 bits each (0xFFFF: none), free components << 16 of z,
+                                           // w: row node of a node's own block, else -1; then 16-bit codes: incidence * 4 +
+                                           // column's local node
+  const int* __restrict__ rn_gpos;         // [node * 3 + c] gradient slot, -1
+  const double* __restrict__ u;
+  const double* __restrict__ dir;
+  const double* __restrict__ rhs;          // may be null
+  long long lo;
+  int nrec, n_tiles;
+};
+
+// geometry of a tet without its nodes
+__device__ __forceinline__ void load_tet_geometry(const Chunk* __restrict__ R, int n, int e, TetElem<float>& t) {
+  const float4 x = ldc_f(R, (long long)n + e), y = ldc_f(R, 2LL * n + e), z = ldc_f(R, 3LL * n + e);
+  const float4 v = ldc_f(R, 4LL * n + e);
+  t.g[0][0] = x.x; t.g[1][0] = x.y; t.g[2][0] = x.z; t.g[3][0] = x.w;
+  t.g[0][1] = y.x; t.g[1][1] = y.y; t.g[2][1] = y.z; t.g[3][1] = y.w;
+  t.g[0][2] = z.x; t.g[1][2] = z.y; t.g[2][2] = z.z; t.g[3][2] = z.w;
+  t.vol = v.x;
+}
+__device__ __forceinline__ void load_tet_geometry(const Chunk* __restrict__ R, int n, int e, TetElem<double>& t) {
+  const double2 a = ldc_d(R, 1LL * n + e), b = ldc_d(R, 2LL * n + e), c = ldc_d(R, 3LL * n + e);
+  const double2 d = ldc_d(R, 4LL * n + e), f = ldc_d(R, 5LL * n + e), g = ldc_d(R, 6LL * n + e);
+  t.vol = ldc_d(R, 7LL * n + e).x;
+  t.g[0][0] = a.x; t.g[1][0] = a.y; t.g[2][0] = b.x; t.g[3][0] = b.y;
+  t.g[0][1] = c.x; t.g[1][1] = c.y; t.g[2][1] = d.x; t.g[3][1] = d.y;
+  t.g[0][2] = f.x; t.g[1][2] = f.y; t.g[2][2] = g.x; t.g[3][2] = g.y;
+}
+
+template <typename Real>
+struct NodeSmem {
+  double u[kNodeUni][3];
+  uint4 blob[kNodeBlob];
+  int4 tile[3][3];              // this tile and the two that follow
+  Real strip[kNodeT * kStrip];  // then the COO slice
+};
+
+template <typename Real, int WANT, typename HOut>
+__global__ void __launch_bounds__(kNodeT, 4) k_nodes_tet(NodeTetArgs A, const Chunk* __restrict__ R, Phys P,
+                                                         double* __restrict__ grad, HOut* __restrict__ hess,
+                                                         EnergyOut eo) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  NodeSmem<Real>& M = *reinterpret_cast<NodeSmem<Real>*>(smem_raw);
+  const int tid = threadIdx.x;
+  const int4* tiles = reinterpret_cast<const int4*>(A.tile);
+  double eacc = 0.0;
+  if (tid < 6 && (int)blockIdx.x + (tid / 3) * (int)gridDim.x < A.n_tiles)
+    M.tile[tid / 3][tid % 3] = __ldg(tiles + 3LL * (blockIdx.x + (tid / 3) * gridDim.x) + tid % 3);
+  __syncthreads();
+  uint2 nw = make_uint2(0u, 0u);  // the next tile's incidence and node code of this thread
+  int ncode = 0;
+  auto ahead = [&](int slot) {
+    const NodeTile& N = *reinterpret_cast<const NodeTile*>(M.tile[slot]);
+    if (tid < N.n_inc) nw = __ldg(A.inc + N.inc0 + tid);
+    if (tid < N.n_uni) ncode = __ldg(A.uni + N.uni0 + tid);
+  };
+  ahead(0);
+  int slot = 0;
+  for (int k = blockIdx.x; k < A.n_tiles; k += gridDim.x) {
+    const NodeTile T = *reinterpret_cast<const NodeTile*>(M.tile[slot]);
+    const bool on = tid < T.n_inc;
+    const uint2 w = nw;
+    const int code = ncode;
+    TetElem<Real> t;
+    if (on) load_tet_geometry(R, A.nrec, (int)(w.x >> 3), t);
+    double uv[3];
+    if (tid < T.n_uni)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) uv[d] = gather(A.u, A.dir, code, d);
+    uint4 bl[kNodeBlob / kNodeT];
+#pragma unroll
+    for (int i = 0; i < kNodeBlob / kNodeT; ++i)
+      if (tid + i * kNodeT < T.n_blob) bl[i] = __ldg(A.blob + T.blob0 + tid + i * kNodeT);
+    int4 nt;
+    const bool two = tid < 3 && k + 2 * (int)gridDim.x < A.n_tiles;
+    if (two) nt = __ldg(tiles + 3LL * (k + 2 * gridDim.x) + tid);
+    const int s1 = slot == 2 ? 0 : slot + 1, s2 = s1 == 2 ? 0 : s1 + 1;
+    if (k + (int)gridDim.x < A.n_tiles) ahead(s1);
+    if (tid < T.n_uni)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) M.u[tid][d] = uv[d];
+#pragma unroll
+    for (int i = 0; i < kNodeBlob / kNodeT; ++i)
+      if (tid + i * kNodeT < T.n_blob) M.blob[tid + i * kNodeT] = bl[i];
+    if (two) M.tile[s2][tid] = nt;
+    slot = s1;
+    __syncthreads();
+    if (on) {
+      const int a = (int)(w.x >> 1) & 3;
+      Real y[4][3];
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) y[b][d] = (Real)M.u[(w.y >> (8 * b)) & 255u][d];
+      HeState<Real> S;
+      he_state(P, y, t, S);
+      if ((WANT & W_E) && (w.x & 1u)) {
+        if constexpr (sizeof(Real) == 8) {  // he_energy's terms from the state at hand
+          double I1 = 0.0;
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) I1 += S.F[i][j] * S.F[i][j];
+          const double J = P.absdet ? fabs(S.J) : S.J;
+          eacc += (P.C1 * (I1 - 3.0 - 2.0 * log(J)) + P.D1 * (J - 1.0) * (J - 1.0)) * t.vol;
+        } else {
+          double yd[4][3];
+#pragma unroll
+          for (int b = 0; b < 4; ++b)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) yd[b][d] = M.u[(w.y >> (8 * b)) & 255u][d];
+          eacc += he_energy<Real>(P, yd, t);
+        }
+      }
+      Real ga[3], cga[3];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) ga[j] = a == 0 ? t.g[0][j] : (a == 1 ? t.g[1][j] : (a == 2 ? t.g[2][j] : t.g[3][j]));
+#pragma unroll
+      for (int c = 0; c < 3; ++c) cga[c] = S.cof[c][0] * ga[0] + S.cof[c][1] * ga[1] + S.cof[c][2] * ga[2];
+      const Real C1 = prm<Real>(P.C1, P.C1f);
+      Real* o = M.strip + kStrip * tid;
+      if (WANT & W_G) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const Real Pg = Real(2) * C1 * (S.F[c][0] * ga[0] + S.F[c][1] * ga[1] + S.F[c][2] * ga[2]);
+          o[36 + c] = t.vol * (Pg + S.c3 * cga[c]);
+        }
+      }
+      if (WANT & W_H) {
+        const Real k1 = t.vol * Real(2) * C1, k2 = t.vol * S.c2, k3 = t.vol * S.c3;
+        const Real ka[3] = {k2 * cga[0], k2 * cga[1], k2 * cga[2]};
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const Real* gb = t.g[b];
+          const Real kd = k1 * (ga[0] * gb[0] + ga[1] * gb[1] + ga[2] * gb[2]);
+          Real cgb[3];
+#pragma unroll
+          for (int d = 0; d < 3; ++d) cgb[d] = S.cof[d][0] * gb[0] + S.cof[d][1] * gb[1] + S.cof[d][2] * gb[2];
+          const Real x0 = ga[1] * gb[2] - ga[2] * gb[1];
+          const Real x1 = ga[2] * gb[0] - ga[0] * gb[2];
+          const Real x2 = ga[0] * gb[1] - ga[1] * gb[0];
+          Real q[3];  // k3 F (g_a x g_b), entering as eps_cdm q_m
+#pragma unroll
+          for (int m = 0; m < 3; ++m) q[m] = k3 * (S.F[m][0] * x0 + S.F[m][1] * x1 + S.F[m][2] * x2);
+          o[9 * b + 0] = ka[0] * cgb[0] + kd;
+          o[9 * b + 1] = ka[0] * cgb[1] + q[2];
+          o[9 * b + 2] = ka[0] * cgb[2] - q[1];
+          o[9 * b + 3] = ka[1] * cgb[0] - q[2];
+          o[9 * b + 4] = ka[1] * cgb[1] + kd;
+          o[9 * b + 5] = ka[1] * cgb[2] + q[0];
+          o[9 * b + 6] = ka[2] * cgb[0] + q[1];
+          o[9 * b + 7] = ka[2] * cgb[1] - q[0];
+          o[9 * b + 8] = ka[2] * cgb[2] + kd;
+        }
+      }
+    }
+    __syncthreads();
+    const unsigned short* codes = reinterpret_cast<const unsigned short*>(M.blob + T.n_blk);
+    Real val[kNodeRounds][3];
+    unsigned pos[kNodeRounds], free_d[kNodeRounds];
+#pragma unroll
+    for (int r = 0; r < kNodeRounds; ++r) {
+      pos[r] = 0xFFFFu;
+      const int i = r * kNodeT + tid, b = i / 3, c = i - 3 * b;
+      if (b >= T.n_blk) continue;
+      const uint4 bw = M.blob[b];
+      const unsigned short* cd = codes + (bw.x & 0xFFFFu);
+      const int n = (int)(bw.x >> 16);
+      // the node's own block lists all its incidences: its gradient row
+      if ((WANT & (W_G | W_E)) && (int)bw.w >= 0) {
+        const int gp = __ldg(A.rn_gpos + 3 * (int)bw.w + c);
+        if (gp >= 0) {
+          if (WANT & W_G) {
+            Real g = Real(0);
+#pragma unroll 4
+            for (int j = 0; j < n; ++j) g += M.strip[kStrip * (cd[j] >> 2) + 36 + c];
+            grad[gp] = (double)g - (A.rhs ? A.rhs[gp] : 0.0);
+          }
+          if ((WANT & W_E) && A.rhs) eacc -= A.rhs[gp] * A.u[A.lo + gp];
+        }
+      }
+      if (WANT & W_H) {
+        Real v0 = Real(0), v1 = Real(0), v2 = Real(0);
+#pragma unroll 4
+        for (int j = 0; j < n; ++j) {
+          const int e = cd[j];
+          const Real* st = M.strip + kStrip * (e >> 2) + 9 * (e & 3) + 3 * c;
+          v0 += st[0];
+          v1 += st[1];
+          v2 += st[2];
+        }
+        val[r][0] = v0;
+        val[r][1] = v1;
+        val[r][2] = v2;
+        pos[r] = c == 0 ? bw.y & 0xFFFFu : (c == 1 ? bw.y >> 16 : bw.z & 0xFFFFu);
+        free_d[r] = (bw.z >> 16) & 7u;
+      }
+    }
+    __syncthreads();  // strips and block list read
+    if (WANT & W_H) {
+#pragma unroll
+      for (int r = 0; r < kNodeRounds; ++r)
+        if (pos[r] != 0xFFFFu) {
+          int p = (int)pos[r];
+#pragma unroll
+          for (int d = 0; d < 3; ++d)
+            if ((free_d[r] >> d) & 1u) M.strip[p++] = val[r][d];
+        }
+      __syncthreads();
+      for (int j = tid; j < T.n_pos; j += kNodeT) hess[T.pos0 + j] = (HOut)M.strip[j];
     }
   }
   if (WANT & W_E) energy_finalize(eacc, eo);
@@ -1421,6 +1678,12 @@ struct fne_handle {
       *bp_rn_inc = nullptr, *bp_con = nullptr, *bp_inc = nullptr;
   unsigned* bp_blk = nullptr;
   int64_t e2_contrib = 0;
+  // node-row kernel (P1 tets)
+  int n_node_tiles = 0;
+  NodeTile* nt_tile = nullptr;
+  uint2* nt_inc = nullptr;
+  int* nt_uni = nullptr;
+  uint4* nt_blob = nullptr;
   Phys phys{};
   // device buffers
   Chunk* rec = nullptr;
@@ -1477,7 +1740,8 @@ void free_handle(fne_handle* h) {
                   h->dir, h->rhs, h->partials, h->dir_const, h->counter, h->h_u, h->h_grad, h->h_energy,
                   h->h_hess, h->e2_kbuf, h->e2_gbuf, h->bp_rn_blk, h->bp_rn_con, h->bp_rn_row,
                   h->bp_rn_gpos, h->bp_rn_inc, h->bp_con, h->bp_inc, h->bp_blk, h->cl_table,
-                  h->cl_codes, h->cl_reals, h->cl_rows, h->cl_runs, h->cl_incs, h->err};
+                  h->cl_codes, h->cl_reals, h->cl_rows, h->cl_runs, h->cl_incs, h->err,
+                  h->nt_tile, h->nt_inc, h->nt_uni, h->nt_blob};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (h->err_host) cudaFreeHost(h->err_host);
@@ -1666,6 +1930,191 @@ cudaError_t launch_tet_t(fne_handle* h, int want, const RowArgs& A, double* grad
     case 8: return launch_tet_g<Real, HOut, 8>(h, want, A, grad, hess, eo, st, set_attr);
     default: return launch_tet_g<Real, HOut, 1>(h, want, A, grad, hess, eo, st, set_attr);
   }
+}
+
+template <typename Real, typename HOut>
+cudaError_t launch_nodes_t(fne_handle* h, int want, const double* u, double* grad, void* hess, EnergyOut eo,
+                           cudaStream_t st, bool set_attr) {
+  const NodeTetArgs A{h->nt_tile, h->nt_inc, h->nt_uni, h->nt_blob, h->bp_rn_gpos, u,
+                      h->dir,     h->rhs,    h->lo,     h->n_local, h->n_node_tiles};
+  const int grid = std::min(h->n_node_tiles, 4 * h->num_sms);
+  HOut* H = static_cast<HOut*>(hess);
+  constexpr size_t sm = sizeof(NodeSmem<Real>);
+#define FNE_NODE_CASE(W)                                                                              \
+  case W:                                                                                             \
+    if (set_attr)                                                                                     \
+      return cudaFuncSetAttribute(k_nodes_tet<Real, W, HOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
+    k_nodes_tet<Real, W, HOut><<<grid, kNodeT, sm, st>>>(A, h->rec, h->phys, grad, H, eo); \
+    return cudaGetLastError();
+  switch (want) {
+    FNE_NODE_CASE(2)
+    FNE_NODE_CASE(3)
+    FNE_NODE_CASE(4)
+    FNE_NODE_CASE(5)
+    FNE_NODE_CASE(6)
+    FNE_NODE_CASE(7)
+  }
+#undef FNE_NODE_CASE
+  return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_nodes(fne_handle* h, int want, const double* u, double* grad, void* hess, EnergyOut eo,
+                         cudaStream_t st, bool set_attr = false) {
+  if (h->precision == FNE_FP64) return launch_nodes_t<double, double>(h, want, u, grad, hess, eo, st, set_attr);
+  if (h->hess_fp32) return launch_nodes_t<float, float>(h, want, u, grad, hess, eo, st, set_attr);
+  return launch_nodes_t<float, double>(h, want, u, grad, hess, eo, st, set_attr);
+}
+
+// Tiles of the node-row kernel from the node-block plan: runs of row nodes
+// whose incidences, referred nodes, output values and COO slice fit one CTA.
+// False when the pattern does not allow it (a node beyond those limits, rows of
+// a node not contiguous): the row kernel then runs.  Small meshes get smaller
+// tiles, so that every SM has two.  elem_code: gather codes of the tets' nodes.
+struct NodePlan {
+  std::vector<NodeTile> tile;
+  std::vector<uint32_t> inc;   // pairs
+  std::vector<int32_t> uni;
+  std::vector<uint32_t> blob;  // 16-byte units
+};
+bool build_node_plan(const BlockPlan& bp, const std::vector<uint8_t>& weight, const std::vector<int32_t>& elem_code,
+                     int64_t n_free, int64_t n_total, int64_t nnz, int num_sms, NodePlan& Q) {
+  const int n = bp.n_rnodes;
+  if (n == 0 || bp.inc.empty()) return false;
+  const int64_t total = (int64_t)bp.inc.size();
+  const int cap = (int)std::min<int64_t>(kNodeT, std::max<int64_t>(kNodeT / 4, total / (2 * num_sms)));
+  // COO range of every row node: its rows must lie together
+  std::vector<int32_t> pos((size_t)n + 1);
+  for (int k = 0; k < n; ++k) {
+    int32_t first = -1;
+    for (int c = 0; c < 3; ++c)
+      if (bp.rn_row[3 * k + c] >= 0 && (first < 0 || bp.rn_row[3 * k + c] < first)) first = bp.rn_row[3 * k + c];
+    pos[k] = first;
+  }
+  pos[n] = (int32_t)nnz;
+  for (int k = 0; k < n; ++k) {
+    if (pos[k] < 0 || pos[k + 1] < pos[k]) return false;
+    int64_t width = 0, rows = 0;  // entries of one row; rows
+    for (int32_t b = bp.rn_blk[k]; b < bp.rn_blk[k + 1]; ++b) width += __builtin_popcount((bp.blk[b] >> 16) & 7u);
+    for (int c = 0; c < 3; ++c) rows += bp.rn_row[3 * k + c] >= 0;
+    if (pos[k + 1] - pos[k] != rows * width) return false;
+    const auto b0 = bp.blk_rn.begin() + bp.rn_blk[k], b1 = bp.blk_rn.begin() + bp.rn_blk[k + 1];
+    if (std::find(b0, b1, k) == b1) return false;  // the gradient rows go with the node's own block
+  }
+  std::vector<uint8_t> seen(weight.size(), 0);
+  std::vector<int32_t> order, first, node, at_of, uni, sorted;
+  std::vector<uint8_t> flag;
+  // tile that last referred to a node (by gather code), and the node's place in it
+  std::vector<int32_t> mark_free((size_t)n_free, -1), mark_dir((size_t)n_total, -1);
+  std::vector<uint8_t> place_free((size_t)n_free), place_dir((size_t)n_total);
+  std::vector<uint16_t> codes;
+  Q.inc.reserve(2 * total);
+  for (int k = 0; k < n;) {
+    // grow the tile node by node
+    int e = k;
+    uni.clear();
+    while (e < n) {
+      if (bp.rn_inc[e + 1] - bp.rn_inc[k] > (e == k ? kNodeT : cap) ||
+          3 * (bp.rn_blk[e + 1] - bp.rn_blk[k]) > kNodeT * kNodeRounds || pos[e + 1] - pos[k] > kNodeT * kStrip)
+        break;
+      const int64_t n_codes = bp.rn_con[e + 1] - bp.rn_con[k], n_blk = bp.rn_blk[e + 1] - bp.rn_blk[k];
+      if (16 * n_blk + 2 * n_codes > 16 * kNodeBlob) break;
+      const size_t before = uni.size();
+      for (int32_t i = bp.rn_inc[e]; i < bp.rn_inc[e + 1]; ++i)
+        for (int b = 0; b < 4; ++b) {
+          const int32_t code = elem_code[(size_t)(bp.inc[i] / 4) * 4 + b];
+          int32_t& m = code >= 0 ? mark_free[code] : mark_dir[-1 - code];
+          if (m != k) uni.push_back(code);
+          m = k;
+        }
+      if ((int)uni.size() > kNodeUni) {
+        uni.resize(before);
+        break;
+      }
+      ++e;
+    }
+    if (e == k) return false;
+    std::sort(uni.begin(), uni.end());
+    for (size_t i = 0; i < uni.size(); ++i) (uni[i] >= 0 ? place_free[uni[i]] : place_dir[-1 - uni[i]]) = (uint8_t)i;
+    NodeTile t{};
+    t.inc0 = bp.rn_inc[k];
+    t.n_inc = bp.rn_inc[e] - t.inc0;
+    t.uni0 = (int)Q.uni.size();
+    t.n_uni = (int)uni.size();
+    t.node0 = k;
+    t.n_node = e - k;
+    t.n_blk = bp.rn_blk[e] - bp.rn_blk[k];
+    t.pos0 = pos[k];
+    t.n_pos = pos[e] - pos[k];
+    Q.uni.insert(Q.uni.end(), uni.begin(), uni.end());
+    // incidences sorted by element; at_of: place of the plan's i-th incidence
+    sorted.resize(t.n_inc);
+    for (int i = 0; i < t.n_inc; ++i) sorted[i] = i;
+    flag.resize(t.n_inc);
+    for (int i = 0; i < t.n_inc; ++i) {  // the energy of a tet goes with its first incidence
+      const int32_t el = bp.inc[t.inc0 + i] / 4;
+      flag[i] = weight[el] && !seen[el];
+      seen[el] = 1;
+    }
+    std::sort(sorted.begin(), sorted.end(), [&](int x, int y) {
+      return flag[x] != flag[y] ? flag[x] > flag[y] : bp.inc[t.inc0 + x] < bp.inc[t.inc0 + y];
+    });
+    at_of.resize(t.n_inc);
+    for (int i = 0; i < t.n_inc; ++i) {
+      at_of[sorted[i]] = i;
+      const int32_t code = bp.inc[t.inc0 + sorted[i]], el = code / 4;
+      uint32_t places = 0;
+      for (int b = 0; b < 4; ++b) {
+        const int32_t ec = elem_code[(size_t)el * 4 + b];
+        places |= (uint32_t)(ec >= 0 ? place_free[ec] : place_dir[-1 - ec]) << (8 * b);
+      }
+      Q.inc.push_back((uint32_t)code * 2u + flag[sorted[i]]);
+      Q.inc.push_back(places);
+    }
+    // blocks with the most contributions first: their longer sums start together
+    first.resize(t.n_blk);
+    node.resize(t.n_blk);
+    order.resize(t.n_blk);
+    const int b0 = bp.rn_blk[k];
+    for (int q = k; q < e; ++q) {
+      int32_t at = bp.rn_con[q];
+      for (int32_t b = bp.rn_blk[q]; b < bp.rn_blk[q + 1]; ++b) {
+        order[b - b0] = b - b0;
+        first[b - b0] = at;
+        node[b - b0] = q;
+        at += (int32_t)(bp.blk[b] >> 19);
+      }
+    }
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int x, int y) { return bp.blk[b0 + x] >> 19 > bp.blk[b0 + y] >> 19; });
+    t.blob0 = (int)(Q.blob.size() / 4);
+    codes.clear();
+    for (const int32_t x : order) {
+      const uint32_t w = bp.blk[b0 + x], cnt = w >> 19;
+      const int q = node[x];
+      uint32_t place[3];  // (a slice has fewer than 0xFFFF values)
+      for (int c = 0; c < 3; ++c)
+        place[c] = bp.rn_row[3 * q + c] < 0 ? 0xFFFFu : (uint32_t)(bp.rn_row[3 * q + c] - t.pos0) + (w & 0xFFFFu);
+      Q.blob.push_back((uint32_t)codes.size() | cnt << 16);
+      Q.blob.push_back(place[0] | place[1] << 16);
+      Q.blob.push_back(place[2] | (w & 0x70000u));
+      Q.blob.push_back(bp.blk_rn[b0 + x] == q ? (uint32_t)q : 0xFFFFFFFFu);
+      const auto i1 = bp.inc.begin() + bp.rn_inc[q + 1];
+      auto it = bp.inc.begin() + bp.rn_inc[q];
+      for (uint32_t j = 0; j < cnt; ++j) {
+        const int32_t con = bp.con[first[x] + j], ea = con / 4, bb = con - 4 * ea;  // el * 4 + a, b
+        it = std::lower_bound(it, i1, ea);  // both lists run in element order
+        if (it == i1 || *it != ea) return false;
+        codes.push_back((uint16_t)(at_of[it - bp.inc.begin() - t.inc0] * 4 + bb));
+      }
+    }
+    for (size_t i = 0; i < codes.size(); i += 2)
+      Q.blob.push_back(codes[i] | (i + 1 < codes.size() ? (uint32_t)codes[i + 1] << 16 : 0u));
+    while (Q.blob.size() % 4) Q.blob.push_back(0u);
+    t.n_blob = (int)(Q.blob.size() / 4) - t.blob0;
+    Q.tile.push_back(t);
+    k = e;
+  }
+  return true;
 }
 
 template <typename Real, typename HOut>
@@ -1862,7 +2311,9 @@ extern "C" int fne_create(const fne_desc* d, fne_handle** out) {
     return set_error(FNE_EINVAL, "fne_create: p-Laplace needs p > 1");
 
   RowPlan plan;
-  int rc = build_row_plan(d, plan);
+  // tets by default: tiles of whole row nodes, which need no incidence words
+  const bool try_nodes = d->family == FNE_NEOHOOKEAN && d->kernel_variant == 0;
+  int rc = build_row_plan(d, plan, !try_nodes);
   if (rc) return rc;
   const bool f32 = d->precision == FNE_FP32;
   const size_t real_size = f32 ? sizeof(float) : sizeof(double);
@@ -1872,6 +2323,20 @@ extern "C" int fne_create(const fne_desc* d, fne_handle** out) {
   cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev_id);
   cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev_id);
   if (smem_optin <= 0) smem_optin = 227 * 1024;
+  BlockPlan nbp;
+  NodePlan nplan;
+  bool use_nodes = false;
+  if (try_nodes) {
+    const int64_t nl = (int64_t)plan.local_elems.size();
+    if (plan.n_rows > 0 && nl * 16 < (int64_t)INT32_MAX) {
+      std::vector<int64_t> edofs((size_t)nl * 12);
+      for (int64_t le = 0; le < nl; ++le)
+        std::copy_n(d->elems + plan.local_elems[le] * 12, 12, edofs.begin() + le * 12);
+      use_nodes = build_block_plan(nl, 4, 3, edofs.data(), d, nbp) == FNE_OK &&
+                  build_node_plan(nbp, plan.elem_weight, plan.elem_code, d->n_free, d->n_total, d->nnz, n_sms, nplan);
+    }
+    if (!use_nodes && (rc = build_row_plan(d, plan, true))) return rc;
+  }
   // banded sweep for triangles (default), incidence-parallel on request,
   // else the row-gather kernel
   IncPlan inc;
@@ -2153,6 +2618,22 @@ extern "C" int fne_create(const fne_desc* d, fne_handle** out) {
       h->e2_gbuf = gb;
     }
   }
+  if (use_nodes) {
+    h->n_node_tiles = (int)nplan.tile.size();
+    h->n_inc = (int64_t)nbp.inc.size();
+    FNE_TRY(upload(h, &h->bp_rn_gpos, nbp.rn_gpos.data(), nbp.rn_gpos.size()));
+    FNE_TRY(upload(h, &h->nt_tile, nplan.tile.data(), nplan.tile.size()));
+    FNE_TRY(upload(h, &h->nt_inc, reinterpret_cast<const uint2*>(nplan.inc.data()), nplan.inc.size() / 2));
+    FNE_TRY(upload(h, &h->nt_uni, nplan.uni.data(), nplan.uni.size()));
+    FNE_TRY(upload(h, &h->nt_blob, reinterpret_cast<const uint4*>(nplan.blob.data()), nplan.blob.size() / 4));
+    for (int want = 2; want <= 7; ++want) {
+      cudaError_t e = launch_nodes(h, want, nullptr, nullptr, nullptr, EnergyOut{}, 0, true);
+      if (e != cudaSuccess) {
+        free_handle(h);
+        return cuda_fail(e, "cudaFuncSetAttribute");
+      }
+    }
+  }
   FNE_TRY(upload(h, &h->dir, d->dirichlet, (size_t)d->n_total));
   if (d->rhs_owned) FNE_TRY(upload(h, &h->rhs, d->rhs_owned, (size_t)(d->hi - d->lo)));
   FNE_TRY(dalloc(h, &h->partials, (size_t)h->n_partials));
@@ -2305,7 +2786,8 @@ extern "C" int fne_eval(fne_handle* h, const double* u, int flags, double* energ
                  h->sw_ent_ptr,  h->sw_inc_base,  h->sw_ent_row,    h->sw_ent_pos,
                  h->sw_ent_meta, h->sw_inc_word,  h->sweep_win_mask, h->sweep_rwin_mask,
                  h->sw_gpos_identity, h->sw_eoff, h->sw_row_of};
-    e = h->use_elem2 ? launch_elem2(h, flags, u, grad, hess, eo, st)
+    e = h->n_node_tiles ? launch_nodes(h, flags, u, grad, hess, eo, st)
+        : h->use_elem2 ? launch_elem2(h, flags, u, grad, hess, eo, st)
                      : launch_rows(h, flags, A, Q, SW, grad, hess, eo, st, false);
     // stream-ordered copy of the status word for fne_poll_device_status
     if (e == cudaSuccess && h->use_cluster)

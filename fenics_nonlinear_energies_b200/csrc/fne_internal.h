@@ -71,7 +71,8 @@ struct RowPlan {
 
 // Builds the plan for node-uniform problems (every node has all or none of
 // its block_size DOFs free).  Returns FNE_OK or an error (set_error called).
-int build_row_plan(const fne_desc* d, RowPlan& P);
+// incidences = false stops before the incidence words (inc_* stay empty).
+int build_row_plan(const fne_desc* d, RowPlan& P, bool incidences = true);
 
 // Incidence-parallel plan (scalar P1 triangles): one thread per
 // (row, element) incidence.  CTA c owns rows [cta_row[c], cta_row[c+1]) and

@@ -17,7 +17,7 @@
 
 namespace fne {
 
-int build_row_plan(const fne_desc* d, RowPlan& P) {
+int build_row_plan(const fne_desc* d, RowPlan& P, bool incidences) {
   const int npe = d->npe, bs = d->block_size, nde = npe * bs;
   const int64_t E = d->n_elem, lo = d->lo, hi = d->hi, nf = d->n_free;
   if (npe < 1 || bs < 1 || bs > 3 || kOffShift + kOffBits * npe > 32)
@@ -149,6 +149,11 @@ int build_row_plan(const fne_desc* d, RowPlan& P) {
     return set_error(FNE_EBOUNDS, "row plan: a row has more than 126 entries");
   const int32_t n_nodes = (int32_t)node_of.size();
   P.n_nodes = n_nodes;
+
+  P.inc_ptr.clear();
+  P.inc_elem.clear();
+  P.inc_info.clear();
+  if (!incidences) return FNE_OK;
 
   // rows of each node (to validate identical column layouts)
   std::vector<std::vector<int32_t>> node_rows(n_nodes);
@@ -590,6 +595,7 @@ int build_block_plan(int64_t n_local, int npn, int bs, const int64_t* elem_dofs,
   std::vector<int32_t> icnt(n_rn + 1, 0), ifill;
   std::vector<int32_t> con, inc;
   P.elem_rn.assign((size_t)n_local * npn, -1);
+  std::vector<int32_t> found((size_t)n_local * npn * npn, -1);  // block of every (element, a, b), found once
   for (int pass = 0; pass < 2; ++pass) {
     if (pass == 1) {
       for (size_t b = 0; b < blk_node.size(); ++b) cnt[b + 1] += cnt[b];
@@ -610,10 +616,15 @@ int build_block_plan(int64_t n_local, int npn, int bs, const int64_t* elem_dofs,
         if (pass == 0) icnt[k + 1]++; else inc[ifill[k]++] = (int32_t)(el * npn + a);
         for (int b = 0; b < npn; ++b) {
           const int64_t nb = ed[b * bs] / bs;
+          int32_t& blk = found[((size_t)el * npn + a) * npn + b];
+          if (pass == 1) {
+            if (blk >= 0) con[fill[blk]++] = (int32_t)((el * npn + a) * npn + b);
+            continue;
+          }
           if (!has_free(nb)) continue;
-          const int32_t blk = find_blk(k, nb);
+          blk = find_blk(k, nb);
           if (blk < 0) return set_error(FNE_ELAYOUT, "Scatter lookup found mismatched owned COO entries");
-          if (pass == 0) cnt[blk + 1]++; else con[fill[blk]++] = (int32_t)((el * npn + a) * npn + b);
+          cnt[blk + 1]++;
         }
       }
     }

@@ -184,8 +184,10 @@ typedef struct {
                                  * 7 = banded sweep; 8 = persistent row-cluster
                                  * kernel (TMA-staged; the banded sweep when
                                  * the mesh does not fit its packed format).
-                                 * P1 tets: 0 = row-gather with automatic lanes
-                                 * per row; 1 = row-gather, one lane per row;
+                                 * P1 tets: 0 = row-gather over tiles of whole
+                                 * row nodes where the pattern fits them, else
+                                 * with automatic lanes per row; 1 = row-gather,
+                                 * one lane per row;
                                  * 2 = element-parallel pass + node-block
                                  * gather; 4 / 5 / 6 = row-gather with 2 / 4 / 8
                                  * lanes per row.
@@ -213,7 +215,9 @@ typedef struct {
                            * 10 row clusters (P1 triangles),
                            * 11 3-D Mohr-Coulomb point-tile element kernel +
                            * node-block gather */
-  int32_t row_lanes;      /* lanes per output row of the tet row kernel, else 1 */
+  int32_t row_lanes;      /* lanes per output row of the tet row kernel (for
+                           * kernel_variant 0 the count it would run with where
+                           * the tiles of row nodes do not apply), else 1 */
 } fne_info;
 
 int fne_create(const fne_desc* desc, fne_handle** out);

@@ -372,3 +372,35 @@ def test_cluster_kernel_is_bit_reproducible(precision):
     b = gpu.eval(ut, 7)
     for x, y in zip(a, b):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("size,shuffle", [((2, 1, 1), False), ((5, 3, 2), True), ((9, 4, 5), False), ((9, 4, 5), True)])
+def test_he_node_tiles_match_row_gather(size, shuffle, precision):
+    """The default tet kernel (tiles of whole row nodes) against the row-gather
+    kernel: tiles that are not full, elements in any order, nodes in any order
+    (neighbours scattered over tiles); FP64 1e-12, FP32 2e-5, bit-repeatable,
+    separate outputs equal to the fused ones."""
+    params, y0 = meshes.he_beam_problem(nx=size[0], ny=size[1], nz=size[2])
+    rng = np.random.default_rng(sum(size))
+    if shuffle:
+        order = rng.permutation(params["elems"].shape[0])
+        for k in ("elems", "elems_scalar", "dphix", "dphiy", "dphiz", "vol"):
+            params[k] = params[k][order]
+    cls = _asm_classes()["he"]
+    hd = torch.float32 if precision == "fp32" else torch.float64
+    kw = {"precision": precision, "hess_dtype": hd}
+    if shuffle:
+        kw.update(perm_override=(3 * rng.permutation(y0.size // 3)[:, None] + np.arange(3)).ravel())
+    a, b = cls(params, **kw), cls(params, kernel_variant="row_gather", **kw)
+    # a twentieth of the smallest cell edge: no inverted tets
+    y = y0 + 0.05 * min(0.4 / size[0], 0.02 / size[1], 0.02 / size[2]) * rng.standard_normal(y0.size)
+    u = torch.as_tensor(y[np.asarray(a.layout.perm)], device="cuda")
+    ea, ga, ha = [t.clone() for t in a.eval(u, 7)]
+    eb, gb, hb = [t.clone() for t in b.eval(u, 7)]
+    assert abs(float(ea.item()) - float(eb.item())) <= 1e-12 * max(1e-3, abs(float(eb.item())))
+    assert _rel(ha.double().cpu().numpy(), hb.double().cpu().numpy()) <= (FP64_TOL if precision == "fp64" else FP32_TOL)
+    assert _rel(ga.cpu().numpy(), gb.cpu().numpy()) <= (FP64_TOL if precision == "fp64" else 1e-4)
+    for flags, k in ((2, 1), (4, 2), (3, 1), (5, 2), (6, 2)):
+        assert torch.equal(a.eval(u, flags)[k], (ea, ga, ha)[k])
+    assert all(torch.equal(x, y) for x, y in zip(a.eval(u, 7), (ea, ga, ha)))
