@@ -168,8 +168,8 @@ class DeviceCG:
                                          ctypes.byref(its), ctypes.byref(why), self._stream()))
         self.reason = self.REASONS[why.value]
         # one initialisation kernel, then graphs of `chunk` iterations of two
-        # kernels until the iteration that stopped the solve
-        self.launches += 1 + 2 * self.chunk * (-(-int(its.value) // self.chunk))
+        # kernels and a state kernel until the one that holds the stop
+        self.launches += 1 + (2 * self.chunk + 1) * max(1, -(-int(its.value) // self.chunk))
         return x, int(its.value)
 
     def close(self):

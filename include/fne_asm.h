@@ -344,8 +344,10 @@ int fne_cg_set_matrix(fne_cg* cg, const void* coo_vals, void* stream);
  * (returning the last iterate, or b itself at the first iteration), or after
  * maxit iterations.  *its = iterations taken (1 for the first-iteration
  * curvature stop, 0 for b = 0); *reason = 0 converged, 1 non-positive
- * curvature, 2 iteration limit, 3 zero right-hand side.  Synchronises the
- * stream once per `chunk` iterations; a handle runs one solve at a time. */
+ * curvature, 2 iteration limit, 3 zero right-hand side.  Waits for the state
+ * once per `chunk` iterations; on return up to one graph of kernels that change
+ * nothing and the copy to x may still be in the stream.  A handle runs one solve
+ * at a time (a later solve on another stream waits for this one). */
 int fne_cg_solve(fne_cg* cg, const double* b, double* x, double rtol, int32_t maxit, int32_t* its, int32_t* reason,
                  void* stream);
 int fne_cg_destroy(fne_cg* cg);
