@@ -246,19 +246,32 @@ __device__ __forceinline__ void rowgrad_node(int A, const int* __restrict__ rn_i
                                              const int* __restrict__ rn_gpos, const Real* __restrict__ gbuf,
                                              const double* __restrict__ rhs, double* __restrict__ grad) {
   Real gs[BS];
-#pragma unroll
-  for (int c = 0; c < BS; ++c) gs[c] = Real(0);
-  const int i1 = __ldg(rn_inc + A + 1);
-  for (int i = __ldg(rn_inc + A); i < i1; ++i) {
-    const long long code = __ldg(inc + i);
-#pragma unroll
-    for (int c = 0; c < BS; ++c) gs[c] += gbuf[code * BS + c];
-  }
+  int gp[BS];
+  const int i0 = __ldg(rn_inc + A), i1 = __ldg(rn_inc + A + 1);
 #pragma unroll
   for (int c = 0; c < BS; ++c) {
-    const int gp = __ldg(rn_gpos + A * BS + c);
-    if (gp >= 0) grad[gp] = (double)gs[c] - (rhs ? rhs[gp] : 0.0);
+    gs[c] = Real(0);
+    gp[c] = __ldg(rn_gpos + A * BS + c);
   }
+  constexpr int U = 6;  // codes, then values, six at a time: two rounds of loads for most nodes
+  for (int i = i0; i < i1; i += U) {
+    int code[U];
+    Real v[U][BS];
+#pragma unroll
+    for (int x = 0; x < U; ++x) code[x] = i + x < i1 ? __ldg(inc + i + x) : -1;
+#pragma unroll
+    for (int x = 0; x < U; ++x)
+#pragma unroll
+      for (int c = 0; c < BS; ++c) v[x][c] = code[x] >= 0 ? gbuf[(long long)code[x] * BS + c] : Real(0);
+#pragma unroll
+    for (int x = 0; x < U; ++x)
+#pragma unroll
+      for (int c = 0; c < BS; ++c)
+        if (code[x] >= 0) gs[c] += v[x][c];
+  }
+#pragma unroll
+  for (int c = 0; c < BS; ++c)
+    if (gp[c] >= 0) grad[gp[c]] = (double)gs[c] - (rhs ? rhs[gp[c]] : 0.0);
 }
 
 // Gradient rows, one thread per row node.

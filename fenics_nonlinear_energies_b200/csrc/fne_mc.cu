@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "fne_gather.cuh"
@@ -335,133 +336,184 @@ __global__ void __launch_bounds__(32 * kMcWarps) k_mc_elem(McArgs A, McConstR<Re
 // reordered_element_assembler.py:335-562).  k_mc_lin stores, at the
 // linearization point u, the weighted consistent tangent w_q C_q (upper
 // triangle, 6 values) of every quadrature point; k_mc_hvp then evaluates per
-// element y_e = sum_q B_q^T (w_q C_q) (B_q x_e) -- or, for the diagonal,
-// d_(a,c) = sum_q B_q[:,(a,c)]^T (w_q C_q) B_q[:,(a,c)] -- without forming
-// K_e; the element vectors are summed per owned row by k_rowgrad.  One warp
-// per element, one lane per quadrature point, then one lane per element DOF.
+// element y_e = sum_q B_q^T (w_q C_q) (B_q x_e), k_mc_hvp_diag the diagonal
+// d_(a,c) = sum_q B_q[:,(a,c)]^T (w_q C_q) B_q[:,(a,c)], without forming
+// K_e; the element vectors are summed per owned row by k_rowgrad.
+//
+// Tangents are stored in tiles of 32 elements, the same value of the 32
+// together, so that the kernels that take one element per lane read and write
+// them in whole lines.
 // ---------------------------------------------------------------------------
+constexpr int kLinTile = 32;
+template <int NQ>
+__device__ __forceinline__ long long lin_at(int e, int q, int k) {
+  return (((long long)(e / kLinTile) * NQ + q) * 6 + k) * kLinTile + e % kLinTile;
+}
+
+// One tile per CTA, threads over (quadrature point, element).
 template <typename Real, int NP, int NQ, bool GQ>
-__global__ void __launch_bounds__(32 * kMcWarps) k_mc_lin(McArgs A, McConstR<Real> M, Real* __restrict__ wct) {
-  constexpr int N = 2 * NP;
-  __shared__ Real s_dh1[NQ * NP], s_dh2[NQ * NP], s_w[NQ];
-  __shared__ Real s_u[kMcWarps][N];
-  for (int i = threadIdx.x; i < NQ * NP; i += blockDim.x) {
-    s_dh1[i] = (Real)A.dhat1[i];
-    s_dh2[i] = (Real)A.dhat2[i];
+__global__ void __launch_bounds__(128) k_mc_lin(McArgs A, McConstR<Real> M, Real* __restrict__ wct) {
+  constexpr int TE = kLinTile, N2 = 2 * NP, NT = 128, US = N2 + 1;
+  constexpr int GS = geo_stride<NQ, GQ>();
+  __shared__ Real sD1[NQ * NP], sD2[NQ * NP], sW[NQ];
+  __shared__ Real sU[TE * US];
+  __shared__ Real sGm[TE * GS];
+  const int tid = threadIdx.x, e0 = blockIdx.x * TE, ne = min(TE, A.n_el - e0);
+  for (int i = tid; i < NQ * NP; i += NT) {
+    sD1[i] = (Real)A.dhat1[i];
+    sD2[i] = (Real)A.dhat2[i];
   }
-  for (int i = threadIdx.x; i < NQ; i += blockDim.x) s_w[i] = (Real)A.qw[i];
+  for (int i = tid; i < NQ; i += NT) sW[i] = (Real)A.qw[i];
+  for (int i = tid; i < ne * N2; i += NT) {
+    const int code = __ldg(A.codes + (long long)e0 * N2 + i);
+    sU[(i / N2) * US + i % N2] = (Real)(code >= 0 ? __ldg(A.u + code) : __ldg(A.dir + (-1 - code)));
+  }
+  for (int i = tid; i < ne * GS; i += NT) sGm[i] = (Real)__ldg(A.geom + (long long)e0 * GS + i);
   __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  Real* ue = s_u[wid];
-  for (int e = blockIdx.x * kMcWarps + wid; e < A.n_el; e += gridDim.x * kMcWarps) {
-    for (int i = lane; i < N; i += 32) {
-      const int code = A.codes[(long long)e * N + i];
-      ue[i] = (Real)(code >= 0 ? A.u[code] : A.dir[-1 - code]);
+  for (int p = tid; p < TE * NQ; p += NT) {
+    const int q = p / TE, el = p - q * TE;
+    if (el >= ne) continue;
+    const Real* gm = sGm + el * GS + (GQ ? 5 * q : 0);
+    const Real i00 = gm[0], i01 = gm[1], i10 = gm[2], i11 = gm[3];
+    const Real* ue = sU + el * US;
+    Real ex = Real(0), ey = Real(0), exy = Real(0);
+    for (int a = 0; a < NP; ++a) {
+      const Real r1 = sD1[q * NP + a], r2 = sD2[q * NP + a];
+      const Real px = i00 * r1 + i01 * r2, py = i10 * r1 + i11 * r2;
+      ex += px * ue[2 * a];
+      ey += py * ue[2 * a + 1];
+      exy += py * ue[2 * a] + px * ue[2 * a + 1];
     }
-    __syncwarp();
-    if (lane < NQ) {
-      const int q = lane;
-      const double* gm = A.geom + (long long)geo_stride<NQ, GQ>() * e + (GQ ? 5 * q : 0);
-      const Real i00 = (Real)gm[0], i01 = (Real)gm[1], i10 = (Real)gm[2], i11 = (Real)gm[3], dj = (Real)gm[4];
-      Real ex = Real(0), ey = Real(0), exy = Real(0);
-      for (int a = 0; a < NP; ++a) {
-        const Real r1 = s_dh1[q * NP + a], r2 = s_dh2[q * NP + a];
-        const Real px = i00 * r1 + i01 * r2, py = i10 * r1 + i11 * r2;
-        ex += px * ue[2 * a];
-        ey += py * ue[2 * a + 1];
-        exy += py * ue[2 * a] + px * ue[2 * a + 1];
-      }
-      Real eps[3] = {ex, ey, exy};
-      if (A.epsp) {
-        const double* ep = A.epsp + ((long long)e * NQ + q) * 3;
-        eps[0] -= (Real)ep[0];
-        eps[1] -= (Real)ep[1];
-        eps[2] -= (Real)ep[2];
-      }
-      Real sig[3], Ct[6], psi;
-      mc_point(M, eps, sig, Ct, psi);
-      const Real w = dj * s_w[q];
-      Real* o = wct + ((long long)e * NQ + q) * 6;
+    Real eps[3] = {ex, ey, exy};
+    if (A.epsp) {
+      const double* ep = A.epsp + ((long long)(e0 + el) * NQ + q) * 3;
+      eps[0] -= (Real)ep[0];
+      eps[1] -= (Real)ep[1];
+      eps[2] -= (Real)ep[2];
+    }
+    Real sig[3], Ct[6], psi;
+    mc_point(M, eps, sig, Ct, psi);
+    const Real w = gm[4] * sW[q];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) o[k] = w * Ct[k];
-    }
-    __syncwarp();
+    for (int k = 0; k < 6; ++k) wct[lin_at<NQ>(e0 + el, q, k)] = w * Ct[k];
   }
 }
 
-template <typename Real, int NP, int NQ, bool DIAG, bool GQ>
-__global__ void __launch_bounds__(32 * kMcWarps) k_mc_hvp(McArgs A, const Real* __restrict__ wct,
-                                                          Real* __restrict__ ebuf) {
+// y = H x, a tile of 32 elements per CTA, one element per lane: warps over the
+// quadrature points form the pulled-back stresses, then warps over pairs of
+// nodes contract them.  The reference gradients are the same for all lanes
+// (broadcast reads); every other shared-memory value serves 32 lanes in two
+// wavefronts and four to eight products.  (One warp per element and one lane
+// per point read four table or vector entries per four products, 50 us for
+// 50,344 P4 elements; x_e and y_e in registers took 246 of them, eight warps
+// per SM, and as long.)
+constexpr int kHvpThreads = 256;
+template <typename Real, int NP, int NQ, bool GQ>
+__global__ void __launch_bounds__(kHvpThreads) k_mc_hvp(McArgs A, const Real* __restrict__ wct,
+                                                        Real* __restrict__ ebuf) {
+  constexpr int TE = kLinTile, N = 2 * NP, NT = kHvpThreads, PS = TE + 1, PAIRS = (NP + 1) / 2;
+  using V2 = typename std::conditional<sizeof(Real) == 8, double2, float2>::type;
+  __shared__ V2 s_tab[NQ * NP + 1];
+  __shared__ Real s_x[N * PS];         // x_e, then y_e: [DOF][element]
+  __shared__ Real s_t[NQ * 4 * TE];    // [point][c, l][element]
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int e0 = blockIdx.x * TE, ne = min(TE, A.n_el - e0);
+  for (int i = tid; i < NQ * NP; i += NT) {
+    V2 t;
+    t.x = (Real)__ldg(A.dhat1 + i);
+    t.y = (Real)__ldg(A.dhat2 + i);
+    s_tab[i] = t;
+  }
+  // tangent direction: free DOFs from x, Dirichlet DOFs zero
+  for (int i = tid; i < ne * N; i += NT) {
+    const int code = __ldg(A.codes + (long long)e0 * N + i);
+    s_x[(i % N) * PS + i / N] = code >= 0 ? (Real)__ldg(A.u + code) : Real(0);
+  }
+  const int e = min(e0 + lane, A.n_el - 1);  // idle lanes follow the last element and store nothing
+  const double* gm = A.geom + (long long)geo_stride<NQ, GQ>() * e;
+  __syncthreads();
+  for (int q = wid; q < NQ; q += NT / 32) {
+    Real c[6], J[4];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) c[k] = __ldg(wct + lin_at<NQ>(e, q, k));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) J[k] = (Real)__ldg(gm + (GQ ? 5 * q : 0) + k);
+    // reference-gradient contraction z[d][l] = sum_b R_qbl x_(b,d); strain
+    // B_q x_e = J^-T-weighted z; s = (w C_q) strain; pulled back
+    // t[c][l] = sum_i J^-1_il s[v(c,i)], so that y_(a,c) = sum_q sum_l R_qal t[c][l]
+    Real z01 = Real(0), z02 = Real(0), z11 = Real(0), z12 = Real(0);
+#pragma unroll
+    for (int a = 0; a < NP; ++a) {
+      const V2 r = s_tab[q * NP + a];
+      const Real x0 = s_x[2 * a * PS + lane], x1 = s_x[(2 * a + 1) * PS + lane];
+      z01 += r.x * x0;
+      z02 += r.y * x0;
+      z11 += r.x * x1;
+      z12 += r.y * x1;
+    }
+    const Real ex = J[0] * z01 + J[1] * z02, ey = J[2] * z11 + J[3] * z12;
+    const Real exy = J[2] * z01 + J[3] * z02 + J[0] * z11 + J[1] * z12;
+    const Real s0 = c[0] * ex + c[1] * ey + c[2] * exy;
+    const Real s1 = c[1] * ex + c[3] * ey + c[4] * exy;
+    const Real s2 = c[2] * ex + c[4] * ey + c[5] * exy;
+    Real* t = s_t + q * 4 * TE + lane;
+    t[0 * TE] = J[0] * s0 + J[2] * s2;  // c = 0, l = 1
+    t[1 * TE] = J[1] * s0 + J[3] * s2;  // c = 0, l = 2
+    t[2 * TE] = J[2] * s1 + J[0] * s2;  // c = 1, l = 1
+    t[3 * TE] = J[3] * s1 + J[1] * s2;  // c = 1, l = 2
+  }
+  __syncthreads();
+  for (int g = wid; g < PAIRS; g += NT / 32) {
+    const int a = 2 * g;
+    Real y[4] = {Real(0), Real(0), Real(0), Real(0)};
+#pragma unroll 4
+    for (int q = 0; q < NQ; ++q) {
+      const Real* t = s_t + q * 4 * TE + lane;
+      const Real t0 = t[0], t1 = t[TE], t2 = t[2 * TE], t3 = t[3 * TE];
+      const V2 r = s_tab[q * NP + a], p = s_tab[q * NP + a + 1];  // (the last of an odd count is not used)
+      y[0] += r.x * t0 + r.y * t1;
+      y[1] += r.x * t2 + r.y * t3;
+      y[2] += p.x * t0 + p.y * t1;
+      y[3] += p.x * t2 + p.y * t3;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (2 * a + k < N) s_x[(2 * a + k) * PS + lane] = y[k];  // (x_e is no longer read)
+  }
+  __syncthreads();
+  for (int i = tid; i < ne * N; i += NT) ebuf[(long long)e0 * N + i] = s_x[(i % N) * PS + i / N];
+}
+
+// The diagonal: one warp per element, lanes over its DOFs.
+template <typename Real, int NP, int NQ, bool GQ>
+__global__ void __launch_bounds__(32 * kMcWarps) k_mc_hvp_diag(McArgs A, const Real* __restrict__ wct,
+                                                               Real* __restrict__ ebuf) {
   constexpr int N = 2 * NP;
   __shared__ Real s_dh1[NQ * NP], s_dh2[NQ * NP];
-  __shared__ Real s_x[kMcWarps][N];
-  __shared__ Real s_s[kMcWarps][NQ * 4];
   for (int i = threadIdx.x; i < NQ * NP; i += blockDim.x) {
     s_dh1[i] = (Real)A.dhat1[i];
     s_dh2[i] = (Real)A.dhat2[i];
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  Real* xe = s_x[wid];
-  Real* ss = s_s[wid];
   for (int e = blockIdx.x * kMcWarps + wid; e < A.n_el; e += gridDim.x * kMcWarps) {
     const double* gm = A.geom + (long long)geo_stride<NQ, GQ>() * e;
-    const Real* wc = wct + (long long)e * NQ * 6;
-    if (!DIAG) {
-      // tangent direction: free DOFs from x, Dirichlet DOFs zero
-      for (int i = lane; i < N; i += 32) {
-        const int code = A.codes[(long long)e * N + i];
-        xe[i] = code >= 0 ? (Real)A.u[code] : Real(0);
-      }
-      __syncwarp();
-      if (lane < NQ) {
-        // reference-gradient contraction z[d][l] = sum_b R_qbl x_(b,d); strain
-        // B_q x_e = J^-T-weighted z; s = (w C_q) strain; pulled back
-        // t[c][l] = sum_i J^-1_il s[v(c,i)], so that y_(a,c) = sum_q sum_l R_qal t[c][l]
-        const int q = lane;
-        const double* gq = gm + (GQ ? 5 * q : 0);
-        const Real i00 = (Real)gq[0], i01 = (Real)gq[1], i10 = (Real)gq[2], i11 = (Real)gq[3];
-        Real z01 = Real(0), z02 = Real(0), z11 = Real(0), z12 = Real(0);
-        for (int a = 0; a < NP; ++a) {
-          const Real r1 = s_dh1[q * NP + a], r2 = s_dh2[q * NP + a];
-          const Real x0 = xe[2 * a], x1 = xe[2 * a + 1];
-          z01 += r1 * x0;
-          z02 += r2 * x0;
-          z11 += r1 * x1;
-          z12 += r2 * x1;
-        }
-        const Real ex = i00 * z01 + i01 * z02, ey = i10 * z11 + i11 * z12;
-        const Real exy = i10 * z01 + i11 * z02 + i00 * z11 + i01 * z12;
-        const Real* C = wc + q * 6;
-        const Real s0 = C[0] * ex + C[1] * ey + C[2] * exy;
-        const Real s1 = C[1] * ex + C[3] * ey + C[4] * exy;
-        const Real s2 = C[2] * ex + C[4] * ey + C[5] * exy;
-        ss[q * 4 + 0] = i00 * s0 + i10 * s2;  // c = 0, l = 1
-        ss[q * 4 + 1] = i01 * s0 + i11 * s2;  // c = 0, l = 2
-        ss[q * 4 + 2] = i10 * s1 + i00 * s2;  // c = 1, l = 1
-        ss[q * 4 + 3] = i11 * s1 + i01 * s2;  // c = 1, l = 2
-      }
-      __syncwarp();
-    }
     for (int i = lane; i < N; i += 32) {
       const int a = i >> 1, c = i & 1;
       Real acc = Real(0);
       for (int q = 0; q < NQ; ++q) {
         const Real r1 = s_dh1[q * NP + a], r2 = s_dh2[q * NP + a];
-        if (DIAG) {
-          // B column (a, c): c = 0 -> (px, 0, py); c = 1 -> (0, py, px)
-          const double* gq = gm + (GQ ? 5 * q : 0);
-          const Real px = (Real)gq[0] * r1 + (Real)gq[1] * r2, py = (Real)gq[2] * r1 + (Real)gq[3] * r2;
-          const Real* C = wc + q * 6;
-          acc += c == 0 ? px * (C[0] * px + C[2] * py) + py * (C[2] * px + C[5] * py)
-                        : py * (C[3] * py + C[4] * px) + px * (C[4] * py + C[5] * px);
-        } else {
-          acc += r1 * ss[q * 4 + 2 * c] + r2 * ss[q * 4 + 2 * c + 1];
-        }
+        // B column (a, c): c = 0 -> (px, 0, py); c = 1 -> (0, py, px)
+        const double* gq = gm + (GQ ? 5 * q : 0);
+        const Real px = (Real)gq[0] * r1 + (Real)gq[1] * r2, py = (Real)gq[2] * r1 + (Real)gq[3] * r2;
+        Real C[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) C[k] = wct[lin_at<NQ>(e, q, k)];
+        acc += c == 0 ? px * (C[0] * px + C[2] * py) + py * (C[2] * px + C[5] * py)
+                      : py * (C[3] * py + C[4] * px) + px * (C[4] * py + C[5] * px);
       }
       ebuf[(long long)e * N + i] = acc;
     }
-    __syncwarp();
   }
 }
 
@@ -2025,15 +2077,16 @@ cudaError_t mc_lin_launch_g(McHandle* h, int op, const double* v, double* out, c
   A.lo = h->lo;
   Real* wct = static_cast<Real*>(h->lin_wct);
   Real* eb = static_cast<Real*>(h->lin_ebuf);
-  const int grid = h->grid_elem, T = 32 * kMcWarps;
+  const int grid = h->grid_elem, T = 32 * kMcWarps, n_tiles = (h->n_local + kLinTile - 1) / kLinTile;
   if (op == 0) {
-    k_mc_lin<Real, NP, NQ, GQ><<<grid, T, 0, st>>>(A, cast_const<Real>(h->mc), wct);
+    if (n_tiles > 0) k_mc_lin<Real, NP, NQ, GQ><<<n_tiles, 128, 0, st>>>(A, cast_const<Real>(h->mc), wct);
     return cudaGetLastError();
   }
-  if (op == 1)
-    k_mc_hvp<Real, NP, NQ, false, GQ><<<grid, T, 0, st>>>(A, wct, eb);
-  else
-    k_mc_hvp<Real, NP, NQ, true, GQ><<<grid, T, 0, st>>>(A, wct, eb);
+  if (op == 1) {
+    if (n_tiles > 0) k_mc_hvp<Real, NP, NQ, GQ><<<n_tiles, kHvpThreads, 0, st>>>(A, wct, eb);
+  } else {
+    k_mc_hvp_diag<Real, NP, NQ, GQ><<<grid, T, 0, st>>>(A, wct, eb);
+  }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (h->use_blk) {
@@ -2067,7 +2120,7 @@ int mc_lin(McHandle* h, int op, const double* v, double* out, void* stream) {
   if (op == 0 && !h->lin_wct) {
     const size_t rsz = h->precision == FNE_FP32 ? sizeof(float) : sizeof(double);
     unsigned char *w = nullptr, *eb = nullptr;
-    int rc = mc_upload(h, &w, (const unsigned char*)nullptr, std::max<size_t>(1, (size_t)h->n_local * h->nq * 6 * rsz));
+    int rc = mc_upload(h, &w, (const unsigned char*)nullptr, std::max<size_t>(1, (size_t)(h->n_local + kLinTile - 1) / kLinTile * kLinTile * h->nq * 6 * rsz));
     if (!rc) rc = mc_upload(h, &eb, (const unsigned char*)nullptr, std::max<size_t>(1, (size_t)h->n_local * h->n * rsz));
     if (rc) {
       if (w) cudaFree(w);
