@@ -1470,6 +1470,191 @@ __global__ void __launch_bounds__(NB, 2) k_push_tri(RowArgs A, SweepArgs S, cons
   if (WANT & W_E) energy_finalize(eacc, eo);
 }
 
+// ---------------------------------------------------------------------------
+// Tile kernel (P1 triangles, default): a CTA owns a compact cluster of rows and
+// evaluates every triangle that touches it once into shared memory: six
+// Hessian values, three gradient entries.  Then one thread per row adds its
+// triangles' diagonal values and gradient entries in element order, and one
+// thread per COO value adds the two triangles of its edge and stores it, rows
+// next to rows.  Every sum has a fixed order: no atomics, bit-reproducible.
+//
+// Why: the pass has to move about 260 MB on a 1024^2 grid (FP64), 40 us at the
+// copy rate, and was bound by latency and issue instead: k_sweep_tri executes
+// some 500 instructions per evaluation, needs half an SM's shared memory for
+// its window of rows (16 warps per SM) and meets a barrier three times per 256
+// elements.  A tile needs neither window nor row search: what every value sums
+// is written down per value in one 32-bit word (at most two triangles meet at
+// an edge), nodal values are fetched once per tile, geometry lies in job order,
+// and four CTAs share an SM: persistent ones where the energy is wanted, which
+// is then reduced once per CTA (93 -> 84 us), else a CTA per tile, whose loads
+// spread better (Hessian 76 -> 70 us).  A compact cluster of 256 rows
+// re-evaluates 1.13x (a segment of the sweep 1.29x).  On 2.1 M triangles,
+// against the sweep: gradient 86 -> 48 us, Hessian 112 -> 70, all three
+// 124 -> 84 (FP32: 50 -> 34, 71 -> 54, 84 -> 65).  What is left is the
+// evaluation's arithmetic between two barriers and the latency of a tile's
+// first loads.
+// ---------------------------------------------------------------------------
+constexpr int kTileT = 256;
+struct TileArgs {
+  const int4* __restrict__ tile;           // [n_tiles * 2]
+  const unsigned* __restrict__ job;
+  const void* __restrict__ geom;           // 7 planes of n_jobs: vol, dvx[3], dvy[3]
+  const int* __restrict__ uni;
+  const int2* __restrict__ row;
+  const unsigned* __restrict__ ent;
+  const uint4* __restrict__ inc;
+  const double* __restrict__ u;
+  const double* __restrict__ dir;
+  const double* __restrict__ rhs;          // may be null
+  long long lo;
+  int n_jobs, n_tiles;
+};
+template <typename Real>
+struct TileSmem {
+  Real v[kTileUni];              // nodal values
+  Real off[3][kTileJobs];        // H01, H02, H12
+  Real diag[3][kTileJobs];       // H00, H11, H22
+  Real g[3][kTileJobs];
+  Real row_diag[kTileRows];
+  int row_pos[kTileRows];
+};
+
+template <typename Real, int FAM, int WANT, typename HOut, int L>
+__global__ void __launch_bounds__(kTileT, 4) k_tiles_tri(TileArgs A, Phys P, double* __restrict__ grad,
+                                                         HOut* __restrict__ hess, EnergyOut eo) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  TileSmem<Real>& M = *reinterpret_cast<TileSmem<Real>*>(smem_raw);
+  const int tid = threadIdx.x;
+  double eacc = 0.0;
+  auto do_tile = [&](const int4 t0, const int4 t1) {
+    const int job0 = t0.x, n_job = t0.y, n_energy = t0.z, row0 = t0.w, n_row = t1.x, uni0 = t1.y, n_uni = t1.z;
+    const Real* __restrict__ geom = static_cast<const Real*>(A.geom) + job0;
+    const size_t np = (size_t)A.n_jobs;
+    // loads that depend on the tile alone
+    constexpr int JPT = kTileJobs / kTileT;  // jobs per thread
+    unsigned job[JPT];
+    TriElem<Real> t[JPT];
+#pragma unroll
+    for (int s = 0; s < JPT; ++s) {
+      const int j = tid + s * kTileT;
+      if (j < n_job) job[s] = __ldg(A.job + job0 + j);
+    }
+    for (int i = tid; i < n_uni; i += kTileT) M.v[i] = (Real)gather(A.u, A.dir, __ldg(A.uni + uni0 + i), 0);
+    int2 row = make_int2(0, 0);
+    uint4 inc[L / 8];
+    if (tid < n_row) {
+      row = __ldg(A.row + row0 + tid);
+      M.row_pos[tid] = row.y;
+#pragma unroll
+      for (int i = 0; i < L / 8; ++i) inc[i] = __ldg(A.inc + (size_t)(row0 + tid) * (L / 8) + i);
+    }
+#pragma unroll
+    for (int s = 0; s < JPT; ++s) {
+      const int j = tid + s * kTileT;
+      if (j < n_job) {
+        t[s].vol = __ldg(geom + j);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          t[s].dvx[a] = __ldg(geom + (1 + a) * np + j);
+          t[s].dvy[a] = __ldg(geom + (4 + a) * np + j);
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < JPT; ++s) {
+      const int j = tid + s * kTileT;
+      if (j >= n_job) continue;
+      const Real v[3] = {M.v[job[s] & 1023u], M.v[(job[s] >> 10) & 1023u], M.v[(job[s] >> 20) & 1023u]};
+      Real g[3], H[6];
+      if ((WANT & W_E) && j < n_energy) {
+        double ee;
+        tri_full<Real, FAM, true>(P, v, t[s], g, H, &ee);
+        eacc += ee;
+      } else {
+        tri_full<Real, FAM>(P, v, t[s], g, H);
+      }
+      if (WANT & W_H) {
+        M.diag[0][j] = H[0];
+        M.diag[1][j] = H[3];
+        M.diag[2][j] = H[5];
+        M.off[0][j] = H[1];
+        M.off[1][j] = H[2];
+        M.off[2][j] = H[4];
+      }
+      if (WANT & W_G) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) M.g[a][j] = g[a];
+      }
+    }
+    // entry words of the first rounds, on their way while the rows are summed
+    constexpr int PF = 8;
+    unsigned ew[PF];
+    if (WANT & W_H) {
+#pragma unroll
+      for (int r = 0; r < PF; ++r) {
+        const int i = tid + r * kTileT;
+        ew[r] = i < n_row * L ? __ldg(A.ent + (size_t)row0 * L + i) : ~0u;
+      }
+    }
+    __syncthreads();
+    if (tid < n_row) {
+      Real gs = Real(0), ds = Real(0);
+#pragma unroll
+      for (int i = 0; i < L / 8; ++i) {
+        const unsigned w[4] = {inc[i].x, inc[i].y, inc[i].z, inc[i].w};
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const unsigned c = (w[k >> 1] >> (16 * (k & 1))) & 0xFFFFu;
+          if (c != 0xFFFFu) {
+            const int at = (int)(c >> 11) * kTileJobs + (int)(c & 2047u);
+            if (WANT & W_G) gs += M.g[0][at];
+            if (WANT & W_H) ds += M.diag[0][at];
+          }
+        }
+      }
+      if (WANT & W_H) M.row_diag[tid] = ds;
+      if (WANT & W_G) grad[row.x] = (double)gs - (A.rhs ? A.rhs[row.x] : 0.0);
+      if ((WANT & W_E) && A.rhs) eacc -= A.rhs[row.x] * A.u[A.lo + row.x];
+    }
+    if (WANT & W_H) {
+      __syncthreads();
+      auto put = [&](int i, unsigned w) {
+        if (w == ~0u) return;
+        const int r = i / L, k = i % L;
+        const unsigned c0 = w & 0xFFFu, c1 = (w >> 12) & 0xFFFu;
+        Real v;
+        if (w & (1u << 24)) {
+          v = M.row_diag[r];
+        } else {
+          v = c0 != 0xFFFu ? M.off[0][c0] : Real(0);
+          if (c1 != 0xFFFu) v += M.off[0][c1];
+        }
+        hess[M.row_pos[r] + k] = (HOut)v;
+      };
+#pragma unroll
+      for (int r = 0; r < PF; ++r) put(tid + r * kTileT, ew[r]);
+      for (int i = tid + PF * kTileT; i < n_row * L; i += kTileT) put(i, __ldg(A.ent + (size_t)row0 * L + i));
+    }
+  };
+  const int4* tile = A.tile + 2 * blockIdx.x;
+  int4 t0 = __ldg(tile), t1 = __ldg(tile + 1);
+  if constexpr ((WANT & W_E) == 0) {
+    do_tile(t0, t1);
+  } else {  // few CTAs, one energy reduction each
+    for (int k = blockIdx.x; k < A.n_tiles; k += gridDim.x) {
+      const int4 c0 = t0, c1 = t1;
+      if (k + (int)gridDim.x < A.n_tiles) {  // the next tile's header
+        t0 = __ldg(A.tile + 2 * (k + gridDim.x));
+        t1 = __ldg(A.tile + 2 * (k + gridDim.x) + 1);
+      }
+      do_tile(c0, c1);
+      __syncthreads();  // the next tile overwrites what this one read
+    }
+    energy_finalize(eacc, eo);
+  }
+}
+
 #include "fne_cluster.cuh"
 
 // ---------------------------------------------------------------------------
@@ -1669,6 +1854,14 @@ struct fne_handle {
   int sw_gpos_identity = 0;
   unsigned *sw_ent_meta = nullptr, *sw_inc_word = nullptr;
   int inc_max_rank = 0, inc_max_rows = 0, inc_max_len = 0;
+  // tile kernel (P1 triangles)
+  int n_tri_tiles = 0, tile_lanes = 0, tile_jobs = 0;
+  int4* tt_tile = nullptr;
+  unsigned *tt_job = nullptr, *tt_ent = nullptr;
+  void* tt_geom = nullptr;
+  int* tt_uni = nullptr;
+  int2* tt_row = nullptr;
+  uint4* tt_inc = nullptr;
   // element-parallel tet pass: per-element blocks + contribution lists
   bool use_elem2 = false;
   int grid_elem2 = 1;
@@ -1741,7 +1934,8 @@ void free_handle(fne_handle* h) {
                   h->h_hess, h->e2_kbuf, h->e2_gbuf, h->bp_rn_blk, h->bp_rn_con, h->bp_rn_row,
                   h->bp_rn_gpos, h->bp_rn_inc, h->bp_con, h->bp_inc, h->bp_blk, h->cl_table,
                   h->cl_codes, h->cl_reals, h->cl_rows, h->cl_runs, h->cl_incs, h->err,
-                  h->nt_tile, h->nt_inc, h->nt_uni, h->nt_blob};
+                  h->nt_tile, h->nt_inc, h->nt_uni, h->nt_blob,
+                  h->tt_tile, h->tt_job, h->tt_ent, h->tt_geom, h->tt_uni, h->tt_row, h->tt_inc};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (h->err_host) cudaFreeHost(h->err_host);
@@ -1894,6 +2088,65 @@ cudaError_t launch_tri_t(fne_handle* h, int want, const RowArgs& A, const IncArg
   }
 #undef FNE_TRI_CASE
   return cudaErrorInvalidValue;
+}
+
+template <typename Real, int FAM, typename HOut, int L>
+cudaError_t launch_tiles_t(fne_handle* h, int want, const double* u, double* grad, void* hess, EnergyOut eo,
+                           cudaStream_t st, bool set_attr) {
+  const TileArgs A{h->tt_tile, h->tt_job, h->tt_geom, h->tt_uni, h->tt_row, h->tt_ent,
+                   h->tt_inc,  u,         h->dir,     h->rhs,    h->lo,     h->tile_jobs, h->n_tri_tiles};
+  const int grid = (want & W_E) ? std::min(h->n_tri_tiles, 4 * h->num_sms) : h->n_tri_tiles;
+  HOut* H = static_cast<HOut*>(hess);
+  constexpr size_t sm = sizeof(TileSmem<Real>);
+#define FNE_TILE_CASE(W)                                                                                        \
+  case W:                                                                                                       \
+    if (set_attr)                                                                                               \
+      return cudaFuncSetAttribute(k_tiles_tri<Real, FAM, W, HOut, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                  (int)sm);                                                                     \
+    k_tiles_tri<Real, FAM, W, HOut, L><<<grid, kTileT, sm, st>>>(A, h->phys, grad, H, eo);            \
+    return cudaGetLastError();
+  switch (want) {
+    FNE_TILE_CASE(2)
+    FNE_TILE_CASE(3)
+    FNE_TILE_CASE(4)
+    FNE_TILE_CASE(5)
+    FNE_TILE_CASE(6)
+    FNE_TILE_CASE(7)
+  }
+#undef FNE_TILE_CASE
+  return cudaErrorInvalidValue;
+}
+
+template <int FAM, int L>
+cudaError_t launch_tiles_f(fne_handle* h, int want, const double* u, double* grad, void* hess, EnergyOut eo,
+                           cudaStream_t st, bool set_attr) {
+  if (h->precision == FNE_FP64) return launch_tiles_t<double, FAM, double, L>(h, want, u, grad, hess, eo, st, set_attr);
+  if (h->hess_fp32) return launch_tiles_t<float, FAM, float, L>(h, want, u, grad, hess, eo, st, set_attr);
+  return launch_tiles_t<float, FAM, double, L>(h, want, u, grad, hess, eo, st, set_attr);
+}
+
+cudaError_t launch_tiles(fne_handle* h, int want, const double* u, double* grad, void* hess, EnergyOut eo,
+                         cudaStream_t st, bool set_attr = false) {
+  if (h->family == FNE_PLAPLACE)
+    return h->tile_lanes == 8 ? launch_tiles_f<FAM_PLAP, 8>(h, want, u, grad, hess, eo, st, set_attr)
+                              : launch_tiles_f<FAM_PLAP, 16>(h, want, u, grad, hess, eo, st, set_attr);
+  return h->tile_lanes == 8 ? launch_tiles_f<FAM_GL, 8>(h, want, u, grad, hess, eo, st, set_attr)
+                            : launch_tiles_f<FAM_GL, 16>(h, want, u, grad, hess, eo, st, set_attr);
+}
+
+// geometry of the tiles' jobs: planes vol, dvx[3], dvy[3]
+template <typename Real>
+void pack_tile_jobs(const fne_desc* d, const RowPlan& P, const TilePlan& T, std::vector<Real>& out) {
+  const size_t n = T.job_elem.size();
+  out.resize(7 * n);
+  for (size_t j = 0; j < n; ++j) {
+    const int64_t e = P.local_elems[T.job_elem[j]];
+    out[j] = (Real)d->e2[e];
+    for (int a = 0; a < 3; ++a) {
+      out[(1 + a) * n + j] = (Real)d->e0[e * 3 + a];
+      out[(4 + a) * n + j] = (Real)d->e1[e * 3 + a];
+    }
+  }
 }
 
 template <typename Real, typename HOut, int G>
@@ -2384,7 +2637,20 @@ extern "C" int fne_create(const fne_desc* d, fne_handle** out) {
       use_cluster = build_cluster_plan(plan, d->lo, d->hi, lay.cr, lay.cj, lay.ci, lay.cw, gid, cplan);
     if (use_cluster && cplan.max_runs > lay.cu) use_cluster = false;
   }
-  if (is_tri(d->family) && plan.n_rows > 0 &&
+  // tiles of rows (triangles by default; 128 -> 84 us for the fused pass over
+  // 2.1 M triangles against the banded sweep, which stays for rows of more than
+  // 16 elements or 14 entries: the row clusters have four bits for a place): small meshes get smaller tiles, two per SM
+  TilePlan tplan;
+  bool use_tiles = false;
+  if (is_tri(d->family) && plan.n_rows > 0 && d->kernel_variant == 0) {
+    bool identity = true;
+    for (int32_t k = 0; k < plan.n_rows && identity; ++k) identity = plan.row_gpos[k] == k;
+    const int64_t jobs = (int64_t)plan.local_elems.size() * 5 / 4 / (2 * (int64_t)n_sms);
+    sort_elements_by_row(plan);
+    use_tiles = build_tile_plan(plan, d->lo, d->hi, (int)std::min<int64_t>(kTileJobs, std::max<int64_t>(64, jobs)),
+                                identity, tplan);
+  }
+  if (is_tri(d->family) && plan.n_rows > 0 && !use_tiles &&
       (d->kernel_variant == 0 || (d->kernel_variant == 8 && !use_cluster) || d->kernel_variant == 7 || want_push)) {
     // shared memory per CTA: 12*nb element quantities (pull sweep only) +
     // entry window + row window, sized so that two CTAs fit on one SM
@@ -2618,6 +2884,37 @@ extern "C" int fne_create(const fne_desc* d, fne_handle** out) {
       h->e2_gbuf = gb;
     }
   }
+  if (use_tiles) {
+    h->n_tri_tiles = (int)(tplan.tile.size() / 8);
+    h->tile_lanes = tplan.lanes;
+    h->tile_jobs = (int)tplan.job.size();
+    if (f32) {
+      std::vector<float> geom;
+      pack_tile_jobs(d, plan, tplan, geom);
+      float* p = nullptr;
+      FNE_TRY(upload(h, &p, geom.data(), geom.size()));
+      h->tt_geom = p;
+    } else {
+      std::vector<double> geom;
+      pack_tile_jobs(d, plan, tplan, geom);
+      double* p = nullptr;
+      FNE_TRY(upload(h, &p, geom.data(), geom.size()));
+      h->tt_geom = p;
+    }
+    FNE_TRY(upload(h, &h->tt_tile, reinterpret_cast<const int4*>(tplan.tile.data()), tplan.tile.size() / 4));
+    FNE_TRY(upload(h, &h->tt_job, tplan.job.data(), tplan.job.size()));
+    FNE_TRY(upload(h, &h->tt_uni, tplan.uni.data(), tplan.uni.size()));
+    FNE_TRY(upload(h, &h->tt_row, reinterpret_cast<const int2*>(tplan.row.data()), tplan.row.size() / 2));
+    FNE_TRY(upload(h, &h->tt_ent, tplan.ent.data(), tplan.ent.size()));
+    FNE_TRY(upload(h, &h->tt_inc, reinterpret_cast<const uint4*>(tplan.inc.data()), tplan.inc.size() / 8));
+    for (int want = 2; want <= 7; ++want) {
+      cudaError_t e = launch_tiles(h, want, nullptr, nullptr, nullptr, EnergyOut{}, 0, true);
+      if (e != cudaSuccess) {
+        free_handle(h);
+        return cuda_fail(e, "cudaFuncSetAttribute");
+      }
+    }
+  }
   if (use_nodes) {
     h->n_node_tiles = (int)nplan.tile.size();
     h->n_inc = (int64_t)nbp.inc.size();
@@ -2682,7 +2979,7 @@ extern "C" int fne_info_get(const fne_handle* h, fne_info* info) {
   info->n_incidences = h->n_inc;
   info->device_bytes = h->device_bytes;
   info->max_row_len = h->max_row_len;
-  info->kernel_variant = is_tri(h->family) ? (h->use_cluster ? 10 : h->use_push ? 8 : (h->use_sweep ? 4 : (h->use_inc ? 3 : 1)))
+  info->kernel_variant = is_tri(h->family) ? (h->n_tri_tiles ? 12 : h->use_cluster ? 10 : h->use_push ? 8 : (h->use_sweep ? 4 : (h->use_inc ? 3 : 1)))
                                            : (h->use_elem2 ? 7 : 2);
   if (h->use_elem2) info->n_incidences = h->e2_contrib;
   info->row_lanes = h->tet_lanes;
@@ -2786,7 +3083,8 @@ extern "C" int fne_eval(fne_handle* h, const double* u, int flags, double* energ
                  h->sw_ent_ptr,  h->sw_inc_base,  h->sw_ent_row,    h->sw_ent_pos,
                  h->sw_ent_meta, h->sw_inc_word,  h->sweep_win_mask, h->sweep_rwin_mask,
                  h->sw_gpos_identity, h->sw_eoff, h->sw_row_of};
-    e = h->n_node_tiles ? launch_nodes(h, flags, u, grad, hess, eo, st)
+    e = h->n_tri_tiles ? launch_tiles(h, flags, u, grad, hess, eo, st)
+        : h->n_node_tiles ? launch_nodes(h, flags, u, grad, hess, eo, st)
         : h->use_elem2 ? launch_elem2(h, flags, u, grad, hess, eo, st)
                      : launch_rows(h, flags, A, Q, SW, grad, hess, eo, st, false);
     // stream-ordered copy of the status word for fne_poll_device_status

@@ -164,6 +164,7 @@ struct ClusterPlan {
   std::vector<int32_t> rows;         // [n_rows_total * 4]
   std::vector<int32_t> runs;         // [n_runs * 4]
   std::vector<uint32_t> incs;        // [n_incs_total]
+  std::vector<int32_t> row_k;        // [n_rows_total] index of the row in the row plan
 };
 constexpr int kClJobBits = 11;
 constexpr uint32_t kClNoCol = 15u;
@@ -174,6 +175,39 @@ constexpr uint32_t kClNoCol = 15u;
 // format (a row longer than 14 entries, a row alone beyond a budget).
 bool build_cluster_plan(const RowPlan& P, int64_t lo, int64_t hi, int max_rows, int max_jobs, int max_incs,
                         int max_win, bool gpos_identity, ClusterPlan& Q);
+
+// Tile plan (scalar P1 triangles): the clusters of a ClusterPlan (at most
+// kTileJobs jobs, kTileRows rows and kTileUni referred nodes) in the form
+// k_tiles_tri reads.
+//   tile: {first job, jobs, energy-counting jobs (they come first), first
+//     row, rows, first referred node, referred nodes, 0};
+//   job: places of its three nodes among the tile's referred nodes, 10 bits
+//     each;
+//   row: {gradient slot, first COO position}; per row `lanes` entry words, one
+//     per COO value: two codes of 12 bits, each the place (pair * kTileJobs +
+//     job, pair 0 = nodes 01, 1 = 02, 2 = 12) of one contribution or 0xFFF;
+//     bit 24: the diagonal; ~0: beyond the row; and `lanes` 16-bit incidence
+//     codes (job | node << 11, 0xFFFF: none) in element order.
+constexpr int kTileJobs = 512;
+constexpr int kTileRows = 256;
+constexpr int kTileUni = 512;
+struct TilePlan {
+  int lanes = 0;                     // 8 or 16 entries and incidences per row
+  std::vector<int32_t> tile;         // [n_tiles * 8]
+  std::vector<int32_t> job_elem;     // [n_jobs] local element
+  std::vector<uint32_t> job;         // [n_jobs]
+  std::vector<int32_t> uni;          // gather codes
+  std::vector<int32_t> row;          // [n_rows * 2]
+  std::vector<uint32_t> ent;         // [n_rows * lanes]
+  std::vector<uint16_t> inc;         // [n_rows * lanes]
+};
+// False when the mesh does not fit (rows or valences beyond 16, an
+// off-diagonal entry with more than two elements, a row without its diagonal).
+bool build_tile_plan(const RowPlan& P, int64_t lo, int64_t hi, int max_jobs, bool gpos_identity, TilePlan& T);
+
+// Sorts P's local elements by the first row that needs them (locality of the
+// element records; sums do not depend on it).
+void sort_elements_by_row(RowPlan& P);
 
 // Node-block gather plan: the element matrices (stored per element as node
 // pairs a <= b of bs x bs blocks) are summed per output block (row node A,

@@ -11,7 +11,6 @@
 // no atomics are needed and the result is bit-reproducible.  As in the
 // reference, a missing (row, col) key is an error (FNE_ELAYOUT).
 #include <algorithm>
-#include <unordered_map>
 
 #include "fne_internal.h"
 
@@ -122,24 +121,13 @@ int build_row_plan(const fne_desc* d, RowPlan& P, bool incidences) {
 
   // row-nodes in order of first appearance; the first row of each node is the
   // one whose column layout defines the offsets (all rows must agree)
-  std::unordered_map<int64_t, int32_t> node_idx;
-  std::vector<int32_t> node_first_row;
-  std::vector<int64_t> node_of;
-  int32_t max_len = 0;
+  std::vector<int32_t> node_idx(d->n_total / bs + 1, -1);
+  int32_t max_len = 0, n_nodes = 0;
   for (int32_t k = 0; k < n_rows; ++k) {
     const int64_t t = rev[row_id[k] - lo];
     const int64_t node = t / bs;
-    auto it = node_idx.find(node);
-    int32_t ni;
-    if (it == node_idx.end()) {
-      ni = (int32_t)node_of.size();
-      node_idx.emplace(node, ni);
-      node_of.push_back(node);
-      node_first_row.push_back(k);
-    } else {
-      ni = it->second;
-    }
-    P.row_node[k] = ni;
+    if (node_idx[node] < 0) node_idx[node] = n_nodes++;
+    P.row_node[k] = node_idx[node];
     P.row_comp[k] = (uint8_t)(t % bs);
     P.row_gpos[k] = (int32_t)(row_id[k] - lo);
     max_len = std::max<int32_t>(max_len, P.row_ptr[k + 1] - P.row_ptr[k]);
@@ -147,7 +135,6 @@ int build_row_plan(const fne_desc* d, RowPlan& P, bool incidences) {
   P.max_row_len = max_len;
   if (max_len >= (int32_t)kNoCol)
     return set_error(FNE_EBOUNDS, "row plan: a row has more than 126 entries");
-  const int32_t n_nodes = (int32_t)node_of.size();
   P.n_nodes = n_nodes;
 
   P.inc_ptr.clear();
@@ -156,8 +143,13 @@ int build_row_plan(const fne_desc* d, RowPlan& P, bool incidences) {
   if (!incidences) return FNE_OK;
 
   // rows of each node (to validate identical column layouts)
-  std::vector<std::vector<int32_t>> node_rows(n_nodes);
-  for (int32_t k = 0; k < n_rows; ++k) node_rows[P.row_node[k]].push_back(k);
+  std::vector<int32_t> node_ptr(n_nodes + 1, 0), node_rows(n_rows);
+  for (int32_t k = 0; k < n_rows; ++k) ++node_ptr[P.row_node[k] + 1];
+  for (int32_t i = 0; i < n_nodes; ++i) node_ptr[i + 1] += node_ptr[i];
+  {
+    std::vector<int32_t> at(node_ptr.begin(), node_ptr.end() - 1);
+    for (int32_t k = 0; k < n_rows; ++k) node_rows[at[P.row_node[k]]++] = k;
+  }
 
   // ---- incidences ----------------------------------------------------------
   std::vector<int32_t> cnt(n_nodes + 1, 0);
@@ -175,9 +167,8 @@ int build_row_plan(const fne_desc* d, RowPlan& P, bool incidences) {
       const int32_t ca = code[e * npe + a];
       if (ca < lo || ca >= hi) continue;  // not an owned row-node
       const int64_t node = rev[ca - lo] / bs;
-      auto it = node_idx.find(node);
-      if (it == node_idx.end()) return set_error(FNE_ELAYOUT, "row plan: owned node has no row");
-      const int32_t ni = it->second;
+      const int32_t ni = node_idx[node];
+      if (ni < 0) return set_error(FNE_ELAYOUT, "row plan: owned node has no row");
       uint32_t info = (uint32_t)a;
       if (!flagged && P.elem_weight[le]) {
         info |= kEnergyFlag;
@@ -189,7 +180,8 @@ int build_row_plan(const fne_desc* d, RowPlan& P, bool incidences) {
         uint32_t off = kNoCol;
         if (cb >= 0) {
           bool first = true;
-          for (int32_t k : node_rows[ni]) {
+          for (int32_t i = node_ptr[ni]; i < node_ptr[ni + 1]; ++i) {
+            const int32_t k = node_rows[i];
             const int64_t s = P.row_ptr[k], len = P.row_ptr[k + 1] - s;
             int64_t pos = -1;
             for (int64_t q = 0; q < len; ++q)
@@ -463,6 +455,125 @@ bool build_sweep_plan(RowPlan& P, int nb, int n_seg, int max_win_entries, int ma
   Q.win_entries = next_pow2(need_entries);
   Q.win_rows = next_pow2(need_rows);
   return Q.win_entries <= max_win_entries && Q.win_rows <= max_win_rows;
+}
+
+}  // namespace fne
+
+namespace fne {
+
+void sort_elements_by_row(RowPlan& P) {
+  const int32_t n_local = (int32_t)P.local_elems.size();
+  const int npe = n_local ? (int)(P.elem_code.size() / n_local) : 3;
+  std::vector<int32_t> first(n_local, P.n_rows), at(P.n_rows + 2, 0), newidx(n_local);
+  for (int32_t k = 0; k < P.n_rows; ++k) {
+    const int32_t nd = P.row_node[k];
+    for (int32_t i = P.inc_ptr[nd]; i < P.inc_ptr[nd + 1]; ++i)
+      first[P.inc_elem[i]] = std::min(first[P.inc_elem[i]], k);
+  }
+  for (int32_t i = 0; i < n_local; ++i) ++at[first[i] + 1];
+  for (int32_t k = 0; k <= P.n_rows; ++k) at[k + 1] += at[k];
+  for (int32_t i = 0; i < n_local; ++i) newidx[i] = at[first[i]]++;
+  std::vector<int64_t> le(n_local);
+  std::vector<int32_t> code(P.elem_code.size());
+  std::vector<uint8_t> w(n_local);
+  for (int32_t i = 0; i < n_local; ++i) {
+    const int32_t to = newidx[i];
+    le[to] = P.local_elems[i];
+    w[to] = P.elem_weight[i];
+    for (int a = 0; a < npe; ++a) code[(size_t)to * npe + a] = P.elem_code[(size_t)i * npe + a];
+  }
+  P.local_elems.swap(le);
+  P.elem_code.swap(code);
+  P.elem_weight.swap(w);
+  for (auto& e : P.inc_elem) e = newidx[e];
+}
+
+bool build_tile_plan(const RowPlan& P, int64_t lo, int64_t hi, int max_jobs, bool gpos_identity, TilePlan& T) {
+  int32_t valence = 0;
+  for (int32_t k = 0; k < P.n_rows; ++k)
+    valence = std::max(valence, P.inc_ptr[P.row_node[k] + 1] - P.inc_ptr[P.row_node[k]]);
+  if (valence > 16) return false;
+  ClusterPlan Q;
+  if (!build_cluster_plan(P, lo, hi, kTileRows, std::min(max_jobs, kTileJobs), 1 << 14, 1 << 14, gpos_identity, Q))
+    return false;
+  T = TilePlan{};
+  const int L = T.lanes = valence <= 8 && P.max_row_len <= 8 ? 8 : 16;
+  T.row.reserve(Q.row_k.size() * 2);
+  T.ent.assign(Q.row_k.size() * L, ~0u);
+  T.inc.assign(Q.row_k.size() * L, 0xFFFF);
+  // place of a node among its tile's (codes of fixed nodes are negative)
+  const auto mm = std::minmax_element(P.elem_code.begin(), P.elem_code.end());
+  const int64_t code0 = P.elem_code.empty() ? 0 : *mm.first;
+  struct Place {
+    int32_t tile, at;
+  };
+  std::vector<Place> place(P.elem_code.empty() ? 0 : *mm.second - code0 + 1, Place{-1, 0});
+  std::vector<int32_t> uni;
+  static const int kPair[3][3] = {{-1, 0, 1}, {0, -1, 2}, {1, 2, -1}};
+  for (int32_t c = 0; c < Q.n_cl; ++c) {
+    const int32_t* t = &Q.table[8 * (size_t)c];
+    const int32_t j0 = t[0], je = t[1], r0 = t[3], r1 = t[4], i0 = t[5];
+    int32_t j1 = t[2];
+    while (j1 > j0 && Q.job_elem[j1 - 1] < 0) --j1;  // (padding jobs)
+    if (j1 - j0 > kTileJobs || r1 - r0 > kTileRows) return false;
+    uni.clear();
+    for (int32_t j = j0; j < j1; ++j)
+      for (int a = 0; a < 3; ++a) {
+        const int32_t code = P.elem_code[(size_t)Q.job_elem[j] * 3 + a];
+        if (place[code - code0].tile != c) {
+          place[code - code0].tile = c;
+          uni.push_back(code);
+        }
+      }
+    std::sort(uni.begin(), uni.end());
+    for (size_t i = 0; i < uni.size(); ++i) place[uni[i] - code0].at = (int32_t)i;
+    if ((int)uni.size() > kTileUni) return false;
+    T.tile.insert(T.tile.end(), {(int32_t)T.job.size(), j1 - j0, std::min(je, j1) - j0, r0, r1 - r0,
+                                 (int32_t)T.uni.size(), (int32_t)uni.size(), 0});
+    T.uni.insert(T.uni.end(), uni.begin(), uni.end());
+    for (int32_t j = j0; j < j1; ++j) {
+      uint32_t w = 0;
+      for (int a = 0; a < 3; ++a)
+        w |= (uint32_t)place[P.elem_code[(size_t)Q.job_elem[j] * 3 + a] - code0].at << (10 * a);
+      T.job.push_back(w);
+      T.job_elem.push_back(Q.job_elem[j]);
+    }
+    for (int32_t r = r0; r < r1; ++r) {
+      const int32_t* row = &Q.rows[4 * (size_t)r];
+      const int len = row[2] & 0xFFFF, n_inc = row[2] >> 16;
+      T.row.push_back(row[0]);
+      T.row.push_back(P.row_ptr[Q.row_k[r]]);
+      uint32_t* ent = &T.ent[(size_t)r * L];
+      for (int k = 0; k < len; ++k) ent[k] = 0xFFFFFFu;  // no contribution
+      bool diag = n_inc == 0;
+      for (int i = 0; i < n_inc; ++i) {
+        const uint32_t w = Q.incs[(size_t)i0 + row[3] + i];
+        const uint32_t j = w & ((1u << kClJobBits) - 1u), a = (w >> kClJobBits) & 3u;
+        T.inc[(size_t)r * L + i] = (uint16_t)(j | a << 11);
+        for (uint32_t b = 0; b < 3; ++b) {
+          const uint32_t off = (w >> (kClJobBits + 2 + 4 * b)) & 15u;
+          if (off == kClNoCol) {
+            if (b == a) return false;
+            continue;
+          }
+          if (b == a) {
+            ent[off] |= 1u << 24;
+            diag = true;
+            continue;
+          }
+          const uint32_t code = (uint32_t)kPair[a][b] * kTileJobs + j;
+          if ((ent[off] & 0xFFFu) == 0xFFFu)
+            ent[off] = (ent[off] & ~0xFFFu) | code;
+          else if (((ent[off] >> 12) & 0xFFFu) == 0xFFFu)
+            ent[off] = (ent[off] & ~0xFFF000u) | code << 12;
+          else
+            return false;
+        }
+      }
+      if (!diag) return false;
+    }
+  }
+  return true;
 }
 
 }  // namespace fne
@@ -867,6 +978,7 @@ bool build_cluster_plan(const RowPlan& P, int64_t lo, int64_t hi, int max_rows, 
     for (int32_t k : rows) {
       const int32_t n_inc = inc_end(k) - inc_begin(k), len = row_len(k);
       if (n_inc > 0x7fff) return false;
+      Q.row_k.push_back(k);
       Q.rows.insert(Q.rows.end(), {gpos_identity ? k : P.row_gpos[k], wo, len | (n_inc << 16),
                                    (int32_t)Q.incs.size() - i0});
       // runs of rows whose COO ranges are adjacent

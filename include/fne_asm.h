@@ -177,8 +177,10 @@ typedef struct {
                                  * free DOF (Ginzburg-Landau assembler,
                                  * src/problems/ginzburg_landau/jax_petsc/
                                  * reordered_element_assembler.py:34-52, 96-97) */
-  int32_t kernel_variant;       /* P1 triangles: 0 = automatic (banded
-                                 * sweep); 1 = row-gather; 2 = incidence-
+  int32_t kernel_variant;       /* P1 triangles: 0 = automatic (tiles of
+                                 * rows; the banded sweep where a row has more
+                                 * than 16 elements or 14 entries or a tile
+                                 * does not fit); 1 = row-gather; 2 = incidence-
                                  * parallel; 3 = banded sweep with shared-
                                  * memory atomics (push; not bit-reproducible);
                                  * 7 = banded sweep; 8 = persistent row-cluster
@@ -214,7 +216,8 @@ typedef struct {
                            * 9 Mohr-Coulomb FP64 DMMA (mma.sync f64),
                            * 10 row clusters (P1 triangles),
                            * 11 3-D Mohr-Coulomb point-tile element kernel +
-                           * node-block gather */
+                           * node-block gather, 12 tiles of rows (P1
+                           * triangles) */
   int32_t row_lanes;      /* lanes per output row of the tet row kernel (for
                            * kernel_variant 0 the count it would run with where
                            * the tiles of row nodes do not apply), else 1 */

@@ -404,3 +404,60 @@ def test_he_node_tiles_match_row_gather(size, shuffle, precision):
     for flags, k in ((2, 1), (4, 2), (3, 1), (5, 2), (6, 2)):
         assert torch.equal(a.eval(u, flags)[k], (ea, ga, ha)[k])
     assert all(torch.equal(x, y) for x, y in zip(a.eval(u, 7), (ea, ga, ha)))
+
+
+def _tri_test_mesh(mesh, rng):
+    """A square of n x n cells, or a node with ``k`` triangles around it in a
+    ring of 2k more, shuffled (nodes stay, elements in any order) on request."""
+    kind, n, shuffle = mesh
+    if kind == "square":
+        nodes, elems, bnd = meshes.square_p1(n, 0.0, 1.0, "x_fast" if shuffle else "x_slow")
+    else:
+        ang = 2.0 * np.pi * np.arange(n) / n
+        ring = np.column_stack((np.cos(ang), np.sin(ang)))
+        nodes = np.vstack((np.zeros((1, 2)), ring, 2.0 * ring))
+        i, j = 1 + np.arange(n), 1 + (np.arange(n) + 1) % n
+        elems = np.vstack((np.column_stack((np.zeros_like(i), i, j)), np.column_stack((i, i + n, j)),
+                           np.column_stack((j, i + n, j + n)))).astype(np.int64)
+        bnd = np.arange(nodes.shape[0]) > n
+    if shuffle:
+        elems = elems[rng.permutation(elems.shape[0])]
+    return nodes, elems, bnd
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("family", ["plaplace", "gl"])
+@pytest.mark.parametrize("mesh", [("square", 2, False), ("square", 3, True), ("square", 33, True), ("square", 64, False),
+                                  ("square", 200, False), ("square", 200, True), ("fan", 7, False), ("fan", 8, True),
+                                  ("fan", 13, True), ("fan", 14, False)])
+def test_tri_tiles_match_row_gather(mesh, family, precision):
+    """The default P1-triangle kernel (tiles of rows) against the row-gather
+    kernel: one row, tiles that are not full, elements and nodes in any order,
+    rows of up to 14 entries; a row of 15 goes to the banded sweep.  FP64 1e-12,
+    FP32 2e-5, bit-repeatable, separate outputs equal to the fused ones."""
+    rng = np.random.default_rng(mesh[1])
+    nodes, elems, bnd = _tri_test_mesh(mesh, rng)
+    dvx, dvy, vol = meshes.p1_triangle_operators(nodes, elems)
+    free = np.flatnonzero(~bnd).astype(np.int64)
+    params = {"nodes": nodes, "u_0": 0.1 * rng.standard_normal(nodes.shape[0]), "freedofs": free, "elems": elems,
+              "dvx": dvx, "dvy": dvy, "vol": vol}
+    if family == "gl":
+        params.update(ip=meshes.GL_IP.copy(), w=meshes.GL_W.copy(), eps=0.01)
+    else:
+        params.update(f=rng.standard_normal(nodes.shape[0]) * vol.mean(), p=3.0)
+    kw = {"precision": precision, "hess_dtype": torch.float32 if precision == "fp32" else torch.float64}
+    if mesh[2]:
+        kw["perm_override"] = rng.permutation(free.size)
+    cls = _asm_classes()[family]
+    a, b = cls(params, **kw), cls(params, kernel_variant="row_gather", **kw)
+    assert a.info["kernel_variant"] == (4 if mesh[:2] == ("fan", 14) else 12)
+    u = torch.as_tensor(rng.uniform(-0.5, 0.5, free.size), device="cuda")
+    ea, ga, ha = [t.clone() for t in a.eval(u, 7)]
+    eb, gb, hb = [t.clone() for t in b.eval(u, 7)]
+    tol = FP64_TOL if precision == "fp64" else FP32_TOL
+    assert abs(float(ea.item()) - float(eb.item())) <= tol * max(1.0, abs(float(eb.item())))
+    assert _rel(ha.double().cpu().numpy(), hb.double().cpu().numpy()) <= tol
+    assert _rel(ga.cpu().numpy(), gb.cpu().numpy()) <= tol
+    for flags, k in ((2, 1), (4, 2), (3, 1), (5, 2), (6, 2)):
+        assert torch.equal(a.eval(u, flags)[k], (ea, ga, ha)[k])
+    assert all(torch.equal(x, y) for x, y in zip(a.eval(u, 7), (ea, ga, ha)))
