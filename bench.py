@@ -523,7 +523,7 @@ REFERENCE_ARCHIVED = {
 KERNEL_NAMES = {1: "k_rows_tri", 2: "k_rows_tet", 3: "k_inc_tri", 4: "k_sweep_tri",
                 5: "k_mc_elem+k_node_gather+k_rowgrad", 6: "k_mc_tc+k_fixup2+k_rowgrad", 7: "k_he_elem+k_node_gather",
                 8: "k_push_tri", 9: "k_mc_dmma+k_fixup2+k_rowgrad", 10: "k_cluster_tri",
-                11: "k_mc3d_elem+k_mc3d_gather", 12: "k_tiles_tri"}
+                11: "k_mc3d_elem+k_node_gather", 12: "k_tiles_tri"}
 
 
 def algorithmic_bytes(w, asm, n_el, energy_only=False):
