@@ -953,11 +953,7 @@ __global__ void __launch_bounds__(McTile<NP, NQ, GQ>::THREADS, McTile<NP, NQ, GQ
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           const int rs = sRow[(el * NP + ra) * 2 + c];
-          if (rs < 0) continue;
-          int k = 0;
-#pragma unroll
-          for (int d = 0; d < 2; ++d)
-            if ((dm >> d) & 1u) hout[rs + off + k++] = (HOut)w[c][d];
+          if (rs >= 0) store_pair(hout + rs + off, dm, w[c][0], w[c][1]);
         }
       };
       if (!*sFail && quad * 32 < NPAIR) {
@@ -1121,6 +1117,12 @@ __global__ void __launch_bounds__(kEgThreads) k_mc_eg(McArgs A, McConstR<Real> M
 // 8 elements) runs NQ MMA steps of four n8 tiles (one per (c, d) component)
 // and writes its blocks; the element gradient follows on the CUDA cores.
 // Two CTAs per SM, so one CTA's return map overlaps the other's MMAs.
+// 50,344 P4 elements, all outputs with the fix-up and the gradient rows
+// (floor 50 us for the bytes, 100 for the MMAs): paired stores 404 -> 385 us,
+// the next tile's nodal values fetched before the gradient instead of at the
+// tile's end 412 -> 404, the buffer positions of the tile's shared slots
+// copied to shared memory during the return map 385 -> 379.  What is left is
+// latency: 16 warps per SM, which meet three barriers per tile.
 // ---------------------------------------------------------------------------
 template <int NP, int NQ, bool GQ = false>
 struct McTileD {
@@ -1144,8 +1146,9 @@ struct McTileD {
   static constexpr int OFF_PLAN = OFF_G + R16(TE * GS * 8);          // [TE][NP * NP] uint16 codes
   static constexpr int PLAN_WORDS = (TE * NP * NP + 1) / 2;
   static constexpr int OFF_ROW = OFF_PLAN + R16(PLAN_WORDS * 4);     // [TE][NP][2] row starts
-  static constexpr int OFF_SB = OFF_ROW + R16(TE * NP * 2 * 4);      // [TE] shared-slot bases
-  static constexpr int SMEM = OFF_SB + R16(TE * 4);
+  static constexpr int OFF_SB = OFF_ROW + R16(TE * NP * 2 * 4);      // [TE + 1] shared-slot bases
+  static constexpr int OFF_IDX = OFF_SB + R16((TE + 1) * 4);         // buffer positions of the tile's slots
+  static constexpr int SMEM = OFF_IDX + R16(TE * NP * NP * 4);
 };
 
 struct McDmArgs {
@@ -1154,6 +1157,7 @@ struct McDmArgs {
   const int* elem_rn;
   const int* rn_row;
   double* sbuf;      // shared-block buffer, 4 doubles per slot
+  int n_slots;       // shared slots of all elements
   const int* sidx;   // buffer position of each element slot (fix-up order), or null (element order)
 };
 
@@ -1186,6 +1190,7 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
   const uint16_t* sPlan = reinterpret_cast<const uint16_t*>(smem + G::OFF_PLAN);
   int* sRow = reinterpret_cast<int*>(smem + G::OFF_ROW);
   int* sSb = reinterpret_cast<int*>(smem + G::OFF_SB);
+  int* sIdx = reinterpret_cast<int*>(smem + G::OFF_IDX);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int gq = lane >> 2, tq = lane & 3;  // MMA fragment group / thread in group
 
@@ -1226,7 +1231,8 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
       const int i = tid + k * NT;
       rnv[k] = i < ne_t * NP ? __ldg(T.elem_rn + (long long)tile * TE * NP + i) : -1;
     }
-    sbv = tid < ne_t ? __ldg(T.sbase + (long long)tile * TE + tid) : 0;
+    sbv = T.n_slots;  // one more than the tile has, for the end of its slots
+    if (tid < ne_t || (tid == ne_t && tile * TE + tid < A.n_el)) sbv = __ldg(T.sbase + (long long)tile * TE + tid);
   };
   auto fetch_values = [&]() {
 #pragma unroll
@@ -1257,7 +1263,7 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
         sRow[2 * (tid + k * NT)] = rsv[k][0];
         sRow[2 * (tid + k * NT) + 1] = rsv[k][1];
       }
-    if (tid < TE) sSb[tid] = sbv;
+    if (tid <= TE) sSb[tid] = sbv;
   };
   // one directed block (ra -> cb) of element el: into the COO rows or the
   // shared-block buffer
@@ -1266,7 +1272,7 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
     if (code == 0xFFFFu) return;
     if (code & 0x8000u) {
       const int slot = sSb[el] + (int)(code & 0x7FFFu);
-      double2* sb = reinterpret_cast<double2*>(T.sbuf) + 2 * (long long)(T.sidx ? __ldg(T.sidx + slot) : slot);
+      double2* sb = reinterpret_cast<double2*>(T.sbuf) + 2 * (long long)(T.sidx ? sIdx[slot - sSb[0]] : slot);
       sb[0] = make_double2(w00, w01);
       sb[1] = make_double2(w10, w11);
       return;
@@ -1277,11 +1283,7 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       const int rs = sRow[(el * NP + ra) * 2 + c];
-      if (rs < 0) continue;
-      int k = 0;
-#pragma unroll
-      for (int d = 0; d < 2; ++d)
-        if ((dm >> d) & 1u) hout[rs + off + k++] = w[c][d];
+      if (rs >= 0) store_pair(hout + rs + off, dm, w[c][0], w[c][1]);
     }
   };
 
@@ -1293,6 +1295,13 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
     const int ne = min(TE, A.n_el - e0);
     stash();
     __syncthreads();
+    if (T.sidx) {  // positions of the tile's shared slots, needed in (2)
+      const int s0 = sSb[0], ns = sSb[ne] - s0;
+      for (int i = tid; i < ns; i += NT)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(sIdx + i)),
+                     "l"(T.sidx + s0 + i)
+                     : "memory");
+    }
     // (1) constitutive update per (quadrature point, element) -> Ã (rows
     // q * 4 + k * 2 + l, columns (c * 2 + d) * TE + el) and the gradient helper
     for (int p = tid; p < TE * NQ; p += NT) {
@@ -1361,6 +1370,7 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
 #pragma unroll
         for (int j = 0; j < 4; ++j) sB[(q * 4 + kl) * NS + j * TE + el] = at[j][kl];
     }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
     // next tile's gather codes and geometry in flight during the MMAs
     fetch_codes(tile + gridDim.x);
@@ -1414,6 +1424,7 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
         }
       }
     }
+    fetch_values();  // on their way during (3)
     // (3) element gradient
     if (WANT & MW_G) {
       for (int i = tid; i < TE * N2; i += NT) {
@@ -1428,7 +1439,6 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
         gbuf[(long long)(e0 + el) * N2 + r] = acc;
       }
     }
-    fetch_values();
     __syncthreads();
   }
   if (WANT & MW_E) {
@@ -1493,6 +1503,7 @@ struct McHandle {
   // direct-write epilogue: per-element codes, shared-block buffer and the
   // fix-up plan over the shared blocks
   uint16_t* dp_code = nullptr;
+  int n_slots = 0;  // shared slots of all elements
   int *dp_sbase = nullptr, *dp_elem_rn = nullptr, *dp_sidx = nullptr;
   void* dp_sbuf = nullptr;  // 4 floats (tensor-core path) or 4 doubles (DMMA path) per slot
   // FP64 DMMA path (P2 / P4)
@@ -1612,7 +1623,7 @@ cudaError_t mc_launch(McHandle* h, int flags, const double* u, double* energy, d
     if (h->dm && (flags & MW_H)) {
       using G = McTileD<NP, NQ, GQ>;
       McDmArgs T{h->dp_code, h->dp_sbase, h->dp_elem_rn, h->bp_rn_row, static_cast<double*>(h->dp_sbuf),
-                 h->dp_sidx};
+                 h->n_slots, h->dp_sidx};
       double* g = static_cast<double*>(h->gbuf);
       double* H = static_cast<double*>(hess);
       const McConstR<double> Md = cast_const<double>(h->mc);
@@ -1985,6 +1996,7 @@ int mc_create(const fne_desc* d, McHandle** out) {
     dp.code.push_back(0xFFFF);
     MC_TRY(mc_upload(h, &h->dp_code, dp.code.data(), dp.code.size()));
     MC_TRY(mc_upload(h, &h->dp_sbase, dp.sbase.data(), dp.sbase.size()));
+    h->n_slots = (int)dp.sidx.size();
     MC_TRY(mc_upload(h, &h->dp_elem_rn, bp.elem_rn.data(), bp.elem_rn.size()));
     unsigned char* sb = nullptr;
     MC_TRY(mc_upload(h, &sb, (const unsigned char*)nullptr,
