@@ -1,7 +1,11 @@
 // libfne_asm.so -- element energy / gradient / Hessian assembly on sm_100a.
 //
-// Two kernel shapes (one per launch, no atomics, bit-reproducible):
+// Three kernel shapes (one per launch, no atomics, bit-reproducible):
 //
+//  * tile kernels (k_tiles_tri, k_nodes_tet; the defaults): a CTA owns a compact
+//    set of rows, evaluates what touches them into shared memory and sums it by
+//    lists written at set-up; the row-gather kernels and the banded sweep
+//    (k_sweep_tri) take the patterns that do not fit.
 //  * row-gather kernels (k_rows_tri, k_rows_tet): one thread per OUTPUT ROW
 //    of the owned COO pattern.  A CTA owns a contiguous block of rows, which
 //    is a contiguous slice of the COO value array -- the reference's overlap
@@ -2590,8 +2594,8 @@ extern "C" int fne_create(const fne_desc* d, fne_handle** out) {
     }
     if (!use_nodes && (rc = build_row_plan(d, plan, true))) return rc;
   }
-  // banded sweep for triangles (default), incidence-parallel on request,
-  // else the row-gather kernel
+  // triangles: tiles of rows (default) or the banded sweep, row clusters or
+  // incidence-parallel on request, else the row-gather kernel
   IncPlan inc;
   SweepPlan sweep;
   bool use_inc = false, use_sweep = false;
@@ -2599,7 +2603,7 @@ extern "C" int fne_create(const fne_desc* d, fne_handle** out) {
   if (is_tri(d->family) && plan.n_rows > 0 && d->kernel_variant == 2)
     use_inc = build_inc_plan(plan, kIncThreads, inc);
   const bool want_push = is_tri(d->family) && d->kernel_variant == 3;
-  // row clusters for triangles (default): windows of at most 8191 slots, sized
+  // row clusters for triangles (on request): windows of at most 8191 slots, sized
   // for three CTAs per SM, and about as many clusters as a whole number of
   // waves of them
   ClusterPlan cplan;

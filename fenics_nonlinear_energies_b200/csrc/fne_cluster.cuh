@@ -1,10 +1,9 @@
 // Row-cluster kernel for P1 triangles (p-Laplace, Ginzburg-Landau): a fused
-// energy / gradient / Hessian pass selected with kernel_variant 8 (the banded
-// sweep stays the default: on the 1024^2 grid this kernel measured 149 us per
-// FP64 pass against the sweep's 134 us, bound by its ~800 instructions per
-// element).  Included by fne_asm.cu
-// after the element physics (tri_full, tri_energy_r) and the FP64 energy
-// reduction.
+// energy / gradient / Hessian pass selected with kernel_variant 8 (not the
+// default: on the 1024^2 grid this kernel measured 149 us per FP64 pass, bound
+// by its ~800 instructions per element, against 83 us of k_tiles_tri).
+// Included by fne_asm.cu after the element physics (tri_full, tri_energy_r)
+// and the FP64 energy reduction.
 //
 // A persistent CTA (one per SM, 512 threads) walks its share of the row
 // clusters (ClusterPlan, fne_internal.h) through a two-deep software
