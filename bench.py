@@ -82,6 +82,7 @@ FLUSH_BYTES = 1 << 30
 # with the profile summary that records it.  Keyed by (workload, kernel).
 NCU_TRAFFIC = {
     ("gl1024_fp32h", "k_sweep_tri"): (213.2e6, "profiles/k_sweep_tri_gl1024_fp32.md"),
+    ("gl1024_fp64", "k_tiles_tri"): (265.0e6, "profiles/k_tiles_tri_gl1024_fp64.md"),
     ("gl1024_fp64", "k_sweep_tri"): (330.6e6, "profiles/k_sweep_tri_gl1024_fp64.md"),
 }
 
