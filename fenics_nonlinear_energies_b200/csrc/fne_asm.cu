@@ -2568,7 +2568,8 @@ extern "C" int fne_create(const fne_desc* d, fne_handle** out) {
     return set_error(FNE_EINVAL, "fne_create: p-Laplace needs p > 1");
 
   RowPlan plan;
-  // tets by default: tiles of whole row nodes, which need no incidence words
+  // tets by default: tiles of whole row nodes, which need no incidence words (a pattern without a place for every
+  // value goes on to the row plan, which refuses it)
   const bool try_nodes = d->family == FNE_NEOHOOKEAN && d->kernel_variant == 0;
   int rc = build_row_plan(d, plan, !try_nodes);
   if (rc) return rc;
@@ -2589,7 +2590,7 @@ extern "C" int fne_create(const fne_desc* d, fne_handle** out) {
       std::vector<int64_t> edofs((size_t)nl * 12);
       for (int64_t le = 0; le < nl; ++le)
         std::copy_n(d->elems + plan.local_elems[le] * 12, 12, edofs.begin() + le * 12);
-      use_nodes = build_block_plan(nl, 4, 3, edofs.data(), d, nbp) == FNE_OK &&
+      use_nodes = build_block_plan(nl, 4, 3, edofs.data(), d, nbp) == FNE_OK && nbp.whole &&
                   build_node_plan(nbp, plan.elem_weight, plan.elem_code, d->n_free, d->n_total, d->nnz, n_sms, nplan);
     }
     if (!use_nodes && (rc = build_row_plan(d, plan, true))) return rc;

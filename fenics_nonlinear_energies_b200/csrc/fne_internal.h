@@ -227,6 +227,9 @@ struct BlockPlan {
   std::vector<int32_t> con, inc;
   std::vector<int32_t> elem_rn;  // [n_local * npn] row node of each element node, -1 if none
   std::vector<int32_t> blk_rn;   // bs = 3: row node that is the block's column node, -1 if it has no owned row
+  // every block with contributions has all bs components and is its row node's only one of that column node: the
+  // pattern holds a place for every value of the node pairs
+  bool whole = true;
 };
 
 // Direct-write plan for kernels that hold whole element matrices: for every

@@ -634,6 +634,7 @@ int build_block_plan(int64_t n_local, int npn, int bs, const int64_t* elem_dofs,
       return set_error(FNE_ELAYOUT, "block plan: owned row without COO entries");
   }
   P.n_rnodes = n_rn;
+  P.whole = true;
   // column-node blocks of every row node: consecutive columns of one node
   // form a block; all rows of the node must agree on the blocks
   std::vector<int32_t> rn_blk(n_rn + 1, 0);
@@ -684,6 +685,8 @@ int build_block_plan(int64_t n_local, int npn, int bs, const int64_t* elem_dofs,
     for (int32_t b = rn_blk[k]; b < rn_blk[k + 1]; ++b) sorted_blk[b] = b;
     std::sort(sorted_blk.begin() + rn_blk[k], sorted_blk.begin() + rn_blk[k + 1],
               [&](int32_t x, int32_t y) { return blk_node[x] < blk_node[y]; });
+    for (int32_t b = rn_blk[k] + 1; b < rn_blk[k + 1]; ++b)
+      P.whole = P.whole && blk_node[sorted_blk[b]] != blk_node[sorted_blk[b - 1]];
   }
   auto find_blk = [&](int32_t k, int64_t node) -> int32_t {
     int32_t a = rn_blk[k], b = rn_blk[k + 1];
@@ -746,6 +749,7 @@ int build_block_plan(int64_t n_local, int npn, int bs, const int64_t* elem_dofs,
     const int32_t c = cnt[b + 1] - cnt[b];
     if (c >= (1 << 13)) return set_error(FNE_EBOUNDS, "block plan: more than 8191 contributions to one block");
     if (bs == 3) P.blk_rn[b] = rn_of[blk_node[b]];
+    P.whole = P.whole && (c == 0 || (blk_word[b] >> 16) == (1u << bs) - 1u);
     P.blk[b] = blk_word[b] | ((uint32_t)c << 19);
   }
   P.rn_blk = std::move(rn_blk);
