@@ -646,7 +646,9 @@ int build_pairs(const BlockPlan& bp, int64_t n_el, int np, std::vector<M3Pair>& 
       p.node_b = -1;
       if (both && B > A) {
         const auto first = order.begin() + bp.rn_blk[B], last = order.begin() + bp.rn_blk[B + 1];
-        const auto it = std::lower_bound(first, last, A, [&](int32_t x, int32_t v) { return bp.blk_rn[x] < v; });
+        auto it = std::lower_bound(first, last, A, [&](int32_t x, int32_t v) { return bp.blk_rn[x] < v; });
+        // (a row that lists a column node twice: the block that holds the contributions)
+        while (it != last && bp.blk_rn[*it] == A && (bp.blk[*it] >> 19) == 0) ++it;
         if (it == last || bp.blk_rn[*it] != A || (int32_t)(bp.blk[*it] >> 19) != cnt)
           return set_error(FNE_ELAYOUT, "Mohr-Coulomb 3-D: COO pattern is not symmetric over the owned rows");
         p.meta |= ((bp.blk[*it] >> 16) & 7u) << 19;

@@ -218,3 +218,37 @@ def test_mc3d_pattern_wider_than_the_element_graph(degree, n):
     assert abs(out["wider"][1] - out["plain"][1]).max() == 0.0
     sym = out["plain"][1]
     assert abs(sym - sym.T).max() <= 1e-12 * abs(sym).max()
+
+
+def test_mc3d_pattern_with_repeated_column_nodes(monkeypatch):
+    """Rows in any order that list all their columns twice: the two places of a value
+    hold it and zero, one way or the other, so their sums are the plain pattern's values."""
+    from scipy import sparse
+
+    from fenics_nonlinear_energies_b200 import _lib
+    from fenics_nonlinear_energies_b200.assembler import SlopeStability3DCudaAssembler
+
+    p = meshes.slope3d_problem(nx=3, ny=2, nz=3, degree=2, lam=1.2)
+    build = _lib.build_layout
+    rng = np.random.default_rng(5)
+
+    def repeated(**kw):
+        lay = build(**kw)
+        rows, cols = lay["owned_rows"], lay["owned_cols"]
+        parts = np.split(np.arange(rows.size), np.flatnonzero(rows[1:] != rows[:-1]) + 1)
+        at = np.concatenate([x for k in rng.permutation(len(parts)) for x in (parts[k], parts[k])])
+        lay["owned_rows"], lay["owned_cols"] = rows[at], cols[at]
+        return lay
+
+    plain = SlopeStability3DCudaAssembler(p)
+    monkeypatch.setattr(_lib, "build_layout", repeated)
+    twice = SlopeStability3DCudaAssembler(p)
+    u = torch.as_tensor(4e-2 * rng.standard_normal(plain.layout.n_free), device="cuda")
+    mats = []
+    for asm in (plain, twice):
+        _, _, h = asm.eval(u, 7)
+        lay = asm.layout
+        mats.append(sparse.coo_matrix((h.cpu().numpy(), (lay.owned_rows, lay.owned_cols)),
+                                      shape=(lay.n_free, lay.n_free)).tocsr())
+    assert twice.layout.owned_rows.size == 2 * plain.layout.owned_rows.size
+    assert abs(mats[1] - mats[0]).max() == 0.0
