@@ -521,6 +521,7 @@ int resident_spmv(const fne_cg* c) {
 
 void cg_free(fne_cg* c) {
   if (!c) return;
+  if (c->done) cudaEventSynchronize(c->done);  // a solve may have left a graph that reads these buffers
   if (c->exec) cudaGraphExecDestroy(c->exec);
   if (c->cap) cudaStreamDestroy(c->cap);
   cudaFree(c->crow);
@@ -674,18 +675,12 @@ extern "C" int fne_cg_set_matrix(fne_cg* c, const void* coo_vals, void* stream) 
   return rc;
 }
 
-extern "C" int fne_cg_solve(fne_cg* c, const double* b, double* x, double rtol, int32_t maxit, int32_t* its,
-                            int32_t* reason, void* stream) {
-  if (!c || (c->n > 0 && (!b || !x)) || maxit < 0 || !(rtol >= 0.0))
-    return set_error(FNE_EINVAL, "fne_cg_solve: bad arguments");
-  if (!c->have_matrix) return set_error(FNE_EINVAL, "fne_cg_solve: fne_cg_set_matrix was not called");
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (!c->exec) {
-    const int rc = build_graph(c);
-    if (rc != FNE_OK) return rc;
-  }
+namespace {
+
+// The work of fne_cg_solve; everything it leaves in `s` is behind it there.
+int cg_run(fne_cg* c, const double* b, double* x, double rtol, int32_t maxit, int32_t* its, int32_t* reason,
+           cudaStream_t s) {
   const fne::CgVecs a = vecs_of(c);
-  if (cudaStreamWaitEvent(s, c->done, 0) != cudaSuccess) return fne::cg_status("fne_cg_solve: stream order");
   fne::k_cg_init<<<c->grid_vec, fne::kCgThreads, 0, s>>>(a, b, rtol, maxit);
   int rc = fne::cg_status("fne_cg_solve: init");
   if (rc != FNE_OK) return rc;
@@ -718,10 +713,28 @@ extern "C" int fne_cg_solve(fne_cg* c, const double* b, double* x, double rtol, 
   const double* src = h->neg_first ? b : a.x;
   if (c->n > 0 && cudaMemcpyAsync(x, src, (size_t)c->n * sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
     return fne::cg_status("fne_cg_solve: result copy");
-  if (cudaEventRecord(c->done, s) != cudaSuccess) return fne::cg_status("fne_cg_solve: stream order");
   if (its) *its = h->neg_first ? 1 : h->its;
   if (reason) *reason = h->reason;
   return FNE_OK;
+}
+
+}  // namespace
+
+extern "C" int fne_cg_solve(fne_cg* c, const double* b, double* x, double rtol, int32_t maxit, int32_t* its,
+                            int32_t* reason, void* stream) {
+  if (!c || (c->n > 0 && (!b || !x)) || maxit < 0 || !(rtol >= 0.0))
+    return set_error(FNE_EINVAL, "fne_cg_solve: bad arguments");
+  if (!c->have_matrix) return set_error(FNE_EINVAL, "fne_cg_solve: fne_cg_set_matrix was not called");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (!c->exec) {
+    const int rc = build_graph(c);
+    if (rc != FNE_OK) return rc;
+  }
+  if (cudaStreamWaitEvent(s, c->done, 0) != cudaSuccess) return fne::cg_status("fne_cg_solve: stream order");
+  const int rc = cg_run(c, b, x, rtol, maxit, its, reason, s);
+  // also after a failure: graphs launched before it may still run
+  if (cudaEventRecord(c->done, s) != cudaSuccess && rc == FNE_OK) return fne::cg_status("fne_cg_solve: stream order");
+  return rc;
 }
 
 extern "C" int fne_cg_destroy(fne_cg* c) {

@@ -1,0 +1,45 @@
+"""The host side of the device CG (``fne_cg_solve``, ``fne_cg_destroy``) on a stand-in for the CUDA runtime
+(``cg_fake_runtime.cu``): which graphs it launches, what it records and waits for, failures included.  Runs on CPU."""
+
+import math
+import os
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+from fenics_nonlinear_energies_b200 import _lib, build
+
+HERE = Path(__file__).resolve().parent
+
+
+@pytest.fixture(scope="module")
+def solve(tmp_path_factory):
+    nvcc = build._nvcc()
+    if shutil.which(nvcc) is None:
+        pytest.skip("needs nvcc")
+    exe = tmp_path_factory.mktemp("cg") / "cg_host"
+    out = subprocess.run([nvcc, "-O0", "-std=c++17", *build.ARCH, "-cudart", "none", "-o", os.fspath(exe),
+                          os.fspath(HERE / "cg_fake_runtime.cu")], capture_output=True, text=True)
+    assert out.returncode == 0, out.stderr[-3000:]
+
+    def run(*residuals, chunk=16, fail_graph=-1, fail_wait=-1):
+        args = [chunk, fail_graph, fail_wait, *residuals]
+        text = subprocess.run([exe, *map(str, args)], capture_output=True, text=True, check=True, timeout=60).stdout
+        head, calls, freed = text.splitlines()
+        code, its, launches = map(int, head.split())
+        return {"code": code, "its": its, "launches": launches, "calls": calls.split(",")[:-1],
+                "destroy": freed.split(",")}
+
+    return run
+
+
+@pytest.mark.parametrize("failure", [{}, {"fail_graph": 1}, {"fail_graph": 2}, {"fail_wait": 0}, {"fail_wait": 1}])
+def test_end_of_work_is_recorded_on_every_way_out(solve, failure):
+    """A solve that put work into the stream leaves the event that a later call on another stream, or the release
+    of the handle, waits for -- also where a graph launch or a wait fails."""
+    r = solve(1e-1, 1e-2, 1e-3, -1, **failure)
+    assert r["code"] == (_lib.FNE_ECUDA if failure else _lib.FNE_OK)
+    assert "graph" in r["calls"] and r["calls"][-1] == "record done"
+    assert r["destroy"][0] == "wait done"
