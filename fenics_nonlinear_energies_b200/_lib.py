@@ -96,6 +96,7 @@ def _load():
         "fne_cg_set_matrix": (C.c_int, [vp, vp, vp]),
         "fne_cg_solve": (C.c_int, [vp, vp, vp, C.c_double, C.c_int32, C.POINTER(C.c_int32), C.POINTER(C.c_int32),
                                    vp]),
+        "fne_cg_launches": (C.c_int, [vp, _i64p]),
         "fne_cg_destroy": (C.c_int, [vp]),
         "fne_energy_p1tri_noalloc": (C.c_int, [C.c_int32, C.c_int64, vp, vp, vp, vp, vp, vp, vp, _f64p, vp,
                                                C.c_int64, C.c_int64, vp, vp]),

@@ -447,6 +447,7 @@ struct fne_cg {
   cudaStream_t cap = nullptr;
   cudaGraphExec_t exec = nullptr;
   bool have_matrix = false;
+  int64_t launches = 0;             // kernels launched by the last solve
 };
 
 namespace {
@@ -684,6 +685,7 @@ int cg_run(fne_cg* c, const double* b, double* x, double rtol, int32_t maxit, in
   fne::k_cg_init<<<c->grid_vec, fne::kCgThreads, 0, s>>>(a, b, rtol, maxit);
   int rc = fne::cg_status("fne_cg_solve: init");
   if (rc != FNE_OK) return rc;
+  c->launches = 1;
   // Graphs of `chunk` iterations run until one reports the stop.  The next is
   // put into the stream before the host has read the state of the one before
   // wherever the residual's mean rate says that it will be needed: a gap of some
@@ -693,6 +695,7 @@ int cg_run(fne_cg* c, const double* b, double* x, double rtol, int32_t maxit, in
   auto run_chunk = [&](int i) {
     if (cudaGraphLaunch(c->exec, s) != cudaSuccess || cudaEventRecord(c->ev[i & 1], s) != cudaSuccess)
       return fne::cg_status("fne_cg_solve: graph launch");
+    c->launches += 2 * c->chunk + 1;
     return (int)FNE_OK;
   };
   if ((rc = run_chunk(0))) return rc;
@@ -731,10 +734,17 @@ extern "C" int fne_cg_solve(fne_cg* c, const double* b, double* x, double rtol, 
     if (rc != FNE_OK) return rc;
   }
   if (cudaStreamWaitEvent(s, c->done, 0) != cudaSuccess) return fne::cg_status("fne_cg_solve: stream order");
+  c->launches = 0;
   const int rc = cg_run(c, b, x, rtol, maxit, its, reason, s);
   // also after a failure: graphs launched before it may still run
   if (cudaEventRecord(c->done, s) != cudaSuccess && rc == FNE_OK) return fne::cg_status("fne_cg_solve: stream order");
   return rc;
+}
+
+extern "C" int fne_cg_launches(const fne_cg* c, int64_t* launches) {
+  if (!c || !launches) return set_error(FNE_EINVAL, "fne_cg_launches: bad arguments");
+  *launches = c->launches;
+  return FNE_OK;
 }
 
 extern "C" int fne_cg_destroy(fne_cg* c) {

@@ -167,9 +167,10 @@ class DeviceCG:
         _lib.check(_lib.lib.fne_cg_solve(self._h, b.data_ptr(), x.data_ptr(), float(rtol), int(maxit),
                                          ctypes.byref(its), ctypes.byref(why), self._stream()))
         self.reason = self.REASONS[why.value]
-        # one initialisation kernel, then graphs of `chunk` iterations of two
-        # kernels and a state kernel until the one that holds the stop
-        self.launches += 1 + (2 * self.chunk + 1) * max(1, -(-int(its.value) // self.chunk))
+        # one initialisation kernel, then graphs of `chunk` iterations of two kernels and a state kernel
+        launches = ctypes.c_int64()
+        _lib.check(_lib.lib.fne_cg_launches(self._h, ctypes.byref(launches)))
+        self.launches += launches.value
         return x, int(its.value)
 
     def close(self):

@@ -353,6 +353,9 @@ int fne_cg_set_matrix(fne_cg* cg, const void* coo_vals, void* stream);
  * at a time (a later solve on another stream waits for this one). */
 int fne_cg_solve(fne_cg* cg, const double* b, double* x, double rtol, int32_t maxit, int32_t* its, int32_t* reason,
                  void* stream);
+/* Kernels that the last fne_cg_solve launched, those of a graph launched ahead
+ * that turned out not to be needed included. */
+int fne_cg_launches(const fne_cg* cg, int64_t* launches);
 int fne_cg_destroy(fne_cg* cg);
 
 /* ---------------------------------------------------------------------------

@@ -136,7 +136,9 @@ int main(int argc, char** argv) {
   calls.clear();
   launches = 0;
   const int rc = fne_cg_solve(c, v, x, 1e-6, 1000000, &its, &why, nullptr);
-  std::printf("%d %d %d\n", rc, its, launches);
+  int64_t told = -1;
+  fne_cg_launches(c, &told);
+  std::printf("%d %d %d %d\n", rc, its, launches, (int)told);
   for (const auto& s : calls) std::printf("%s,", s.c_str());
   calls.clear();
   fne_cg_destroy(c);

@@ -28,8 +28,8 @@ def solve(tmp_path_factory):
         args = [chunk, fail_graph, fail_wait, *residuals]
         text = subprocess.run([exe, *map(str, args)], capture_output=True, text=True, check=True, timeout=60).stdout
         head, calls, freed = text.splitlines()
-        code, its, launches = map(int, head.split())
-        return {"code": code, "its": its, "launches": launches, "calls": calls.split(",")[:-1],
+        code, its, launches, told = map(int, head.split())
+        return {"code": code, "its": its, "launches": launches, "told": told, "calls": calls.split(",")[:-1],
                 "destroy": freed.split(",")}
 
     return run
@@ -43,3 +43,16 @@ def test_end_of_work_is_recorded_on_every_way_out(solve, failure):
     assert r["code"] == (_lib.FNE_ECUDA if failure else _lib.FNE_OK)
     assert "graph" in r["calls"] and r["calls"][-1] == "record done"
     assert r["destroy"][0] == "wait done"
+
+
+@pytest.mark.parametrize("residuals", [(-1,), (1e-1, -1), (1e-1, 1e-2, -1), (0.9, 0.8, 0.7, -1), (0.5, 1e-14, -1)])
+def test_launches_count_the_graph_launched_ahead(solve, residuals):
+    """The kernels a solve reports are those it launched, where the graph after the one with the stop was launched too."""
+    r = solve(*residuals)
+    assert r["its"] == 16 * len(residuals) and r["told"] == r["launches"]
+    assert r["launches"] == 1 + 33 * r["calls"].count("graph")
+
+
+def test_a_graph_ahead_is_launched_in_these_cases(solve):
+    assert solve(0.9, 0.8, 0.7, -1)["calls"].count("graph") == 5
+    assert solve(-1)["calls"].count("graph") == 1
