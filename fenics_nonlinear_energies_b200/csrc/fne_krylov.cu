@@ -708,8 +708,10 @@ int cg_run(fne_cg* c, const double* b, double* x, double rtol, int32_t maxit, in
     h = c->st_host + (i & 1);
     if (h->stop) break;
     if (launched == i + 1 && (rc = run_chunk(launched++))) return rc;
-    // iterations still to go at the mean rate so far (rtol = 0: without end; not a number: unknown, wait)
-    const double rate = std::log(h->rr / h->rr0) / h->it, left = rate < 0.0 ? std::log(h->tol2 / h->rr) / rate : 1e9;
+    // iterations still to go at the mean rate so far (rtol = 0 or no decrease yet: without end; a residual that is
+    // not a finite number: none, the next iteration may stop)
+    const double rate = std::log(h->rr / h->rr0) / h->it;
+    const double left = rate < 0.0 ? std::log(h->tol2 / h->rr) / rate : std::isfinite(rate) ? 1e9 : 0.0;
     const bool more = left > c->chunk && h->it + c->chunk < h->maxit;
     if (more && launched == i + 2 && (rc = run_chunk(launched++))) return rc;
   }

@@ -56,3 +56,10 @@ def test_launches_count_the_graph_launched_ahead(solve, residuals):
 def test_a_graph_ahead_is_launched_in_these_cases(solve):
     assert solve(0.9, 0.8, 0.7, -1)["calls"].count("graph") == 5
     assert solve(-1)["calls"].count("graph") == 1
+
+
+@pytest.mark.parametrize("after_first", [math.nan, math.inf])
+def test_no_graph_ahead_of_a_residual_without_a_rate(solve, after_first):
+    """A residual that is not a number (or has overflowed) gives no rate to guess by: the next graph waits for the state."""
+    calls = solve(after_first, -1)["calls"]
+    assert calls == ["graph", "record ev0", "wait ev0", "graph", "record ev1", "wait ev1", "copy", "record done"]
