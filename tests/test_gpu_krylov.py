@@ -163,3 +163,60 @@ def test_cg_on_assembled_hessian(family):
     cg.close()
     asm.cleanup()
     del ref
+
+
+def _band_coo(n, m, seed, dense=0):
+    """SPD matrix of 2 m + 1 diagonals (ends cut), and a first row and column of ``dense`` entries; shuffled COO order."""
+    rng = np.random.default_rng(seed)
+    offs = np.sort(rng.choice(np.arange(1, 4 * m + 2), m, replace=False))
+    rows = np.concatenate([np.arange(n - d) for d in offs] + ([np.zeros(dense, dtype=np.int64)] if dense else []))
+    cols = np.concatenate([np.arange(d, n) for d in offs] + ([n - 1 - np.arange(dense)] if dense else []))
+    w = -(0.5 + rng.random(rows.size))
+    diag = np.full(n, 0.3)
+    np.add.at(diag, rows, -w)
+    np.add.at(diag, cols, -w)
+    r, c, v = np.r_[rows, cols, np.arange(n)], np.r_[cols, rows, np.arange(n)], np.r_[w, w, diag]
+    order = rng.permutation(r.size)
+    return n, r[order], c[order], v[order]
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("m,dense", [(3, 0), (4, 0), (5, 0), (7, 0), (2, 40), (4, 40), (9, 40), (9, 0), (20, 0)])
+def test_cg_row_lengths_match_oracle(m, dense, fp32):
+    """Every form of the product: rows of 7, 9, 11 and 15 entries stored column-major, and rows on CSR with 4, 8, 16
+    and 32 lanes (one row of 40 and more, or rows of 19 and 41), with a last batch of rows that is not full.  FP64
+    arithmetic in another order: the oracle's iteration count, and its iterate to 1e-9."""
+    n, rows, cols, vals = _band_coo(1003, m, 10 * m + dense, dense)
+    b = np.random.default_rng(m).standard_normal(n)
+    x, it, why, x_ref, it_ref, why_ref = _solve_both(n, rows, cols, vals, b, 1e-8, 500, fp32=fp32)
+    assert (it, why) == (it_ref, why_ref) == (it_ref, krylov.CONVERGED)
+    np.testing.assert_allclose(x, x_ref, rtol=0, atol=1e-9 * np.abs(x_ref).max())
+
+
+@pytest.mark.parametrize("m", [3, 9])
+def test_cg_one_handle_on_two_streams(m):
+    """Matrices and solves of one handle in turn on two streams, nothing waited for in between: a later call finds the
+    earlier solve finished, so every result is that of the same call on its own."""
+    from fenics_nonlinear_energies_b200.newton import DeviceCG
+
+    n, rows, cols, vals = _band_coo(200_003, m, 77)
+    b = torch.as_tensor(np.random.default_rng(1).standard_normal(n), device="cuda")
+    mats = [torch.as_tensor(vals * (1.0 + k * (rows == cols)), device="cuda") for k in range(4)]
+    alone = []
+    for v in mats:
+        cg = DeviceCG(n, rows, cols)
+        cg.update(v)
+        alone.append(cg.solve(b, rtol=1e-8, maxit=300))
+        torch.cuda.synchronize()
+        cg.close()
+    cg = DeviceCG(n, rows, cols)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    outs = []
+    for k, v in enumerate(mats):
+        with torch.cuda.stream(streams[k % 2]):
+            cg.update(v)
+            outs.append(cg.solve(b, rtol=1e-8, maxit=300))
+    torch.cuda.synchronize()
+    cg.close()
+    for (x, it), (x1, it1) in zip(outs, alone):
+        assert it == it1 and torch.equal(x, x1)
