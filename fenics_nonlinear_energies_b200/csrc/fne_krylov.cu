@@ -38,8 +38,10 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <memory>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "fne_internal.h"
@@ -61,7 +63,7 @@ struct alignas(16) CgState {
 };
 
 struct CgVecs {
-  const int32_t* crow;  // CSR, or null: column-major rows of `width` entries at stride `stride`, column -1 = none
+  const int32_t* crow;  // CSR; with width > 0 col and vals hold column-major rows of `width` entries at stride `stride`, column -1 = none
   const int32_t* col;
   const void* vals;
   const double* dinv;
@@ -413,6 +415,15 @@ __global__ void k_cg_values(int64_t nnz, int32_t n, const int32_t* __restrict__ 
   }
 }
 
+// Column-major rows from CSR: entry k of a row at k * stride, -1 beyond its end.
+__global__ void k_cg_columns(int32_t n, int32_t stride, int32_t width, const int32_t* __restrict__ crow,
+                             const int32_t* __restrict__ csr, int32_t* __restrict__ out) {
+  const int32_t row = blockIdx.x * blockDim.x + threadIdx.x;
+  if (row >= stride) return;
+  const int32_t k0 = row < n ? crow[row] : 0, len = row < n ? crow[row + 1] - k0 : 0;
+  for (int32_t k = 0; k < width; ++k) out[(size_t)k * stride + row] = k < len ? csr[k0 + k] : -1;
+}
+
 int cg_status(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(FNE_ECUDA, std::string(what) + ": " + cudaGetErrorString(e));
@@ -432,7 +443,7 @@ struct fne_cg {
   int grid_spmv = 1, grid_vec = 1;
   int width = 0;        // entries per row of the column-major form, 0: CSR
   int64_t n_vals = 0;   // stored values
-  int32_t* crow = nullptr;
+  int32_t* crow = nullptr;  // with diag, partial and st in one allocation
   int32_t* col = nullptr;
   int32_t* order = nullptr;
   int32_t* diag = nullptr;
@@ -528,12 +539,9 @@ void cg_free(fne_cg* c) {
   cudaFree(c->crow);
   cudaFree(c->col);
   cudaFree(c->order);
-  cudaFree(c->diag);
   cudaFree(c->vals);
   cudaFree(c->dinv);
   cudaFree(c->work);
-  cudaFree(c->partial);
-  cudaFree(c->st);
   if (c->st_host) cudaFreeHost(c->st_host);
   for (cudaEvent_t e : {c->ev[0], c->ev[1], c->done})
     if (e) cudaEventDestroy(e);
@@ -577,7 +585,7 @@ extern "C" int fne_cg_create(int32_t n, int64_t nnz, const int64_t* rows, const 
   if (!out || n < 0 || nnz < 0 || (nnz > 0 && (!rows || !cols)) || nnz > INT32_MAX || chunk < 1 || chunk > 4096)
     return set_error(FNE_EINVAL, "fne_cg_create: bad arguments");
   *out = nullptr;
-  std::vector<int32_t> crow((size_t)n + 1, 0), col((size_t)nnz), order((size_t)nnz), diag((size_t)n, -1);
+  std::vector<int32_t> crow((size_t)n + 1, 0);
   for (int64_t k = 0; k < nnz; ++k) {
     if (rows[k] < 0 || rows[k] >= n || cols[k] < 0 || cols[k] >= n)
       return set_error(FNE_EBOUNDS, "fne_cg_create: COO entry " + std::to_string(k) + " outside the n x n block");
@@ -598,18 +606,21 @@ extern "C" int fne_cg_create(int32_t n, int64_t nnz, const int64_t* rows, const 
   // column-major rows while they are short and padding stays within a quarter
   if (longest > 0 && longest <= 16 && c->nv * longest <= nnz + nnz / 4 + 4096) c->width = longest;
   c->n_vals = c->width ? c->nv * c->width : nnz;
-  std::vector<int32_t> fill(crow.begin(), crow.end() - 1);
-  if (c->width) {
-    col.assign((size_t)c->n_vals, -1);
-    order.assign((size_t)c->n_vals, -1);
+  // CSR on the host, written in the order of the rows; a scatter into column-major rows here would take twice as long
+  // as all of this (k_cg_columns does it on the device).  The arrays need no initial values.
+  std::unique_ptr<int32_t[]> col(new (std::nothrow) int32_t[(size_t)nnz]), order(new (std::nothrow) int32_t[(size_t)nnz]),
+      diag(new (std::nothrow) int32_t[(size_t)n]);
+  if (!col || !order || !diag) {
+    cg_free(c);
+    return set_error(FNE_EINVAL, "fne_cg_create: out of host memory");
   }
+  std::fill_n(diag.get(), n, -1);
+  std::vector<int32_t> fill(crow.begin(), crow.end() - 1);
   for (int64_t k = 0; k < nnz; ++k) {  // stable: COO order within a row
-    const int64_t row = rows[k];
-    const int32_t at = fill[(size_t)row]++;
-    const size_t pos = c->width ? (size_t)(at - crow[row]) * c->nv + row : (size_t)at;
+    const int32_t pos = fill[(size_t)rows[k]]++;
     order[pos] = (int32_t)k;
     col[pos] = (int32_t)cols[k];
-    if (row == cols[k]) diag[(size_t)row] = (int32_t)k;
+    if (rows[k] == cols[k]) diag[rows[k]] = (int32_t)k;
   }
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -624,28 +635,43 @@ extern "C" int fne_cg_create(int32_t n, int64_t nnz, const int64_t* rows, const 
   c->grid_spmv = (int)std::max<int64_t>(1, std::min<int64_t>(want_spmv, (int64_t)sms * per_sm_spmv));
   c->grid_vec = (int)std::max<int64_t>(1, std::min<int64_t>(want_vec, (int64_t)sms * per_sm_vec));
   const size_t vsz = c->vals_fp32 ? sizeof(float) : sizeof(double);
-  bool ok = cudaMalloc(&c->crow, crow.size() * sizeof(int32_t)) == cudaSuccess &&
-            cudaMalloc(&c->col, std::max<size_t>(1, col.size()) * sizeof(int32_t)) == cudaSuccess &&
-            cudaMalloc(&c->order, std::max<size_t>(1, order.size()) * sizeof(int32_t)) == cudaSuccess &&
-            cudaMalloc(&c->diag, std::max<size_t>(1, diag.size()) * sizeof(int32_t)) == cudaSuccess &&
+  auto up = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+  const size_t o_diag = up(((size_t)n + 1) * sizeof(int32_t)), o_part = o_diag + up((size_t)n * sizeof(int32_t));
+  const size_t o_st = o_part + up(((size_t)c->grid_spmv + 2 * (size_t)c->grid_vec) * sizeof(double));
+  char* base = nullptr;
+  bool ok = cudaMalloc(&base, o_st + 2 * sizeof(fne::CgState)) == cudaSuccess &&
+            cudaMalloc(&c->col, std::max<size_t>(1, (size_t)c->n_vals) * sizeof(int32_t)) == cudaSuccess &&
+            cudaMalloc(&c->order, std::max<size_t>(1, (size_t)c->n_vals) * sizeof(int32_t)) == cudaSuccess &&
             cudaMalloc(&c->vals, std::max<size_t>(1, (size_t)c->n_vals) * vsz) == cudaSuccess &&
             cudaMalloc(&c->dinv, std::max<size_t>(32, (size_t)c->nv) * sizeof(double)) == cudaSuccess &&
             cudaMalloc(&c->work, std::max<size_t>(32, 6 * (size_t)c->nv) * sizeof(double)) == cudaSuccess &&
-            cudaMalloc(&c->partial, ((size_t)c->grid_spmv + 2 * (size_t)c->grid_vec) * sizeof(double)) == cudaSuccess &&
-            cudaMalloc(&c->st, 2 * sizeof(fne::CgState)) == cudaSuccess &&
             cudaHostAlloc(&c->st_host, 2 * sizeof(fne::CgState), cudaHostAllocDefault) == cudaSuccess &&
             cudaEventCreateWithFlags(&c->ev[0], cudaEventDisableTiming) == cudaSuccess &&
             cudaEventCreateWithFlags(&c->ev[1], cudaEventDisableTiming) == cudaSuccess &&
             cudaEventCreateWithFlags(&c->done, cudaEventDisableTiming) == cudaSuccess &&
             cudaStreamCreateWithFlags(&c->cap, cudaStreamNonBlocking) == cudaSuccess;
-  ok = ok && cudaMemcpy(c->crow, crow.data(), crow.size() * sizeof(int32_t), cudaMemcpyHostToDevice) == cudaSuccess;
-  ok = ok && (nnz == 0 || (cudaMemcpy(c->col, col.data(), col.size() * sizeof(int32_t), cudaMemcpyHostToDevice) ==
-                               cudaSuccess &&
-                           cudaMemcpy(c->order, order.data(), order.size() * sizeof(int32_t),
-                                      cudaMemcpyHostToDevice) == cudaSuccess));
-  ok = ok && (n == 0 || cudaMemcpy(c->diag, diag.data(), diag.size() * sizeof(int32_t), cudaMemcpyHostToDevice) ==
-                            cudaSuccess);
+  c->crow = reinterpret_cast<int32_t*>(base);
+  if (base) {
+    c->diag = reinterpret_cast<int32_t*>(base + o_diag);
+    c->partial = reinterpret_cast<double*>(base + o_part);
+    c->st = reinterpret_cast<fne::CgState*>(base + o_st);
+  }
+  auto put = [&](void* dst, const int32_t* src, size_t count) {
+    ok = ok && (count == 0 || cudaMemcpy(dst, src, count * sizeof(int32_t), cudaMemcpyHostToDevice) == cudaSuccess);
+  };
+  put(c->crow, crow.data(), crow.size());
+  put(c->diag, diag.get(), (size_t)n);
+  for (auto [dst, src] : {std::pair(c->col, col.get()), std::pair(c->order, order.get())}) {
+    // (the values' place, at least as long, is free until fne_cg_set_matrix)
+    put(c->width ? c->vals : dst, src, (size_t)nnz);
+    if (ok && c->width) {
+      fne::k_cg_columns<<<(int)((c->nv + 255) / 256), 256>>>(n, (int32_t)c->nv, c->width, c->crow,
+                                                           static_cast<const int32_t*>(c->vals), dst);
+      ok = cudaGetLastError() == cudaSuccess;
+    }
+  }
   ok = ok && cudaMemset(c->st, 0, 2 * sizeof(fne::CgState)) == cudaSuccess;
+  ok = ok && cudaStreamSynchronize(0) == cudaSuccess;  // (a solve may use a stream that does not wait for this one)
   if (!ok) {
     cudaGetLastError();
     cg_free(c);
