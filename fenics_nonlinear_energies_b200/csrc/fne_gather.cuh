@@ -164,13 +164,15 @@ __global__ void __launch_bounds__(256) k_node_gather(NodeGatherArgs G, const Rea
 
 // One row of a 2x2 node block: its free components (bits of dm) at
 // consecutive positions from o.  Blocks of a row lie apart, so every store is
-// a sector of its own in L2, and the pair is one store where it is aligned
-// (fixed components give rows of odd length, so it may not be): half of the
-// P4 pass's 46 M sectors (FP64: 381 -> 354 us for the Hessian on 50,344
-// elements).
-template <typename HOut, typename T>
+// a sector of its own in L2, and PAIR makes the pair one store where it is
+// aligned (fixed components give rows of odd length, so it may not be): half of
+// the P4 pass's 46 M sectors (FP64: 381 -> 354 us for the Hessian on 50,344
+// elements).  A P2 pass writes a fifth of them and is bound by instructions,
+// where the test and the second way to store cost more than the sectors (FP32:
+// 86 -> 98 us, FP64: 73 -> 77): PAIR is for P4.
+template <bool PAIR, typename HOut, typename T>
 __device__ __forceinline__ void store_pair(HOut* __restrict__ o, unsigned dm, T v0, T v1) {
-  if (dm == 3u && (reinterpret_cast<uintptr_t>(o) & (2 * sizeof(HOut) - 1)) == 0) {
+  if (PAIR && dm == 3u && (reinterpret_cast<uintptr_t>(o) & (2 * sizeof(HOut) - 1)) == 0) {
     if constexpr (sizeof(HOut) == 8)
       *reinterpret_cast<double2*>(o) = make_double2((double)v0, (double)v1);
     else
@@ -188,8 +190,8 @@ __device__ __forceinline__ void store_pair(HOut* __restrict__ o, unsigned dm, T 
 // fix-up order and the block's contributions are the consecutive slots
 // desc.z .. desc.z + count - 1 (streamed); else they are the buffer slots
 // slots[desc.z .. desc.z + count) (gathered).  SB: the buffer's value type
-// (float: tensor-core path; double: FP64 DMMA path).
-template <typename HOut, typename SB>
+// (float: tensor-core path; double: FP64 DMMA path); PAIR: see store_pair.
+template <typename HOut, typename SB, bool PAIR>
 __global__ void __launch_bounds__(256) k_fixup2(int n_blk, const int4* __restrict__ desc,
                                                 const int* __restrict__ slots, const SB* __restrict__ sbuf,
                                                 HOut* __restrict__ out) {
@@ -249,8 +251,8 @@ __global__ void __launch_bounds__(256) k_fixup2(int n_blk, const int4* __restric
         }
       }
     }
-    if (ds.x >= 0) store_pair(out + ds.x, dm, a00, a01);
-    if (ds.y >= 0) store_pair(out + ds.y, dm, a10, a11);
+    if (ds.x >= 0) store_pair<PAIR>(out + ds.x, dm, a00, a01);
+    if (ds.y >= 0) store_pair<PAIR>(out + ds.y, dm, a10, a11);
   }
 }
 

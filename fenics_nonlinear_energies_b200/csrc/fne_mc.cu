@@ -953,7 +953,7 @@ __global__ void __launch_bounds__(McTile<NP, NQ, GQ>::THREADS, McTile<NP, NQ, GQ
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           const int rs = sRow[(el * NP + ra) * 2 + c];
-          if (rs >= 0) store_pair(hout + rs + off, dm, w[c][0], w[c][1]);
+          if (rs >= 0) store_pair<(NP > 6)>(hout + rs + off, dm, w[c][0], w[c][1]);
         }
       };
       if (!*sFail && quad * 32 < NPAIR) {
@@ -1148,7 +1148,8 @@ struct McTileD {
   static constexpr int OFF_ROW = OFF_PLAN + R16(PLAN_WORDS * 4);     // [TE][NP][2] row starts
   static constexpr int OFF_SB = OFF_ROW + R16(TE * NP * 2 * 4);      // [TE + 1] shared-slot bases
   static constexpr int OFF_IDX = OFF_SB + R16((TE + 1) * 4);         // buffer positions of the tile's slots
-  static constexpr int SMEM = OFF_IDX + R16(TE * NP * NP * 4);
+  static constexpr bool FX = NP > 6;                                 // shared slots in fix-up order (P4)
+  static constexpr int SMEM = OFF_IDX + (FX ? R16(TE * NP * NP * 4) : 0);
 };
 
 struct McDmArgs {
@@ -1231,8 +1232,8 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
       const int i = tid + k * NT;
       rnv[k] = i < ne_t * NP ? __ldg(T.elem_rn + (long long)tile * TE * NP + i) : -1;
     }
-    sbv = T.n_slots;  // one more than the tile has, for the end of its slots
-    if (tid < ne_t || (tid == ne_t && tile * TE + tid < A.n_el)) sbv = __ldg(T.sbase + (long long)tile * TE + tid);
+    sbv = T.n_slots;  // in fix-up order one more than the tile has, for the end of its slots
+    if (tid < ne_t || (G::FX && tid == ne_t && tile * TE + tid < A.n_el)) sbv = __ldg(T.sbase + (long long)tile * TE + tid);
   };
   auto fetch_values = [&]() {
 #pragma unroll
@@ -1272,7 +1273,7 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
     if (code == 0xFFFFu) return;
     if (code & 0x8000u) {
       const int slot = sSb[el] + (int)(code & 0x7FFFu);
-      double2* sb = reinterpret_cast<double2*>(T.sbuf) + 2 * (long long)(T.sidx ? sIdx[slot - sSb[0]] : slot);
+      double2* sb = reinterpret_cast<double2*>(T.sbuf) + 2 * (long long)(G::FX ? sIdx[slot - sSb[0]] : slot);
       sb[0] = make_double2(w00, w01);
       sb[1] = make_double2(w10, w11);
       return;
@@ -1283,7 +1284,7 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       const int rs = sRow[(el * NP + ra) * 2 + c];
-      if (rs >= 0) store_pair(hout + rs + off, dm, w[c][0], w[c][1]);
+      if (rs >= 0) store_pair<(NP > 6)>(hout + rs + off, dm, w[c][0], w[c][1]);
     }
   };
 
@@ -1295,7 +1296,7 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
     const int ne = min(TE, A.n_el - e0);
     stash();
     __syncthreads();
-    if (T.sidx) {  // positions of the tile's shared slots, needed in (2)
+    if constexpr (G::FX) {  // positions of the tile's shared slots, needed in (2)
       const int s0 = sSb[0], ns = sSb[ne] - s0;
       for (int i = tid; i < ns; i += NT)
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(sIdx + i)),
@@ -1370,7 +1371,7 @@ __global__ void __launch_bounds__(McTileD<NP, NQ, GQ>::THREADS, McTileD<NP, NQ, 
 #pragma unroll
         for (int j = 0; j < 4; ++j) sB[(q * 4 + kl) * NS + j * TE + el] = at[j][kl];
     }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    if constexpr (G::FX) asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
     // next tile's gather codes and geometry in flight during the MMAs
     fetch_codes(tile + gridDim.x);
@@ -1548,12 +1549,12 @@ cudaError_t mc_gathers(McHandle* h, int flags, const Real* K, const Real* g, dou
         if (h->n_fix > 0) {
           const int gf = std::max(1, std::min(h->num_sms * 16, (h->n_fix + 255) / 256));
           if (h->dm)
-            k_fixup2<HOut, double><<<gf, 256, 0, st>>>(h->n_fix, reinterpret_cast<const int4*>(h->fx_desc),
-                                                       h->dp_sidx ? nullptr : h->fx_con,
-                                                       static_cast<const double*>(h->dp_sbuf), H);
+            k_fixup2<HOut, double, (NP > 6)><<<gf, 256, 0, st>>>(h->n_fix, reinterpret_cast<const int4*>(h->fx_desc),
+                                                                 h->dp_sidx ? nullptr : h->fx_con,
+                                                                 static_cast<const double*>(h->dp_sbuf), H);
           else
-            k_fixup2<HOut, float><<<gf, 256, 0, st>>>(h->n_fix, reinterpret_cast<const int4*>(h->fx_desc),
-                                                      h->fx_con, static_cast<const float*>(h->dp_sbuf), H);
+            k_fixup2<HOut, float, (NP > 6)><<<gf, 256, 0, st>>>(h->n_fix, reinterpret_cast<const int4*>(h->fx_desc),
+                                                                h->fx_con, static_cast<const float*>(h->dp_sbuf), H);
         }
       } else {
         NodeGatherArgs G{h->n_rnodes, h->bp_rn_blk, h->bp_rn_con, h->bp_rn_row, h->bp_rn_gpos,
