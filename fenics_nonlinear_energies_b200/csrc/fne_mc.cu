@@ -350,7 +350,9 @@ __device__ __forceinline__ long long lin_at(int e, int q, int k) {
   return (((long long)(e / kLinTile) * NQ + q) * 6 + k) * kLinTile + e % kLinTile;
 }
 
-// One tile per CTA, threads over (quadrature point, element).
+// Threads over (quadrature point, element) of a tile, the points dealt out over
+// blockIdx.y: a mesh of few tiles leaves SMs idle while every thread runs up to
+// five point updates one after the other (mc_lin_launch_g's rule).
 template <typename Real, int NP, int NQ, bool GQ>
 __global__ void __launch_bounds__(128) k_mc_lin(McArgs A, McConstR<Real> M, Real* __restrict__ wct) {
   constexpr int TE = kLinTile, N2 = 2 * NP, NT = 128, US = N2 + 1;
@@ -370,7 +372,7 @@ __global__ void __launch_bounds__(128) k_mc_lin(McArgs A, McConstR<Real> M, Real
   }
   for (int i = tid; i < ne * GS; i += NT) sGm[i] = (Real)__ldg(A.geom + (long long)e0 * GS + i);
   __syncthreads();
-  for (int p = tid; p < TE * NQ; p += NT) {
+  for (int p = blockIdx.y * NT + tid; p < TE * NQ; p += gridDim.y * NT) {
     const int q = p / TE, el = p - q * TE;
     if (el >= ne) continue;
     const Real* gm = sGm + el * GS + (GQ ? 5 * q : 0);
@@ -2092,7 +2094,10 @@ cudaError_t mc_lin_launch_g(McHandle* h, int op, const double* v, double* out, c
   Real* eb = static_cast<Real*>(h->lin_ebuf);
   const int grid = h->grid_elem, T = 32 * kMcWarps, n_tiles = (h->n_local + kLinTile - 1) / kLinTile;
   if (op == 0) {
-    if (n_tiles > 0) k_mc_lin<Real, NP, NQ, GQ><<<n_tiles, 128, 0, st>>>(A, cast_const<Real>(h->mc), wct);
+    // four CTAs per SM at least, as far as the points of a tile can be dealt out
+    const int rounds = (kLinTile * NQ + 127) / 128;
+    const int slices = std::min(rounds, n_tiles > 0 ? (4 * h->num_sms + n_tiles - 1) / n_tiles : 1);
+    if (n_tiles > 0) k_mc_lin<Real, NP, NQ, GQ><<<dim3(n_tiles, slices), 128, 0, st>>>(A, cast_const<Real>(h->mc), wct);
     return cudaGetLastError();
   }
   if (op == 1) {
