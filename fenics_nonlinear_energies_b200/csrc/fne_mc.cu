@@ -486,37 +486,57 @@ __global__ void __launch_bounds__(kHvpThreads) k_mc_hvp(McArgs A, const Real* __
   for (int i = tid; i < ne * N; i += NT) ebuf[(long long)e0 * N + i] = s_x[(i % N) * PS + i / N];
 }
 
-// The diagonal: one warp per element, lanes over its DOFs.
+// The diagonal, over the same tiles: one element per lane, warps over pairs of
+// nodes, which share the loads of a point's tangent (whole lines, from L1 after
+// the first warp).  With one warp per element the tangents' tiles were read six
+// values 256 bytes apart (72 us for
+// 50,344 P4 elements with the gradient rows, 39 us so; P2 39 and 21).
 template <typename Real, int NP, int NQ, bool GQ>
-__global__ void __launch_bounds__(32 * kMcWarps) k_mc_hvp_diag(McArgs A, const Real* __restrict__ wct,
-                                                               Real* __restrict__ ebuf) {
-  constexpr int N = 2 * NP;
-  __shared__ Real s_dh1[NQ * NP], s_dh2[NQ * NP];
-  for (int i = threadIdx.x; i < NQ * NP; i += blockDim.x) {
-    s_dh1[i] = (Real)A.dhat1[i];
-    s_dh2[i] = (Real)A.dhat2[i];
+__global__ void __launch_bounds__(kHvpThreads) k_mc_hvp_diag(McArgs A, const Real* __restrict__ wct,
+                                                             Real* __restrict__ ebuf) {
+  constexpr int TE = kLinTile, N = 2 * NP, NT = kHvpThreads, PS = TE + 1, PAIRS = (NP + 1) / 2;
+  using V2 = typename std::conditional<sizeof(Real) == 8, double2, float2>::type;
+  __shared__ V2 s_tab[NQ * NP + 1];
+  __shared__ Real s_y[N * PS];  // [DOF][element]
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int e0 = blockIdx.x * TE, ne = min(TE, A.n_el - e0);
+  for (int i = tid; i < NQ * NP; i += NT) {
+    V2 t;
+    t.x = (Real)__ldg(A.dhat1 + i);
+    t.y = (Real)__ldg(A.dhat2 + i);
+    s_tab[i] = t;
+  }
+  const int e = min(e0 + lane, A.n_el - 1);  // idle lanes follow the last element and store nothing
+  const double* gm = A.geom + (long long)geo_stride<NQ, GQ>() * e;
+  __syncthreads();
+  for (int g = wid; g < PAIRS; g += NT / 32) {
+    Real y[4] = {Real(0), Real(0), Real(0), Real(0)}, J[4];
+    if (!GQ)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) J[k] = (Real)__ldg(gm + k);
+#pragma unroll 2
+    for (int q = 0; q < NQ; ++q) {
+      Real C[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) C[k] = __ldg(wct + lin_at<NQ>(e, q, k));
+      if (GQ)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) J[k] = (Real)__ldg(gm + 5 * q + k);
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        // B columns of node a: (px, 0, py) and (0, py, px)
+        const V2 r = s_tab[q * NP + 2 * g + n];  // (the last of an odd count is not used)
+        const Real px = J[0] * r.x + J[1] * r.y, py = J[2] * r.x + J[3] * r.y;
+        y[2 * n] += px * (C[0] * px + C[2] * py) + py * (C[2] * px + C[5] * py);
+        y[2 * n + 1] += py * (C[3] * py + C[4] * px) + px * (C[4] * py + C[5] * px);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (4 * g + k < N) s_y[(4 * g + k) * PS + lane] = y[k];
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int e = blockIdx.x * kMcWarps + wid; e < A.n_el; e += gridDim.x * kMcWarps) {
-    const double* gm = A.geom + (long long)geo_stride<NQ, GQ>() * e;
-    for (int i = lane; i < N; i += 32) {
-      const int a = i >> 1, c = i & 1;
-      Real acc = Real(0);
-      for (int q = 0; q < NQ; ++q) {
-        const Real r1 = s_dh1[q * NP + a], r2 = s_dh2[q * NP + a];
-        // B column (a, c): c = 0 -> (px, 0, py); c = 1 -> (0, py, px)
-        const double* gq = gm + (GQ ? 5 * q : 0);
-        const Real px = (Real)gq[0] * r1 + (Real)gq[1] * r2, py = (Real)gq[2] * r1 + (Real)gq[3] * r2;
-        Real C[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) C[k] = wct[lin_at<NQ>(e, q, k)];
-        acc += c == 0 ? px * (C[0] * px + C[2] * py) + py * (C[2] * px + C[5] * py)
-                      : py * (C[3] * py + C[4] * px) + px * (C[4] * py + C[5] * px);
-      }
-      ebuf[(long long)e * N + i] = acc;
-    }
-  }
+  for (int i = tid; i < ne * N; i += NT) ebuf[(long long)e0 * N + i] = s_y[(i % N) * PS + i / N];
 }
 
 // ---------------------------------------------------------------------------
@@ -2103,7 +2123,7 @@ cudaError_t mc_lin_launch_g(McHandle* h, int op, const double* v, double* out, c
   if (op == 1) {
     if (n_tiles > 0) k_mc_hvp<Real, NP, NQ, GQ><<<n_tiles, kHvpThreads, 0, st>>>(A, wct, eb);
   } else {
-    k_mc_hvp_diag<Real, NP, NQ, GQ><<<grid, T, 0, st>>>(A, wct, eb);
+    if (n_tiles > 0) k_mc_hvp_diag<Real, NP, NQ, GQ><<<n_tiles, kHvpThreads, 0, st>>>(A, wct, eb);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
