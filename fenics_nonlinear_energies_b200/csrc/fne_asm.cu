@@ -2800,11 +2800,14 @@ extern "C" int fne_create(const fne_desc* d, fne_handle** out) {
     FNE_TRY(upload(h, &h->rec, recs.data(), recs.size()));
     FNE_TRY(upload(h, &h->rec_dir_only, dro.data(), dro.size()));
   }
-  FNE_TRY(upload(h, &h->row_ptr, plan.row_ptr.data(), plan.row_ptr.size()));
-  FNE_TRY(upload(h, &h->row_node, plan.row_node.data(), plan.row_node.size()));
-  FNE_TRY(upload(h, &h->row_comp, plan.row_comp.data(), plan.row_comp.size()));
-  FNE_TRY(upload(h, &h->row_gpos, plan.row_gpos.data(), plan.row_gpos.size()));
-  FNE_TRY(upload(h, &h->inc_ptr, plan.inc_ptr.data(), plan.inc_ptr.size()));
+  const bool own_lists = use_tiles || use_nodes;  // tiles read no rows or incidences of the row plan
+  if (!own_lists) {
+    FNE_TRY(upload(h, &h->row_ptr, plan.row_ptr.data(), plan.row_ptr.size()));
+    FNE_TRY(upload(h, &h->row_node, plan.row_node.data(), plan.row_node.size()));
+    FNE_TRY(upload(h, &h->row_comp, plan.row_comp.data(), plan.row_comp.size()));
+    FNE_TRY(upload(h, &h->row_gpos, plan.row_gpos.data(), plan.row_gpos.size()));
+    FNE_TRY(upload(h, &h->inc_ptr, plan.inc_ptr.data(), plan.inc_ptr.size()));
+  }
   if (use_cluster) {
     std::vector<int32_t> codes;
     if (f32) {
@@ -2855,7 +2858,7 @@ extern "C" int fne_create(const fne_desc* d, fne_handle** out) {
     FNE_TRY(upload(h, &h->inc_elem2, inc.inc_elem.data(), inc.inc_elem.size()));
     FNE_TRY(upload(h, &h->inc_word, inc.inc_word.data(), inc.inc_word.size()));
     FNE_TRY(upload(h, &h->inc_rowl, inc.inc_rowl.data(), inc.inc_rowl.size()));
-  } else {
+  } else if (!own_lists) {
     FNE_TRY(upload(h, &h->inc_elem, plan.inc_elem.data(), plan.inc_elem.size()));
     FNE_TRY(upload(h, &h->inc_info, plan.inc_info.data(), plan.inc_info.size()));
   }

@@ -489,8 +489,8 @@ __global__ void __launch_bounds__(kHvpThreads) k_mc_hvp(McArgs A, const Real* __
 // The diagonal, over the same tiles: one element per lane, warps over pairs of
 // nodes, which share the loads of a point's tangent (whole lines, from L1 after
 // the first warp).  With one warp per element the tangents' tiles were read six
-// values 256 bytes apart (72 us for
-// 50,344 P4 elements with the gradient rows, 39 us so; P2 39 and 21).
+// values 256 bytes apart (72 us for 50,344 P4 elements with the gradient rows,
+// 39 us so; P2 39 and 21).
 template <typename Real, int NP, int NQ, bool GQ>
 __global__ void __launch_bounds__(kHvpThreads) k_mc_hvp_diag(McArgs A, const Real* __restrict__ wct,
                                                              Real* __restrict__ ebuf) {

@@ -461,3 +461,13 @@ def test_tri_tiles_match_row_gather(mesh, family, precision):
     for flags, k in ((2, 1), (4, 2), (3, 1), (5, 2), (6, 2)):
         assert torch.equal(a.eval(u, flags)[k], (ea, ga, ha)[k])
     assert all(torch.equal(x, y) for x, y in zip(a.eval(u, 7), (ea, ga, ha)))
+
+
+def test_tiles_hold_no_row_lists():
+    """Device memory of a triangle handle on the tile kernel: records (80 bytes) and the tiles' lists (per triangle
+    1.2 x 60 bytes of words and geometry, 28 of row words, some 6 of node lists and Dirichlet values), not the rows
+    and incidences (32 bytes more) that only the row-gather kernel reads."""
+    params, _ = meshes.gl_problem(n=200)
+    asm = _asm_classes()["gl"](params)
+    assert asm.info["kernel_variant"] == 12
+    assert asm.info["device_bytes"] <= 200 * params["elems"].shape[0]
