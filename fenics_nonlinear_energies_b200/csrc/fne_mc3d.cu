@@ -613,46 +613,63 @@ int m3_upload(Mc3dHandle* h, T** p, const T* src, size_t count) {
 
 // Pairs of row nodes from the node-block plan: every block (A, B) with element
 // contributions once, from the row node with the smaller index when both have
-// owned rows.  Codes stay
-// below 2^31: n_elem * pairs * 9 < 2^33 is checked by the caller.
+// owned rows.  Codes stay below 2^31: n_elem * pairs * 9 < 2^33 is checked by the
+// caller.
 int build_pairs(const BlockPlan& bp, int64_t n_el, int np, std::vector<M3Pair>& pairs, std::vector<int32_t>& pair_a,
                 std::vector<int32_t>& con) {
   const int npair = np * (np + 1) / 2, n = bp.n_rnodes;
-  // blocks of every row node in the order of their column's row node, to find (B, A)
-  std::vector<int32_t> order(bp.blk.size());
-  for (int32_t k = 0; k < n; ++k) {
-    for (int32_t b = bp.rn_blk[k]; b < bp.rn_blk[k + 1]; ++b) order[b] = b;
-    std::sort(order.begin() + bp.rn_blk[k], order.begin() + bp.rn_blk[k + 1],
-              [&](int32_t x, int32_t y) { return bp.blk_rn[x] < bp.blk_rn[y]; });
+  // blocks with contributions by their column's row node, to find (B, A): those in column A give every row B its block
+  std::vector<int32_t> col_ptr((size_t)n + 1, 0), col_blk, blk_row(bp.blk.size()), block_in_col((size_t)n, -1);
+  for (int32_t k = 0; k < n; ++k)
+    for (int32_t b = bp.rn_blk[k]; b < bp.rn_blk[k + 1]; ++b) {
+      blk_row[b] = k;
+      if (bp.blk_rn[b] >= 0 && (bp.blk[b] >> 19)) ++col_ptr[bp.blk_rn[b] + 1];
+    }
+  for (int32_t k = 0; k < n; ++k) col_ptr[k + 1] += col_ptr[k];
+  col_blk.resize((size_t)col_ptr[n]);
+  {
+    std::vector<int32_t> at(col_ptr.begin(), col_ptr.end() - 1);
+    for (int32_t b = 0; b < (int32_t)bp.blk.size(); ++b)
+      if (bp.blk_rn[b] >= 0 && (bp.blk[b] >> 19)) col_blk[at[bp.blk_rn[b]]++] = b;
   }
-  pairs.reserve(bp.blk.size() / 2 + n);
-  pair_a.reserve(bp.blk.size() / 2 + n);
+  // element contributions come in both directions; a block without any (a pattern wider than the element graph,
+  // which need not be symmetric) is a zero of its own
+  const auto mirrored = [&](int32_t A, int32_t b) { return (bp.blk[b] >> 19) && bp.blk_rn[b] >= 0 && bp.blk_rn[b] < A; };
+  // in the order of their first contributing element (pairs without one first): the blocks are then read as
+  // they lie, once; in row-node order the vertices' and the edge nodes' pairs each swept the whole buffer
+  std::vector<int32_t> place((size_t)n_el + 2, 0);
+  const auto bucket = [&](int32_t b, int64_t first) { return (bp.blk[b] >> 19) ? bp.con[first] / (np * np) + 1 : 0; };
   for (int32_t A = 0; A < n; ++A) {
     int64_t at = bp.rn_con[A];
+    for (int32_t b = bp.rn_blk[A]; b < bp.rn_blk[A + 1]; at += bp.blk[b++] >> 19)
+      if (!mirrored(A, b)) ++place[bucket(b, at) + 1];
+  }
+  for (size_t k = 1; k < place.size(); ++k) place[k] += place[k - 1];
+  pairs.resize((size_t)place.back());
+  pair_a.resize((size_t)place.back());
+  for (int32_t A = 0; A < n; ++A) {
+    int64_t at = bp.rn_con[A];
+    for (int32_t j = col_ptr[A]; j < col_ptr[A + 1]; ++j) block_in_col[blk_row[col_blk[j]]] = col_blk[j];
     for (int32_t b = bp.rn_blk[A]; b < bp.rn_blk[A + 1]; ++b) {
       const uint32_t w = bp.blk[b];
       const int32_t cnt = (int32_t)(w >> 19), B = bp.blk_rn[b];
       const int64_t c0 = at;
       at += cnt;
-      // element contributions come in both directions; a block without any (a pattern wider than the element
-      // graph, which need not be symmetric) is a zero of its own
-      const bool both = cnt > 0 && B >= 0;
-      if (both && B < A) continue;
-      M3Pair p;
+      if (mirrored(A, b)) continue;
+      const int32_t to = place[bucket(b, c0)]++;
+      pair_a[to] = A;
+      M3Pair& p = pairs[to];
       for (int x = 0; x < 4; ++x) p.code[x] = -1;
       p.start = (int32_t)con.size();
       p.meta = (uint32_t)cnt | ((w >> 16) & 7u) << 16;
       p.off = w & 0xFFFFu;
       p.node_b = -1;
-      if (both && B > A) {
-        const auto first = order.begin() + bp.rn_blk[B], last = order.begin() + bp.rn_blk[B + 1];
-        auto it = std::lower_bound(first, last, A, [&](int32_t x, int32_t v) { return bp.blk_rn[x] < v; });
-        // (a row that lists a column node twice: the block that holds the contributions)
-        while (it != last && bp.blk_rn[*it] == A && (bp.blk[*it] >> 19) == 0) ++it;
-        if (it == last || bp.blk_rn[*it] != A || (int32_t)(bp.blk[*it] >> 19) != cnt)
+      if (cnt > 0 && B > A) {
+        const int32_t m = block_in_col[B];  // of column A, or of an earlier one
+        if (m < 0 || bp.blk_rn[m] != A || (int32_t)(bp.blk[m] >> 19) != cnt)
           return set_error(FNE_ELAYOUT, "Mohr-Coulomb 3-D: COO pattern is not symmetric over the owned rows");
-        p.meta |= ((bp.blk[*it] >> 16) & 7u) << 19;
-        p.off |= (bp.blk[*it] & 0xFFFFu) << 16;
+        p.meta |= ((bp.blk[m] >> 16) & 7u) << 19;
+        p.off |= (bp.blk[m] & 0xFFFFu) << 16;
         p.node_b = B;
       }
       for (int64_t k = c0; k < c0 + cnt; ++k) {
@@ -665,25 +682,8 @@ int build_pairs(const BlockPlan& bp, int64_t n_el, int np, std::vector<M3Pair>& 
         else
           con.push_back(code);
       }
-      pairs.push_back(p);
-      pair_a.push_back(A);
     }
   }
-  // in the order of their first contributing element (pairs without one first): the blocks are then read as
-  // they lie, once; in row-node order the vertices' and the edge nodes' pairs each swept the whole buffer
-  const auto bucket = [&](const M3Pair& p) { return p.code[0] < 0 ? 0 : p.code[0] / 2 / npair + 1; };
-  std::vector<int32_t> at((size_t)n_el + 2, 0);
-  for (const M3Pair& p : pairs) ++at[bucket(p) + 1];
-  for (size_t k = 1; k < at.size(); ++k) at[k] += at[k - 1];
-  std::vector<M3Pair> sorted(pairs.size());
-  std::vector<int32_t> sorted_a(pairs.size());
-  for (size_t k = 0; k < pairs.size(); ++k) {
-    const int32_t to = at[bucket(pairs[k])]++;
-    sorted[to] = pairs[k];
-    sorted_a[to] = pair_a[k];
-  }
-  pairs.swap(sorted);
-  pair_a.swap(sorted_a);
   return FNE_OK;
 }
 
