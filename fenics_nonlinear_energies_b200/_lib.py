@@ -97,6 +97,7 @@ def _load():
         "fne_cg_solve": (C.c_int, [vp, vp, vp, C.c_double, C.c_int32, C.POINTER(C.c_int32), C.POINTER(C.c_int32),
                                    vp]),
         "fne_cg_launches": (C.c_int, [vp, _i64p]),
+        "fne_cg_kernels": (C.c_char_p, [vp]),
         "fne_cg_destroy": (C.c_int, [vp]),
         "fne_energy_p1tri_noalloc": (C.c_int, [C.c_int32, C.c_int64, vp, vp, vp, vp, vp, vp, vp, _f64p, vp,
                                                C.c_int64, C.c_int64, vp, vp]),
@@ -117,6 +118,7 @@ def _load():
         "fne_mlp_adam_set": (C.c_int, [C.c_int, vp, vp, vp, vp, vp, vp, C.c_float, C.c_float, C.c_float, C.c_float,
                                        C.c_int, vp]),
         "fne_mlp_cast_bf16": (C.c_int, [C.c_int64, vp, vp, vp]),
+        "fne_kernels": (C.c_char_p, [vp]),
         "fne_last_error": (C.c_char_p, []),
         "fne_version": (C.c_char_p, []),
     }

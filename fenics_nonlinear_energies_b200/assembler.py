@@ -138,6 +138,7 @@ class CudaElementAssemblerBase:
         info = _lib.Info()
         check(lib.fne_info_get(self._handle, _lib.C.byref(info)))
         self.info = {k: getattr(info, k) for k, _ in _lib.Info._fields_}
+        self.kernels = lib.fne_kernels(self._handle).decode()  # of a fused pass
 
         dev = self.device
         self._u = torch.zeros(max(1, int(lay["n_free"])), dtype=torch.float64, device=dev)

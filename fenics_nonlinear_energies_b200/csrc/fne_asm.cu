@@ -2994,6 +2994,19 @@ extern "C" int fne_info_get(const fne_handle* h, fne_info* info) {
   return FNE_OK;
 }
 
+extern "C" const char* fne_kernels(const fne_handle* h) {
+  if (!h) return "";
+  if (h->mc) return mc_kernels(h->mc);
+  if (h->mc3) return mc3d_kernels(h->mc3);
+  if (!is_tri(h->family)) return h->n_node_tiles ? "k_nodes_tet" : h->use_elem2 ? "k_he_elem+k_node_gather" : "k_rows_tet";
+  return h->n_tri_tiles   ? "k_tiles_tri"
+         : h->use_cluster ? "k_cluster_tri"
+         : h->use_push    ? "k_push_tri"
+         : h->use_sweep   ? "k_sweep_tri"
+         : h->use_inc     ? "k_inc_tri"
+                          : "k_rows_tri";
+}
+
 extern "C" int fne_hvp_prepare(fne_handle* h, const double* u, void* stream) {
   if (!h || (!u && h->n_free > 0)) return set_error(FNE_EINVAL, "fne_hvp_prepare: null argument");
   if (!h->mc) return set_error(FNE_EINVAL, "fne_hvp_prepare: matrix-free products exist for the Mohr-Coulomb family");

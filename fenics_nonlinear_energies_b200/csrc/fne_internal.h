@@ -273,6 +273,7 @@ int mc_create(const fne_desc* d, McHandle** out);
 int mc_eval(McHandle* h, const double* u, int flags, double* energy, double* grad, void* hess, void* stream);
 int mc_set_dirichlet(McHandle* h, const double* dirichlet);
 void mc_info(const McHandle* h, fne_info* info);
+const char* mc_kernels(const McHandle* h);
 int mc_check_status(McHandle* h);
 int mc_poll_status(McHandle* h);
 int mc_set_wait_limit(McHandle* h, long long polls);
@@ -287,6 +288,7 @@ int mc3d_create(const fne_desc* d, Mc3dHandle** out);
 int mc3d_eval(Mc3dHandle* h, const double* u, int flags, double* energy, double* grad, void* hess, void* stream);
 int mc3d_set_dirichlet(Mc3dHandle* h, const double* dirichlet);
 void mc3d_info(const Mc3dHandle* h, fne_info* info);
+const char* mc3d_kernels(const Mc3dHandle* h);
 void mc3d_destroy(Mc3dHandle* h);
 
 // Gather code of one element node: >= 0 reordered id of component 0 (free

@@ -775,6 +775,10 @@ extern "C" int fne_cg_launches(const fne_cg* c, int64_t* launches) {
   return FNE_OK;
 }
 
+extern "C" const char* fne_cg_kernels(const fne_cg* c) {
+  return !c ? "" : c->width ? "k_cg_spmv_rows+k_cg_update" : "k_cg_spmv+k_cg_update";
+}
+
 extern "C" int fne_cg_destroy(fne_cg* c) {
   cg_free(c);
   return FNE_OK;

@@ -2218,4 +2218,11 @@ void mc_info(const McHandle* h, fne_info* info) {
   info->row_lanes = 1;
 }
 
+const char* mc_kernels(const McHandle* h) {
+  return h->tc        ? "k_mc_tc+k_fixup2+k_rowgrad"
+         : h->dm      ? "k_mc_dmma+k_fixup2+k_rowgrad"
+         : h->use_blk ? "k_mc_elem+k_node_gather+k_rowgrad"
+                      : "k_mc_elem+k_mc_gather+k_mc_grad_gather";
+}
+
 }  // namespace fne

@@ -941,4 +941,8 @@ void mc3d_info(const Mc3dHandle* h, fne_info* info) {
   info->row_lanes = 1;
 }
 
+const char* mc3d_kernels(const Mc3dHandle* h) {
+  return h->np == 35 ? "k_mc3d_elem_hi+k_mc3d_gather" : "k_mc3d_elem+k_mc3d_gather";
+}
+
 }  // namespace fne

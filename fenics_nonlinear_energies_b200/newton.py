@@ -139,6 +139,7 @@ class DeviceCG:
         self._h = h
         self.chunk = int(chunk)
         self.reason = None
+        self.kernels = _lib.lib.fne_cg_kernels(h).decode()  # of an iteration
         self.launches = 0  # kernels launched by update() and solve() so far
 
     @classmethod

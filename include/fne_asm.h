@@ -225,6 +225,10 @@ typedef struct {
 
 int fne_create(const fne_desc* desc, fne_handle** out);
 int fne_info_get(const fne_handle* h, fne_info* info);
+/* The kernels that a fused pass of this handle launches, joined by '+' (a constant string).
+ * fne_info.kernel_variant numbers families of kernels: 2 is the row-gather over tiles of
+ * row nodes (k_nodes_tet) as well as the one over rows (k_rows_tet). */
+const char* fne_kernels(const fne_handle* h);
 /*
  * Matrix-free Hessian products (Mohr-Coulomb handles), replacing the
  * reference's prepare_matrix_free_operator / matrix_free_mult /
@@ -356,6 +360,8 @@ int fne_cg_solve(fne_cg* cg, const double* b, double* x, double rtol, int32_t ma
 /* Kernels that the last fne_cg_solve launched, those of a graph launched ahead
  * that turned out not to be needed included. */
 int fne_cg_launches(const fne_cg* cg, int64_t* launches);
+/* The two kernels of an iteration on this pattern (a constant string). */
+const char* fne_cg_kernels(const fne_cg* cg);
 int fne_cg_destroy(fne_cg* cg);
 
 /* ---------------------------------------------------------------------------

@@ -471,3 +471,73 @@ def test_tiles_hold_no_row_lists():
     asm = _asm_classes()["gl"](params)
     assert asm.info["kernel_variant"] == 12
     assert asm.info["device_bytes"] <= 200 * params["elems"].shape[0]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_tets_run_the_node_tiles(precision):
+    """The default tet pass runs k_nodes_tet on the beams, small and shuffled ones too (the comparison with the
+    row-gather kernel above would also pass if every mesh fell back to it)."""
+    cls = _asm_classes()["he"]
+    hd = torch.float32 if precision == "fp32" else torch.float64
+    rng = np.random.default_rng(2)
+    for size in ((2, 1, 1), (5, 3, 2), (9, 4, 5), (40, 8, 8)):
+        params, y0 = meshes.he_beam_problem(nx=size[0], ny=size[1], nz=size[2])
+        perm = (3 * rng.permutation(y0.size // 3)[:, None] + np.arange(3)).ravel()
+        for kw in ({}, {"perm_override": perm}):
+            assert cls(params, precision=precision, hess_dtype=hd, **kw).kernels == "k_nodes_tet"
+        assert cls(params, precision=precision, hess_dtype=hd, kernel_variant="row_gather").kernels == "k_rows_tet"
+
+
+def _star_problem(n, free_ring):
+    """Tets from a centre node to the 4 n - 4 triangles of a sphere of 2 n nodes, fixed except ``free_ring`` of them."""
+    ang = 2.0 * np.pi * np.arange(n - 1) / (n - 1)
+    north, south = [[0.0, 0.0, 1.0]], [[0.0, 0.0, -1.0]]
+    rings = [np.column_stack((np.sqrt(1 - z * z) * np.cos(ang + z), np.sqrt(1 - z * z) * np.sin(ang + z), np.full(n - 1, z)))
+             for z in (0.4, -0.4)]
+    nodes = np.vstack([[[0.0, 0.0, 0.0]], north, *rings, south])
+    a = 2 + np.arange(n - 1)
+    b, nxt = a + n - 1, 2 + (np.arange(n - 1) + 1) % (n - 1)
+    nxtb, s = nxt + n - 1, nodes.shape[0] - 1
+    tri = np.vstack([np.column_stack(t) for t in ((np.full(n - 1, 1), a, nxt), (a, b, nxt), (nxt, b, nxtb),
+                                                  (np.full(n - 1, s), nxtb, b))])
+    es = np.column_stack([np.zeros(tri.shape[0], dtype=np.int64), tri]).astype(np.int64)
+    dphix, dphiy, dphiz, vol = meshes.p1_tet_operators(nodes, es)
+    free_nodes = np.arange(free_ring + 1) + (np.arange(free_ring + 1) > 0)
+    u0 = nodes.reshape(-1).copy()
+    return {"u_0": u0.copy(), "u_0_ref": u0.copy(), "freedofs": (3 * free_nodes[:, None] + np.arange(3)).ravel(),
+            "elems": meshes.expand_connectivity_to_dofs(es, 3), "elems_scalar": es, "dphix": dphix, "dphiy": dphiy,
+            "dphiz": dphiz, "vol": vol, "C1": 1.0, "D1": 2.0, "nodes2coord": nodes}
+
+
+@pytest.mark.parametrize("n,kernel", [(33, "k_nodes_tet"), (34, "k_rows_tet"), (60, "k_rows_tet")])
+def test_a_node_of_many_tets_falls_back_to_rows(n, kernel):
+    """A node of 128 tets fills a tile of row nodes; one of more goes, with its mesh, to the row-gather kernel."""
+    params = _star_problem(n, 5)
+    gpu, ref = _make("he", params)
+    assert params["elems"].shape[0] == 4 * n - 4 and gpu.kernels == kernel
+    u = params["u_0"][params["freedofs"]] + 0.02 * np.random.default_rng(n).standard_normal(params["freedofs"].size)
+    _check(gpu, ref, u[np.asarray(gpu.layout.perm)], FP64_TOL, energy_scale=_abs_energy_scale(ref, u[np.asarray(gpu.layout.perm)]))
+
+
+def test_rows_of_a_node_apart_fall_back_to_rows(monkeypatch):
+    """A COO pattern that lists all rows of the first component, then the second, then the third: the same values."""
+    params, y0 = meshes.he_beam_problem(nx=6, ny=2, nz=3)
+    cls = _asm_classes()["he"]
+    build = _lib.build_layout
+
+    def apart(**kw):
+        lay = build(**kw)
+        at = np.argsort(lay["owned_rows"] % 3, kind="stable")
+        lay["owned_rows"], lay["owned_cols"] = lay["owned_rows"][at], lay["owned_cols"][at]
+        lay["at"] = at
+        return lay
+
+    a = cls(params)
+    monkeypatch.setattr(_lib, "build_layout", apart)
+    b = cls(params)
+    assert (a.kernels, b.kernels) == ("k_nodes_tet", "k_rows_tet")
+    u = torch.as_tensor(y0 + 1e-3 * np.random.default_rng(1).standard_normal(y0.size), device="cuda")
+    ea, ga, ha = [t.cpu().numpy().copy() for t in a.eval(u, 7)]
+    eb, gb, hb = [t.cpu().numpy() for t in b.eval(u, 7)]
+    assert abs(ea - eb) <= 1e-12 * max(1e-3, abs(eb)) and _rel(ga, gb) <= FP64_TOL
+    assert _rel(ha[b.layout.at], hb) <= FP64_TOL
