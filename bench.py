@@ -519,6 +519,8 @@ REFERENCE_ARCHIVED = {
                    "hardware not recorded"},
 }
 
+# Kernels by fne_info.kernel_variant, as first numbered.  The benchmark line prints what the handle reports
+# (``assembler.kernels``, ``DeviceCG.kernels``): 2 stands for two kernels, and 11 has its own gather since.
 KERNEL_NAMES = {1: "k_rows_tri", 2: "k_rows_tet", 3: "k_inc_tri", 4: "k_sweep_tri",
                 5: "k_mc_elem+k_node_gather+k_rowgrad", 6: "k_mc_tc+k_fixup2+k_rowgrad", 7: "k_he_elem+k_node_gather",
                 8: "k_push_tri", 9: "k_mc_dmma+k_fixup2+k_rowgrad", 10: "k_cluster_tri",
@@ -991,8 +993,8 @@ def run_newton(args, w, world, rank, local):
     s_per_solve = total_s / args.steps
     e2e_s = _max_over_ranks(sum(a.elapsed_time(b) for a, b in e2e) * 1e-3, world) / args.steps
 
-    # roofline of the dominant kernel pair (one CG iteration: k_cg_spmv +
-    # k_cg_update) on the Hessian at the solution, timed on its own
+    # roofline of the dominant kernel pair (one CG iteration: product and
+    # update) on the Hessian at the solution, timed on its own
     from fenics_nonlinear_energies_b200 import _lib
 
     asm.eval(x, _lib.FNE_HESS)
@@ -1011,7 +1013,7 @@ def run_newton(args, w, world, rank, local):
     alg = nnz * (vb + 4) + (n + 1) * 4 + 12 * n * 8
     peak, peak_kind = _peaks()
     achieved = alg / (us_it * 1e-6) / 1e9
-    traffic = NCU_TRAFFIC.get((w.name, "k_cg_spmv+k_cg_update"))
+    traffic = NCU_TRAFFIC.get((w.name, cg.kernels))
     its = [i["iterations"] for i in infos]
     ksp = [sum(h["ksp_its"] for h in i["history"]) for i in infos]
     if rank == 0:
@@ -1031,7 +1033,7 @@ def run_newton(args, w, world, rank, local):
                          "peak_kind": f"{peak_kind} burst copy (hbm_gbs)",
                          "traffic": traffic[0] if traffic else None,
                          "traffic_source": traffic[1] if traffic else None,
-                         "algorithmic_bytes_per_launch": alg, "kernel": "k_cg_spmv+k_cg_update",
+                         "algorithmic_bytes_per_launch": alg, "kernel": cg.kernels,
                          "unit_of_launch": "one CG iteration (two kernels)", "us_per_cg_iteration": us_it,
                          "cg_iterations_timed": cg_its},
             "e2e": {"value": e2e_s, "unit": "s", "h2d_bytes_per_step": int(u0.nbytes),
@@ -1129,7 +1131,7 @@ def run(args):
     peak, peak_kind = _peaks()
     avg_launch_s = (sum(kernel_ms) / len(kernel_ms)) * 1e-3
     achieved = alg_bytes / avg_launch_s / 1e9
-    kname = ENERGY_KERNELS[w.family] if energy_only else KERNEL_NAMES.get(asm.info["kernel_variant"], "?")
+    kname = ENERGY_KERNELS[w.family] if energy_only else asm.kernels
     traffic = NCU_TRAFFIC.get((w.name, kname))
     nnz = int(asm.owned_values.numel())
 
