@@ -184,3 +184,51 @@ def test_fused_layer_edges(rows, din, dout):
     _lib.check(L.fne_mlp_linear_bwd_weight(rows, dout, din, vp(Zp), ldz, vp(Xp), ldx, vp(gP), None, None, None))
     assert torch.equal(gP, gW)
     _lib.check(L.fne_gemm_check_status())
+
+
+@pytest.mark.parametrize("rows", [1, 129, 1300])
+@pytest.mark.parametrize("din,dout", [(12, 64), (64, 3), (40, 33), (72, 200), (1100, 40)])
+def test_fused_layers_equal_their_separate_calls(rows, din, dout):
+    """The fused forward and input gradient give the bits of the product followed by the elementwise call, and the
+    optimiser over a set of tensors those of one call per tensor."""
+    from fenics_nonlinear_energies_b200 import _lib
+    from fenics_nonlinear_energies_b200.warmstart import gemm
+
+    L, vp = _lib.lib, lambda t: t.data_ptr()  # noqa: E731
+    g = torch.Generator().manual_seed(rows + din + dout)
+    rand = lambda *s: torch.randn(*s, generator=g, dtype=torch.float32).cuda()  # noqa: E731
+    new = lambda *s, dtype=torch.float32: torch.full(s, 7.0, dtype=dtype, device="cuda")  # noqa: E731
+    X, W, b = rand(rows, din).bfloat16(), (rand(dout, din) / din ** 0.5).bfloat16(), rand(dout)
+    for act in (0, 1):
+        Z, H, H16 = new(rows, dout), new(rows, dout), new(rows, dout, dtype=torch.bfloat16)
+        Z1, H1, H161 = new(rows, dout), new(rows, dout), new(rows, dout, dtype=torch.bfloat16)
+        _lib.check(L.fne_mlp_linear_fwd(rows, din, dout, vp(X), vp(W), vp(b), act, vp(Z), vp(H), vp(H16), None))
+        gemm(X, din, 1, W, 1, din, rows, dout, din, Z1)
+        _lib.check(L.fne_mlp_bias_act(rows, dout, vp(Z1), vp(b), act, vp(H1), vp(H161), None))
+        assert torch.equal(Z, Z1) and torch.equal(H, H1) and torch.equal(H16, H161)
+        dZ, Zin = rand(rows, dout).bfloat16(), rand(rows, din)
+        d16, part = new(rows, din, dtype=torch.bfloat16), new(-(-rows // 128), din, dtype=torch.float64)
+        C, d161 = new(rows, din), new(rows, din, dtype=torch.bfloat16)
+        _lib.check(L.fne_mlp_linear_bwd_data(rows, din, dout, vp(dZ), dout, vp(W), vp(Zin), act, vp(d16), vp(part), None))
+        gemm(dZ, dout, 1, W, din, 1, rows, din, dout, C)
+        _lib.check(L.fne_mlp_act_bwd(rows * din, vp(Zin), vp(C), act, vp(C), vp(d161), None))
+        assert torch.equal(d16, d161)
+        # C holds the FP32 gradients; the sums of a tile are FP64 sums of 128 of them in some order
+        sums = torch.stack([C[k:k + 128].double().sum(0) for k in range(0, rows, 128)])
+        assert (part - sums).abs().max() <= 128 * 2.0 ** -53 * C.double().abs().max() * 128
+    sizes = (dout * din, dout, 1)
+    sets = [[[rand(n), rand(n), rand(n).abs(), rand(n).abs()] for n in sizes]]  # p, g, m, v
+    sets.append([[t.clone() for t in s] for s in sets[0]])
+    p16 = [[new(n, dtype=torch.bfloat16) for n in sizes[:2]] + [None] for _ in range(2)]
+    args = (1e-3, 0.9, 0.999, 1e-8, 3)
+    import ctypes
+
+    ptrs = [(ctypes.c_void_p * 3)(*(vp(s[k]) for s in sets[0])) for k in range(4)]
+    h16 = (ctypes.c_void_p * 3)(*(vp(t) if t is not None else None for t in p16[0]))
+    _lib.check(L.fne_mlp_adam_set(3, (ctypes.c_int64 * 3)(*sizes), *ptrs, h16, *args, None))
+    for s, t in zip(sets[1], p16[1]):
+        _lib.check(L.fne_mlp_adam(s[0].numel(), *(vp(x) for x in s), *args, vp(t) if t is not None else None, None))
+    for s, s1 in zip(*sets):
+        assert all(torch.equal(x, y) for x, y in zip(s, s1))
+    assert all(torch.equal(x, y) for x, y in zip(p16[0][:2], p16[1][:2]))
+    _lib.check(L.fne_gemm_check_status())
