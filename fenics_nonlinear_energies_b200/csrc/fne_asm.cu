@@ -1494,7 +1494,7 @@ __global__ void __launch_bounds__(NB, 2) k_push_tri(RowArgs A, SweepArgs S, cons
 // spread better (Hessian 76 -> 70 us).  A compact cluster of 256 rows
 // re-evaluates 1.13x (a segment of the sweep 1.29x).  On 2.1 M triangles,
 // against the sweep: gradient 86 -> 48 us, Hessian 112 -> 70, all three
-// 124 -> 84 (FP32: 50 -> 34, 71 -> 54, 84 -> 65).  What is left is the
+// 128 -> 83 (FP32: 50 -> 34, 71 -> 53, 84 -> 65).  What is left is the
 // evaluation's arithmetic between two barriers and the latency of a tile's
 // first loads.
 // ---------------------------------------------------------------------------
@@ -2642,9 +2642,10 @@ extern "C" int fne_create(const fne_desc* d, fne_handle** out) {
       use_cluster = build_cluster_plan(plan, d->lo, d->hi, lay.cr, lay.cj, lay.ci, lay.cw, gid, cplan);
     if (use_cluster && cplan.max_runs > lay.cu) use_cluster = false;
   }
-  // tiles of rows (triangles by default; 128 -> 84 us for the fused pass over
+  // tiles of rows (triangles by default; 128 -> 83 us for the fused pass over
   // 2.1 M triangles against the banded sweep, which stays for rows of more than
-  // 16 elements or 14 entries: the row clusters have four bits for a place): small meshes get smaller tiles, two per SM
+  // 16 elements or 14 entries: the row clusters have four bits for a place);
+  // small meshes get smaller tiles, two per SM
   TilePlan tplan;
   bool use_tiles = false;
   if (is_tri(d->family) && plan.n_rows > 0 && d->kernel_variant == 0) {

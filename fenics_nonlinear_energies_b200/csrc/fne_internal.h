@@ -201,7 +201,7 @@ struct TilePlan {
   std::vector<uint32_t> ent;         // [n_rows * lanes]
   std::vector<uint16_t> inc;         // [n_rows * lanes]
 };
-// False when the mesh does not fit (rows or valences beyond 16, an
+// False when the mesh does not fit (rows beyond 14 entries, valences beyond 16, an
 // off-diagonal entry with more than two elements, a row without its diagonal).
 bool build_tile_plan(const RowPlan& P, int64_t lo, int64_t hi, int max_jobs, bool gpos_identity, TilePlan& T);
 

@@ -13,7 +13,7 @@
 // same fixed order, and so knows alpha (or beta and the stop flags) without any
 // block waiting for a last one to publish it (the ticket, fence and single-block
 // reduction at the end of each kernel were about 3 us).  One thread per block
-// reads the 80-byte state and partials come through L1: read by every warp, that
+// reads the 96-byte state and partials come through L1: read by every warp, that
 // one line was 20,000 requests to one L2 slice.  Block 0 records the
 // scalars in one of two states, spmv in `after_update`, the update in
 // `after_spmv`, each read only by the other kernel.  A kernel whose state says
@@ -25,7 +25,8 @@
 // completion).  z and p_old of a row lie side by side, one 16-byte gather.
 // Short rows (at most 16 entries, little padding: the triangle meshes) are
 // stored column-major with one thread per row, coalesced and without shuffles;
-// longer rows take G lanes per row on CSR.
+// longer rows take G lanes per row on CSR.  Creation writes CSR on the host and
+// turns it around on the device.
 // Reductions use a fixed launch shape and a fixed order: the result of a solve
 // is reproducible bit for bit.
 //
@@ -61,6 +62,7 @@ struct alignas(16) CgState {
   int32_t chunk;   // graphs run (its low bit: the host slot)
   double rr, rr0;  // ||r||^2 now and at the start
 };
+static_assert(sizeof(CgState) == 96, "the state's size is named above");
 
 struct CgVecs {
   const int32_t* crow;  // CSR; with width > 0 col and vals hold column-major rows of `width` entries at stride `stride`, column -1 = none

@@ -1,4 +1,4 @@
-// 3-D Mohr-Coulomb slope family (P1 / P2 tetrahedra, 3 DOFs per node):
+// 3-D Mohr-Coulomb slope family (P1 / P2 / P4 tetrahedra, 3 DOFs per node):
 // element energy, gradient and constitutive Hessian on the GPU, scattered
 // into the owned gradient and COO values.
 //
@@ -14,18 +14,18 @@
 // quad_weight and the material fields c_bar_q, sin_phi_q, shear_q, bulk_q,
 // lame_q (E, nq).
 //
-// k_mc3d_elem: a CTA of 128 threads takes a tile of 128 / nq elements.  One
-// thread per (element, quadrature point) forms the strain and runs the
-// constitutive point function (FP64: eigen-decomposition by cyclic
-// Jacobi, branch potentials, spectral tangent) and stores w sigma and the
-// upper triangle of w D in shared memory.  Then one warp per element: lanes
-// over (node, component) form the element gradient; per quadrature point,
-// lanes over nodes form (w D) B(b) from the three nonzeros of each column of
-// B and lanes over node pairs a <= b add B(a)^T (w D) B(b) to their 3 x 3
-// blocks.  Blocks and gradients go to per-element buffers that the
-// node-block gather (fne_gather.cuh: per output block, contributions in
-// element order, no atomics) sums into the COO values and the gradient.  FP32 mode keeps the point function in FP64 and runs the
-// contraction, the buffers and the Hessian output in FP32.
+// k_mc3d_elem (P1 / P2): a CTA of 128 threads takes a tile of 128 / nq elements.
+// One thread per (element, quadrature point) forms the strain and runs the
+// constitutive point function (FP64: eigen-decomposition by cyclic Jacobi,
+// branch potentials, spectral tangent) and stores w sigma and the upper triangle
+// of w D in shared memory.  Then one lane per node b of an element forms
+// (w D) B(b) and its products with B(a) in registers, every unordered pair of
+// nodes once, and its three gradient entries.  k_mc3d_elem_hi (P4) contracts one
+// node at a time.  Blocks and gradients go to per-element buffers, which
+// k_mc3d_gather sums by pairs of row nodes into the COO values and the gradient
+// (contributions in element order, no atomics).  FP32 mode keeps the point
+// function in FP64 and runs the contraction, the buffers and the Hessian output
+// in FP32.
 #include <cuda_runtime.h>
 
 #include <algorithm>

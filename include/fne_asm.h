@@ -216,8 +216,8 @@ typedef struct {
                            * 9 Mohr-Coulomb FP64 DMMA (mma.sync f64),
                            * 10 row clusters (P1 triangles),
                            * 11 3-D Mohr-Coulomb point-tile element kernel +
-                           * node-block gather, 12 tiles of rows (P1
-                           * triangles) */
+                           * gather by pairs of nodes, 12 tiles of rows (P1
+                           * triangles); fne_kernels names the kernels */
   int32_t row_lanes;      /* lanes per output row of the tet row kernel (for
                            * kernel_variant 0 the count it would run with where
                            * the tiles of row nodes do not apply), else 1 */
