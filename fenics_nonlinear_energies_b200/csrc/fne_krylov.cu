@@ -759,6 +759,11 @@ extern "C" int fne_cg_solve(fne_cg* c, const double* b, double* x, double rtol, 
     return set_error(FNE_EINVAL, "fne_cg_solve: bad arguments");
   if (!c->have_matrix) return set_error(FNE_EINVAL, "fne_cg_solve: fne_cg_set_matrix was not called");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();  // (nor may `done` become an event of a capture)
+    return set_error(FNE_ECUDA, "fne_cg_solve: the stream is being captured, and the host drives a solve");
+  }
   if (!c->exec) {
     const int rc = build_graph(c);
     if (rc != FNE_OK) return rc;

@@ -354,7 +354,8 @@ int fne_cg_set_matrix(fne_cg* cg, const void* coo_vals, void* stream);
  * curvature, 2 iteration limit, 3 zero right-hand side.  Waits for the state
  * once per `chunk` iterations; on return up to one graph of kernels that change
  * nothing and the copy to x may still be in the stream.  A handle runs one solve
- * at a time (a later solve on another stream waits for this one). */
+ * at a time (a later solve on another stream waits for this one).  The host
+ * drives a solve: refused on a stream under capture. */
 int fne_cg_solve(fne_cg* cg, const double* b, double* x, double rtol, int32_t maxit, int32_t* its, int32_t* reason,
                  void* stream);
 /* Kernels that the last fne_cg_solve launched, those of a graph launched ahead

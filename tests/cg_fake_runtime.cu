@@ -20,7 +20,7 @@ namespace {
 std::vector<std::string> calls;             // graph launches, waits, event records, frees
 std::vector<double> residual;               // ||r||^2 after graph k; -1: this one reports the stop
 cudaError_t last = cudaSuccess;
-int launches = 0, graphs = 0, fail_graph = -1, fail_wait = -1, waits = 0;
+int launches = 0, graphs = 0, fail_graph = -1, fail_wait = -1, waits = 0, capturing = 0;
 fne::CgState* host_state = nullptr;
 int chunk = 0, handles = 0;
 std::vector<void*> events;
@@ -62,7 +62,9 @@ cudaError_t cudaEventSynchronize(cudaEvent_t e) {
   return name_of(e) != "done" && waits++ == fail_wait ? last = cudaErrorLaunchFailure : cudaSuccess;
 }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
-cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) { return *s = cudaStreamCaptureStatusNone, cudaSuccess; }
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) {
+  return *s = capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone, cudaSuccess;
+}
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { return *s = (cudaStream_t)std::malloc(1), cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
@@ -121,12 +123,12 @@ char __cudaInitModule(void**) { return 1; }
 }
 #endif
 
-// usage: chunk, graph launch that fails (-1: none), wait that fails (-1), residual after each graph ... (the last for
-// all that follow; -1: stop; nan)
+// usage: chunk, graph launch that fails (-1: none), wait that fails (-1), whether the solve's stream is being captured,
+// residual after each graph ... (the last for all that follow; -1: stop; nan)
 int main(int argc, char** argv) {
   fail_graph = std::atoi(argv[2]);
   fail_wait = std::atoi(argv[3]);
-  for (int k = 4; k < argc; ++k) residual.push_back(std::atof(argv[k]));
+  for (int k = 5; k < argc; ++k) residual.push_back(std::atof(argv[k]));
   const int64_t idx[4] = {0, 1, 2, 3};
   const double v[4] = {1, 1, 1, 1};
   double x[4];
@@ -136,6 +138,7 @@ int main(int argc, char** argv) {
   fne_cg_set_matrix(c, v, nullptr);
   calls.clear();
   launches = 0;
+  capturing = std::atoi(argv[4]);
   const int rc = fne_cg_solve(c, v, x, 1e-6, 1000000, &its, &why, nullptr);
   int64_t told = -1;
   fne_cg_launches(c, &told);

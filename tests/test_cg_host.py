@@ -24,8 +24,8 @@ def solve(tmp_path_factory):
                           os.fspath(HERE / "cg_fake_runtime.cu")], capture_output=True, text=True)
     assert out.returncode == 0, out.stderr[-3000:]
 
-    def run(*residuals, chunk=16, fail_graph=-1, fail_wait=-1):
-        args = [chunk, fail_graph, fail_wait, *residuals]
+    def run(*residuals, chunk=16, fail_graph=-1, fail_wait=-1, capturing=0):
+        args = [chunk, fail_graph, fail_wait, capturing, *residuals]
         text = subprocess.run([exe, *map(str, args)], capture_output=True, text=True, check=True, timeout=60).stdout
         head, calls, freed = text.splitlines()
         code, its, launches, told = map(int, head.split())
@@ -63,3 +63,10 @@ def test_no_graph_ahead_of_a_residual_without_a_rate(solve, after_first):
     """A residual that is not a number (or has overflowed) gives no rate to guess by: the next graph waits for the state."""
     calls = solve(after_first, -1)["calls"]
     assert calls == ["graph", "record ev0", "wait ev0", "graph", "record ev1", "wait ev1", "copy", "record done"]
+
+
+def test_a_solve_under_capture_is_refused_before_it_leaves_anything(solve):
+    """A solve is driven by the host, so it cannot be captured: nothing goes into the stream, the event least of all
+    (a captured one would be refused by every later wait)."""
+    r = solve(-1, capturing=1)
+    assert r["code"] == _lib.FNE_ECUDA and r["calls"] == [] and r["launches"] == 0

@@ -220,3 +220,27 @@ def test_cg_one_handle_on_two_streams(m):
     cg.close()
     for (x, it), (x1, it1) in zip(outs, alone):
         assert it == it1 and torch.equal(x, x1)
+
+
+def test_cg_solve_is_refused_under_capture_and_runs_after_it():
+    from fenics_nonlinear_energies_b200 import _lib
+    from fenics_nonlinear_energies_b200.newton import DeviceCG
+
+    n, rows, cols, vals = _band_coo(1003, 3, 30)
+    b = torch.as_tensor(np.random.default_rng(3).standard_normal(n), device="cuda")
+    cg = DeviceCG(n, rows, cols)
+    cg.update(torch.as_tensor(vals, device="cuda"))
+    x, it = cg.solve(b, rtol=1e-8)
+    out = torch.empty_like(b)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out.add_(1.0)
+        with pytest.raises(_lib.FneError):
+            cg.solve(b, rtol=1e-8, out=torch.empty_like(b))
+    side = torch.cuda.Stream()
+    for stream in (torch.cuda.current_stream(), side):
+        with torch.cuda.stream(stream):
+            x1, it1 = cg.solve(b, rtol=1e-8)
+        torch.cuda.synchronize()
+        assert it1 == it and torch.equal(x1, x)
+    cg.close()
